@@ -16,10 +16,8 @@ from pathlib import Path
 
 import torch
 
-_ROOT = Path(__file__).resolve().parent.parent
-for _p in (_ROOT / "pytorch-apple_b200", _ROOT):
-    if str(_p) not in sys.path:
-        sys.path.insert(0, str(_p))
+# the package of the tree in the working folder, whichever tree this file itself lies in
+sys.path.insert(0, str(Path.cwd() / "pytorch-apple_b200"))
 
 import model_zoo as mz  # noqa: E402
 from cuda_compiler import compile_subgraph, is_cuda_op_supported  # noqa: E402
