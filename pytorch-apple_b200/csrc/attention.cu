@@ -319,30 +319,74 @@ __global__ void __launch_bounds__(128, STAGES == 2 ? 3 : 2) attn_decode_kernel(c
   }
 }
 
-// grid = B*Hq blocks of 128 threads (one per head dim)
+// Adds up the splits' partial results.  grid = (B*Hq, HD / 32), 256 threads: thread (grp = tid / 8, c4 = tid % 8)
+// owns 4 of the block's 32 dims and every 32nd split, so a 32768-row cache (256 splits) costs a thread eight
+// independent loads; the 32 groups then meet in shared memory.  Bound by the latency of an L2 round trip: 12
+// blocks of one thread per dim, each walking all splits, made the decode step of one sequence over a 32768-row
+// cache with 20000 rows filled 2171 us; this way it takes 1390 us (28 us less per layer).
+constexpr int MRG_GROUPS = 32, MRG_DIMS = 32, MRG_PITCH = MRG_DIMS + 4;
 template <typename T>
-__global__ void __launch_bounds__(128) attn_decode_merge_kernel(const float* __restrict__ part_acc, const float* __restrict__ part_ml,
+__global__ void __launch_bounds__(256) attn_decode_merge_kernel(const float* __restrict__ part_acc, const float* __restrict__ part_ml,
                                                                 T* __restrict__ out, int Hq, int Hkv, int G, int splits) {
+  __shared__ __align__(16) float s_acc[MRG_GROUPS][MRG_PITCH];
+  __shared__ float s_m[MRG_GROUPS], s_l[MRG_GROUPS];
   const int64_t bh = blockIdx.x, b = bh / Hq;
   const int h = static_cast<int>(bh % Hq), hk = h / G, r = h % G;
-  pdl_wait();
+  const int grp = threadIdx.x >> 3, c4 = threadIdx.x & 7;
   pdl_trigger();
+  pdl_wait();
   const int64_t base = (b * Hkv + hk) * splits;
-  // (the loads of different splits are independent: unrolled, they overlap instead of queueing up one
-  // L2 round trip each - 256 splits of a 32768-row cache took 20 us that way)
-  float m_all = -INFINITY;
-#pragma unroll 8
-  for (int s = 0; s < splits; ++s) m_all = fmaxf(m_all, __ldg(&part_ml[((base + s) * G + r) * 2]));
-  const float m_use = m_all == -INFINITY ? 0.f : m_all;
-  float acc = 0.f, l = 0.f;
-#pragma unroll 8
-  for (int s = 0; s < splits; ++s) {
-    const int64_t i = (base + s) * G + r;
-    const float f = ex2_approx(__ldg(&part_ml[i * 2]) - m_use);   // maxima are stored in the log2 domain
-    l += __ldg(&part_ml[i * 2 + 1]) * f;
-    acc += __ldg(&part_acc[i * HD + threadIdx.x]) * f;
+  const int d0 = blockIdx.y * MRG_DIMS + c4 * 4;
+  constexpr int BATCH = 8;   // splits whose loads are in flight together
+  const bool vec = (reinterpret_cast<uintptr_t>(part_acc) & 15u) == 0;   // the caller's workspace need not be 16-byte aligned
+  float m_run = -INFINITY, l = 0.f;
+  float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+  for (int s0 = grp; s0 < splits; s0 += BATCH * MRG_GROUPS) {
+    float2 ml[BATCH];
+    float4 a[BATCH];
+#pragma unroll
+    for (int j = 0; j < BATCH; ++j) {
+      const int s = s0 + j * MRG_GROUPS;
+      const int64_t i = (base + s) * G + r;
+      ml[j] = make_float2(-INFINITY, 0.f);   // (max in the log2 domain, sum)
+      a[j] = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (s < splits) {
+        const float* pa = part_acc + i * HD + d0;
+        ml[j] = make_float2(__ldg(part_ml + 2 * i), __ldg(part_ml + 2 * i + 1));
+        a[j] = vec ? __ldg(reinterpret_cast<const float4*>(pa)) : make_float4(__ldg(pa), __ldg(pa + 1), __ldg(pa + 2), __ldg(pa + 3));
+      }
+    }
+    float m_new = m_run;
+#pragma unroll
+    for (int j = 0; j < BATCH; ++j) m_new = fmaxf(m_new, ml[j].x);
+    const float m_use = m_new == -INFINITY ? 0.f : m_new;
+    const float c = ex2_approx(m_run - m_use);
+    l *= c; acc.x *= c; acc.y *= c; acc.z *= c; acc.w *= c;
+#pragma unroll
+    for (int j = 0; j < BATCH; ++j) {
+      const float f = ex2_approx(ml[j].x - m_use);
+      l += ml[j].y * f;
+      acc.x += a[j].x * f; acc.y += a[j].y * f; acc.z += a[j].z * f; acc.w += a[j].w * f;
+    }
+    m_run = m_new;
   }
-  out[bh * HD + threadIdx.x] = from_f32<T>(l > 0.f ? acc / l : 0.f);
+  *reinterpret_cast<float4*>(&s_acc[grp][c4 * 4]) = acc;
+  if (c4 == 0) { s_m[grp] = m_run; s_l[grp] = l; }
+  __syncthreads();
+  if (threadIdx.x < MRG_DIMS) {
+    float m_all = -INFINITY;
+#pragma unroll
+    for (int g = 0; g < MRG_GROUPS; ++g) m_all = fmaxf(m_all, s_m[g]);
+    const float m_use = m_all == -INFINITY ? 0.f : m_all;
+    float o = 0.f, lt = 0.f;
+#pragma unroll
+    for (int g = 0; g < MRG_GROUPS; ++g) {
+      const float f = ex2_approx(s_m[g] - m_use);
+      lt += s_l[g] * f;
+      o += s_acc[g][threadIdx.x] * f;
+    }
+    out[bh * HD + blockIdx.y * MRG_DIMS + threadIdx.x] = from_f32<T>(lt > 0.f ? o / lt : 0.f);
+  }
 }
 
 // ===========================================================================
@@ -710,7 +754,7 @@ extern "C" int b200_attn_decode(const void* q, const void* k, const void* v, con
       cudaLaunchKernelEx(&cfg, attn_decode_kernel<T, 2, true>, p);
     } else {
       launch_pdl(attn_decode_kernel<T, 2, false>, grid, dim3(128), 4 * 2 * DEC_STAGE_BYTES, st, p);
-      launch_pdl(attn_decode_merge_kernel<T>, dim3(static_cast<unsigned>(B * Hq)), dim3(128), 0, st, static_cast<const float*>(p.part_acc),
+      launch_pdl(attn_decode_merge_kernel<T>, dim3(static_cast<unsigned>(B * Hq), HD / MRG_DIMS), dim3(256), 0, st, static_cast<const float*>(p.part_acc),
                  static_cast<const float*>(p.part_ml), static_cast<T*>(out), Hq, Hkv, p.G, d.splits);
     }
   });

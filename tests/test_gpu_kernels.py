@@ -318,6 +318,27 @@ def test_attn_decode(lib, B, S, valid):
     close(out, attn_ref(q, k, v, None, D ** -0.5, dtype)[:, :, 0], rtol=2e-2, atol=5e-3)
 
 
+@pytest.mark.parametrize("B,S,valid,shift", [(1, 32768, 20001, 0), (1, 32768, 32768, 1), (2, 17000, 1, 0), (3, 448, 447, 0), (1, 16, 5, 1), (1, 64, 64, 0)])
+def test_attn_decode_merge_of_workspace_partials(lib, B, S, valid, shift):
+    """Caches outside 512..16384 rows leave their splits' partial sums in the workspace for a second kernel: one
+    split, fewer splits than the kernel has groups, 256 of them with the masked ones empty; a workspace that is
+    only 4-byte aligned."""
+    import model_zoo as mz
+
+    dtype, Hq, Hkv, D = torch.bfloat16, 12, 2, 128
+    q, k, v = gen((B, Hq, 1, D), dtype), gen((B, Hkv, S, D), dtype, 1), gen((B, Hkv, S, D), dtype, 2)
+    mask = mz.causal_mask(B, 1, S, valid - 1)
+    ref = attn_ref(q, k, v, mask, D ** -0.5, dtype)[:, :, 0]
+    Q, K, V, M = q.cuda(), k.cuda(), v.cuda(), mask.cuda()
+    out = torch.empty(B, Hq, D, dtype=dtype, device="cuda")
+    need = lib.b200_attn_decode_workspace_bytes(B, Hq, Hkv, S, D)
+    assert need > 0
+    ws = torch.full((need // 4 + 1,), float("nan"), device="cuda")[shift:]   # every partial that is read has been written
+    ok(lib, lib.b200_attn_decode(Q.data_ptr(), K.data_ptr(), V.data_ptr(), M.data_ptr(), out.data_ptr(), B, Hq, Hkv, S, D, Hq * D,
+                                 Hkv * S * D, S * D, S, D ** -0.5, 2, ws.data_ptr(), need, stream()))
+    close(out, ref, rtol=2e-2, atol=5e-3)
+
+
 @pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
 @pytest.mark.parametrize("B", [2, 12])
 def test_attn_decode_small_batches_in_both_dtypes(lib, dtype, B):
