@@ -85,7 +85,11 @@ __global__ void __launch_bounds__(128, STAGES == 2 ? 3 : 2) attn_decode_kernel(c
   const int n_keys = static_cast<int>(s_end - s_begin);
   const int nblk = (n_keys + 15) / 16;
 
-  pdl_trigger();
+  // The successor's start: with clusters of 16 the whole grid is resident, and weight loads that begin here compete with
+  // the keys and values, so it is put off to the end (decode layer of eight sequences 45.3 -> 44.2 us, one sequence
+  // 34.1 -> 33.5); a grid of several waves triggers at once (step of 64 sequences 2.742 ms, at the end 2.755).
+  const bool trigger_late = CM && p.splits == 16;
+  if (!trigger_late) pdl_trigger();
   if (CM) tc5::cluster_sync();   // every CTA of the cluster runs before anyone writes into a peer (overlaps the predecessor)
   pdl_wait();   // q, the new cache rows and the mask come from the kernels before this one
 
@@ -254,6 +258,7 @@ __global__ void __launch_bounds__(128, STAGES == 2 ? 3 : 2) attn_decode_kernel(c
   }
   cp_async_wait<0>();
 
+  if (trigger_late) pdl_trigger();
   // ---- merge the four warps: every warp parks its accumulators (and running max / sum) in the
   // shared memory its own ring occupied; after one barrier thread d adds up dim d of every head ----
 #pragma unroll

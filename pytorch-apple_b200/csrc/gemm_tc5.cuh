@@ -60,6 +60,10 @@ int conv_tc5(const Tc5Args& a, const Tc5Conv& g, cudaStream_t stream);
 // out = epi(A W^T + bias + residual) on the tcgen05 path.  Returns B200_ENOTSUP when the
 // operands do not meet the TMA alignment rules (the caller then uses the mma.sync tiles).
 int linear_tc5(const Tc5Args& a, cudaStream_t stream);
+// The same for a few rows (M <= STREAM_MAX_ROWS), all fused forms included; operands as checked by
+// linear_tc5.  B200_ENOTSUP for shapes that are not whole column blocks and chunks.
+constexpr int STREAM_MAX_ROWS = 12;   // decode step over 4352 rows: 12 sequences 1546 -> 1523 us, 16 sequences 1637 -> 1651 (not taken)
+int linear_stream(const Tc5Args& a, cudaStream_t stream);
 bool tc5_enabled();
 // Scratch bytes linear_tc5 needs for (M, N, K): always 0.
 int64_t linear_tc5_workspace_bytes(int64_t M, int64_t N, int64_t K);

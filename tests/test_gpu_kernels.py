@@ -204,6 +204,41 @@ def test_linear_norm_fused_rmsnorm(lib, M, N, K, mode):
     assert code.value == 0
 
 
+@pytest.mark.parametrize("M", [1, 8, 9, 12, 13])
+@pytest.mark.parametrize("N,K,shift,ldx", [
+    (64, 64, 0, 0),           # one block, one chunk: three of the four warps have none
+    (128, 320, 0, 16),        # five chunks, strided rows
+    (192, 2112, 16, 0),       # eight splits of uneven length; W 32-byte aligned inside its buffer
+    (192, 2112, 8, 0),        # W only 16-byte aligned: the tensor-map kernel
+    (64 * 300, 192, 0, 0),    # more blocks than resident CTAs: a CTA walks two
+    (64 * 150, 25664, 0, 0),  # no split and rows too long to keep: the tensor-map kernel
+    (200, 328, 0, 0),         # ragged block and chunk
+])
+def test_linear_few_rows_edges(lib, M, N, K, shift, ldx):
+    """Edges of the weight-streaming kernel and of its rule; residual, bias and ReLU in the final pass.  The bound: fp32
+    sums in any order (K * 2^-24 of the sum of magnitudes, products exact), and two roundings to bf16
+    (eight significant bits: at most 2^-8 of the value each)."""
+    lda, ldo = K + ldx, N + ldx
+    A = torch.full((M, lda), float("nan"), dtype=torch.bfloat16, device="cuda")
+    A[:, :K] = gen((M, K)).cuda()
+    g = torch.Generator(device="cuda").manual_seed(1)
+    Wb = torch.randn(N * K + shift, generator=g, device="cuda").mul_(K ** -0.5).bfloat16()
+    W = Wb[shift:].view(N, K)
+    b, r = gen((N,), seed=2).cuda(), torch.zeros(M, ldo, dtype=torch.bfloat16, device="cuda")
+    r[:, :N] = gen((M, N), seed=3).cuda()
+    out = torch.full((M, ldo), 7.0, dtype=torch.bfloat16, device="cuda")
+    ws = torch.zeros(1 << 22, dtype=torch.uint8, device="cuda")
+    ok(lib, lib.b200_linear(A.data_ptr(), W.data_ptr(), b.data_ptr(), r.data_ptr(), out.data_ptr(), M, N, K, lda, K, ldo, ldo, 2, 2,
+                            1 | 8, None, 0, ws.data_ptr(), ws.numel(), stream()))
+    x, w = A[:, :K].double(), W.double()
+    lin = x @ w.T + b.double()
+    want = (lin + r[:, :N].double()).clamp(min=0)
+    bound = (x.abs() @ w.abs().T) * (K * 2.0 ** -24) + (lin.abs() + want) * 2.0 ** -8 * 1.01 + 1e-6
+    err = (out[:, :N].double() - want).abs()
+    assert (err <= bound).all(), float((err - bound).max())
+    assert (out[:, N:] == 7.0).all()
+
+
 def test_linear_norm_rejects_shapes_outside_the_fused_kernel(lib):
     t = torch.zeros(128 * 1536, dtype=torch.bfloat16, device="cuda")
     f = torch.zeros(4096, device="cuda")
