@@ -1071,6 +1071,21 @@ class _Lowering:
                               "pad_w": pad[1], "has_bias": a["has_bias"], "groups": 1, "c_pad": Cp, "relu": a["relu"],
                               "bn_folded": a["bn"]}), names + [out.name])
 
+    def _aligned_mask(self, name: str, T: int) -> str:
+        """The mask with rows at multiples of 16 bytes, as tensor maps need them: one copy that all layers of a call
+        share.  A 777-token prompt takes the mma.sync attention otherwise (145 us per layer and call; the tensor-map
+        kernel 27); the copy of its 1.2 MB mask is 7 us once."""
+        v = self.view(name)
+        if len(v.shape) < 2 or v.shape[-2] != T or v.strides[-1] != 1 or (v.offset % 8 == 0 and all(s % 8 == 0 for s in v.strides[:-1])):
+            return name
+        dst = f"{name}__rows16"
+        if dst not in self.out.views:
+            padded = v.shape[:-1] + (-(-v.shape[-1] // 8) * 8,)
+            full = self.alloc(dst, padded, v.dtype)
+            self.out.views[dst] = TensorView(dst, 0, v.shape, full.strides, v.dtype)
+            self.copy(name, dst)
+        return dst
+
     def lower_attention(self, node: OpNode) -> None:
         a = node.attrs
         q, k, v = node.inputs[:3]
@@ -1090,8 +1105,12 @@ class _Lowering:
             ok = qv.strides[1] == D and kv.strides[2] == D and vv.strides[2] == D and tuple(kv.strides) == tuple(vv.strides)
         if not ok:
             return self.lower_original(node)
+        mname = mask.name if mask is not None else None
+        if mask is not None and T > 1:
+            mname = self._aligned_mask(mname, T)
+            mv = V.broadcast_to(self.view(mname), (B, 1, T, S))
         o = self.alloc(out.name, out.shape, dt)
-        names = [q.name, k.name, v.name] + ([mask.name] if mask is not None else [])
+        names = [q.name, k.name, v.name] + ([mname] if mask is not None else [])
         p = {"op": "attention", "q": qv, "k": kv, "v": vv, "mask": mv, "y": o, "scale": a["scale"], "B": B, "Hq": Hq, "Hkv": Hkv,
              "T": T, "S": S, "D": D, "decode": T == 1, "workspace": None}
         if T == 1:

@@ -452,6 +452,26 @@ def test_attn_prefill(lib, B, T):
     assert code.value == 0
 
 
+@pytest.mark.parametrize("B,T,aligned", [(1, 777, True), (1, 777, False), (2, 33, True), (1, 129, True), (1, 65, True)])
+def test_attn_prefill_ragged_lengths(lib, B, T, aligned):
+    """Lengths that are no multiple of eight: mask rows padded to 16 bytes (the tensor-map kernel; the padding is NaN and
+    must not be read as a mask) and dense rows (the mma.sync kernel)."""
+    import model_zoo as mz
+
+    dtype, Hq, Hkv, D = torch.bfloat16, 4, 2, 128
+    q, k, v = gen((B, Hq, T, D), dtype), gen((B, Hkv, T, D), dtype, 1), gen((B, Hkv, T, D), dtype, 2)
+    mask = mz.causal_mask(B, T, T, 0)
+    Tp = -(-T // 8) * 8 if aligned else T
+    M = torch.full((B, 1, T, Tp), float("nan"), dtype=dtype, device="cuda")
+    M[..., :T] = mask.cuda()
+    Q, K, V = q.cuda(), k.cuda(), v.cuda()
+    out = torch.full((B, T, Hq, D), float("nan"), dtype=dtype, device="cuda")
+    st = lambda t: (C.c_int64 * 3)(*t.stride()[:3])
+    ok(lib, lib.b200_attn_prefill(Q.data_ptr(), K.data_ptr(), V.data_ptr(), M.data_ptr(), out.data_ptr(), B, Hq, Hkv, T, T, D,
+                                  st(Q), st(K), st(V), T * Tp, Tp, D ** -0.5, 2, stream()))
+    close(out, attn_ref(q, k, v, mask, D ** -0.5, dtype).transpose(1, 2), rtol=2e-2, atol=5e-3)
+
+
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
 def test_attn_prefill_arbitrary_masks_and_no_mask(lib, dtype):
     """Nothing in the kernels assumes a causal mask: a per-sequence mask with windows, holes and key

@@ -181,6 +181,26 @@ def test_qwen_tiny_golden_prefill_then_decode(fake_native):
     assert fake_native.calls.count("attn_decode") == L and fake_native.calls.count("attn_prefill") == L
 
 
+@pytest.mark.parametrize("B,T", [(1, 13), (2, 9), (1, 16)])
+def test_prefill_mask_rows_are_aligned_once_per_call(fake_native, B, T):
+    """A prompt whose length is no multiple of eight: one copy of the mask with padded rows, read by every layer;
+    an aligned mask is read in place."""
+    from cuda_compiler import compile_subgraph
+    from golden.make_golden import tiny_qwen
+
+    cfg, sd, model = tiny_qwen()
+    ir = extract_ir(mz.QwenPrefillWrapper(model), mz.qwen2_example_inputs(cfg, B, T, None, device="cpu"), "p")
+    ids = torch.randint(0, cfg.vocab_size, (B, T), generator=torch.Generator().manual_seed(0))
+    ins = (ids, mz.causal_mask(B, T, T, 0), torch.arange(T)[None].expand(B, T).contiguous(), torch.arange(T))
+    out, _ = run_backend(ir, mz.state_dict_numpy(sd), np_inputs(ir, ins))
+    name = ir["graph_outputs"][0]["name"]
+    ref = IRInterpreter(ir, sd).execute(dict(zip([s["name"] for s in ir["graph_inputs"]], ins)))[name]
+    assert np.abs(to_f32(out[name]) - ref.float().numpy()).max() < 0.1
+    copies = [st for st in compile_subgraph(ir).steps if getattr(st, "kernel_name", "") == "strided_copy"]
+    assert len(copies) == (0 if T % 8 == 0 else 1)
+    assert fake_native.calls.count("attn_prefill") == cfg.num_hidden_layers
+
+
 def test_mixed_partitions_use_the_injected_cpu_executor(fake_native):
     from cuda_compiler import compile_subgraph
     from cuda_runtime import CUDABackend
