@@ -27,7 +27,7 @@ constexpr int NORM_MAX_PARTS = 32;   // row scaling: at most this many sum-of-sq
 // Kernel modes.
 //   0  compute-bound shapes (several row tiles): two CTAs per SM with a short ring, so that
 //      one CTA's epilogue overlaps the other's main loop;
-//   1  a single row tile with 64 < M <= 128: pure weight streaming, one CTA per SM, deep ring;
+//   1  a single row tile with 64 < M <= 128 (pure weight streaming) and convolutions with few tiles: one CTA per SM, deep ring;
 //   2  M <= 64 (decode): the activation tile is loaded 64 rows high (the MMA still reads 128
 //      rows; the upper half is whatever follows in shared memory and only feeds accumulator
 //      rows that are never stored), which halves the stage size; one CTA per SM with a ring of
@@ -90,8 +90,8 @@ __global__ void __launch_bounds__(224, Cfg<BN, MODE>::CTAS) gemm_tc5_kernel(cons
   const int nstg = (nkb + KPS - 1) / KPS;                // ring stages this CTA fills
   auto stage_cnt = [&](int i) { return nkb - i * KPS < KPS ? nkb - i * KPS : KPS; };   // k-blocks of stage i
   // single-row-tile shapes and split-K stage the accumulator through shared memory (see the end of the kernel)
-  const bool gather = CONV && !p.g.im2col;   // convolution A tile copied by the epilogue warps instead of TMA
-  const bool staged = !CONV && (MODE >= 1 || p.splits > 1);   // MODE >= 1: known at compile time, the direct epilogue is dropped
+  const bool gather = CONV && MODE == 0 && !p.g.im2col;   // convolution A tile copied by the epilogue warps instead of TMA
+  const bool staged = MODE >= 1 || (!CONV && p.splits > 1);   // MODE >= 1: known at compile time, the direct epilogue is dropped
   const bool glu = (p.epilogue & B200_EPI_GLU) != 0;       // host guarantees BN == 128 and N % 128 == 0
   const bool rope = CAN_NORM && BN == 128 && p.rope.cos != nullptr;   // tile = one attention head (host: BN == 128, N % 128 == 0)
   const int rows_valid = static_cast<int>(p.M - m0 < BM ? p.M - m0 : BM);
@@ -194,11 +194,17 @@ __global__ void __launch_bounds__(224, Cfg<BN, MODE>::CTAS) gemm_tc5_kernel(cons
         const int cpb = p.g.C / BK;
         const int img = m0 / (p.g.Ho * p.g.Wo), rem = m0 - img * (p.g.Ho * p.g.Wo), oh = rem / p.g.Wo, ow = rem - oh * p.g.Wo;
         const int base_w = ow * p.g.sw - p.g.pw, base_h = oh * p.g.sh - p.g.ph;
-        int cb = 0, sx = 0, r = 0;
-        drain(produce(0, [&](int, int st) {
-          tc5::mbar_arrive_expect_tx_a(full0 + 8u * st, A_STAGE);
-          tc5::tma_load_im2col_4d_a(ring_addr + st * STAGE, &map_a, full0 + 8u * st, cb * BK, base_w, base_h, img, sx, r);
-          if (++cb == cpb) { cb = 0; if (++sx == p.g.KW) { sx = 0; ++r; } }
+        const int tap = kb0 / cpb;   // (kb0 != 0 with split-K only)
+        int cb = kb0 - tap * cpb, r = tap / p.g.KW, sx = tap - r * p.g.KW;
+        drain(produce(0, [&](int i, int st) {
+          const int cnt = stage_cnt(i);
+          tc5::mbar_arrive_expect_tx_a(full0 + 8u * st, cnt * A_STAGE);
+#pragma unroll
+          for (int j = 0; j < KPS; ++j)
+            if (j < cnt) {
+              tc5::tma_load_im2col_4d_a(ring_addr + st * STAGE + j * A_STAGE, &map_a, full0 + 8u * st, cb * BK, base_w, base_h, img, sx, r);
+              if (++cb == cpb) { cb = 0; if (++sx == p.g.KW) { sx = 0; ++r; } }
+            }
         }));
       }
     }
@@ -1595,6 +1601,27 @@ Tc5Plan plan_tc5(int64_t M, int64_t N, int64_t K, bool glu = false) {
   return plan_for_bn(128, M, N, K);
 }
 
+// Convolutions with fewer 64-wide tiles than SMs (all layers of one image, the late ones of small batches): the k-blocks
+// of a tile are split over a cluster of up to eight CTAs, and the staged epilogue writes whole rows with every thread
+// even where nothing is left to split.  One 128-wide tile per CTA, each walking all taps, left four CTAs to the 7x7
+// layers: one image, in a graph, us before -> after: 3x3 with 128 / 256 / 512 channels 12.5 -> 6.2, 17.9 -> 6.5, 28.4 ->
+// 6.6; 1x1 2048 -> 512 at 7x7 16.0 -> 5.1, 512 -> 2048 with residual 12.7 -> 5.0; all 53 layers 568 -> 300, four images
+// 548 -> 356.  (Fetching the weights ahead of the predecessor changed nothing: they are in L2.)
+Tc5Plan plan_conv_split(int64_t M, int64_t N, int64_t K) {
+  Tc5Plan pl;
+  pl.bn = 64;
+  pl.tiles_n = ceil_div(N, 64);
+  pl.tiles_m = ceil_div(M, BM);
+  const int64_t KB = K / BK;
+  int64_t splits = SPLIT_TARGET_CTAS / (pl.tiles_n * pl.tiles_m);
+  if (splits > KB / SPLIT_MIN_KB) splits = KB / SPLIT_MIN_KB;
+  if (splits > MAX_SPLITS) splits = MAX_SPLITS;
+  if (splits < 1) splits = 1;
+  pl.kb_per_split = static_cast<int>(ceil_div(KB, splits));
+  pl.splits = static_cast<int>(ceil_div(KB, pl.kb_per_split));
+  return pl;
+}
+
 template <typename T, int BN, bool CONV, int MODE = 0>
 int launch(const Tc5Args& a, const Tc5Plan& plan, cudaStream_t st, const Tc5Conv* g = nullptr) {
   Tc5Plan pl = plan;
@@ -1647,6 +1674,7 @@ int launch(const Tc5Args& a, const Tc5Plan& plan, cudaStream_t st, const Tc5Conv
   p.g = g ? *g : Tc5Conv{};
   if (CONV) {
     p.g.im2col = make_im2col_map(&ma, a.A, p.g, a.dtype) ? 1 : 0;
+    if (!p.g.im2col && MODE > 0) return B200_ENOTSUP;
     if (!p.g.im2col) ma = mw;   // unused: the epilogue warps gather the A tile
   } else if (!make_map(&ma, a.A, a.M, a.K, a.lda, Cfg<BN, MODE>::AROWS, a.dtype)) {
     return B200_ENOTSUP;
@@ -1658,7 +1686,7 @@ int launch(const Tc5Args& a, const Tc5Plan& plan, cudaStream_t st, const Tc5Conv
   if ((a.sumsq_in || a.sumsq_out) && (CONV || MODE < 2)) return B200_ENOTSUP;
   p.rope = a.rope;
   if (a.rope.cos && (CONV || MODE < 2 || BN != 128 || a.N % 128)) return B200_ENOTSUP;
-  if (CONV && pl.splits != 1) return B200_ENOTSUP;
+  if (CONV && MODE == 0 && pl.splits != 1) return B200_ENOTSUP;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(static_cast<unsigned>(pl.tiles_n), static_cast<unsigned>(pl.tiles_m), static_cast<unsigned>(pl.splits));
   cfg.blockDim = dim3(224);
@@ -2032,6 +2060,11 @@ int conv_tc5(const Tc5Args& a, const Tc5Conv& g, cudaStream_t st) {
   }
   if (g.C % BK || a.K != static_cast<int64_t>(g.KH) * g.KW * g.C || a.ldw % 8 || !aligned16(a.A) || !aligned16(a.W)) return B200_ENOTSUP;
   if (const int bn = persistent_bn(a.M, a.N, a.K, false, a.residual != nullptr)) return dispatch_persistent<true>(bn, a, st, &g);
+  {   // fewer tiles than SMs; falls through without an im2col map
+    const Tc5Plan sp = plan_conv_split(a.M, a.N, a.K);
+    const int rc = a.dtype == B200_BF16 ? launch<__nv_bfloat16, 64, true, 1>(a, sp, st, &g) : launch<__half, 64, true, 1>(a, sp, st, &g);
+    if (rc != B200_ENOTSUP) return rc;
+  }
   Tc5Plan pl;
   pl.bn = a.N >= 128 ? 128 : 64;
   pl.tiles_n = ceil_div(a.N, pl.bn);

@@ -293,6 +293,11 @@ def test_linear_rejects_unaligned(lib):
     (16, 128, 28, 256, 1, 1, 0, True, True),   # 128-wide tiles, two column tiles, residual
     (52, 256, 28, 64, 1, 1, 0, False, False),  # resident weights with four k-blocks per tile, ragged last tile
     (41, 128, 28, 512, 1, 1, 0, True, True),   # column tiles fastest: each CTA keeps one of four column tiles, ragged last row tile
+    (1, 64, 56, 256, 1, 1, 0, True, True),     # few tiles, nothing to split: one k-block, the staged epilogue
+    (1, 2048, 7, 512, 1, 1, 0, False, True),   # few tiles, taps split eight ways (four k-blocks each), 49 rows
+    (2, 512, 14, 512, 3, 2, 1, False, True),   # 72 k-blocks over eight CTAs: a split starts inside a filter tap
+    (3, 192, 9, 72, 3, 2, 1, True, False),     # 27 k-blocks in uneven splits, output channels past a whole tile
+    (1, 128, 56, 130, 1, 2, 0, False, True),   # output rows without 8-byte alignment
     (37, 256, 14, 1024, 1, 1, 0, True, False), # column tiles fastest with eight column tiles (grid trimmed to a multiple of 8)
 ])
 def test_conv2d_nhwc(lib, N, C, H, O, k, s, p, res, relu):
