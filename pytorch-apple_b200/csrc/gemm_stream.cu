@@ -1,4 +1,4 @@
-// Weight-streaming GEMM for a few rows (decode):  out[M,N] = epi(A[M,K] * W[N,K]^T + bias + residual), M <= 12.
+// Weight-streaming GEMM for a few rows (decode):  out[M,N] = epi(A[M,K] * W[N,K]^T + bias + residual), M <= 24.
 //
 // With a handful of rows the weights are the work: every byte of W is read once and nothing else matters as long
 // as enough of them are in flight, from before the predecessor has finished until the last one has arrived.
@@ -21,7 +21,9 @@
 //    1 row    6.3 ->  4.0    5.0 ->  3.1   13.3 ->  9.6    9.3 ->  7.2   vocabulary (467 MB) 105 -> 74 (6.3 TB/s)
 //    8 rows   6.6 ->  4.7    5.4 ->  3.5   12.8 -> 10.5    9.8 ->  7.7                       100 -> 76
 //   16 rows   7.7 ->  6.0    5.4 ->  4.0   13.4 -> 13.5    9.8 ->  9.3                        99 -> 84
-// From about 12 rows on the activation words of a chunk outweigh the rest and the tensor-map kernel is the faster one.
+// The activations of a CTA's K range stay in shared memory, which bounds the rows that two CTAs per SM can take: 16 for
+// a 1536-wide unsplit row, 24 where K is split (q/k/v and output projection at 19 rows 7.4 -> 6.1 and 5.4 -> 4.1 us); wider
+// unsplit rows and more sequences stay with the tensor-map kernel (gate/up at 19 rows: 13.1 there, 22 here).
 // Measured and not used: the same loop on a cp.async ring (paced by shared-memory traffic and waits: 28.9 against 24.6 us
 // per layer), prefetching a later part of the weights into L2 (every form slower, by up to 13 us per layer).
 #include "gemm_epilogue.cuh"
@@ -33,7 +35,8 @@ namespace {
 constexpr int SW_COLS = 64, SW_WARPS = 4, SW_THREADS = SW_WARPS * 32, SW_CHUNK = 64, SW_PITCH = SW_COLS + 4;
 constexpr int SW_STRIDE = SW_WARPS * SW_CHUNK;   // k from one chunk of a warp to its next
 constexpr int SW_DEPTH = 2;                      // weight chunks in flight per warp
-constexpr int SW_SMEM_MAX = 110 * 1024;          // two CTAs per SM
+constexpr int SW_CARVEOUT = 60;                  // percent of the 228 KB, see launch_stream
+constexpr int SW_SMEM_MAX = 66 * 1024;           // two CTAs in that share (1 KB each is the system's)
 
 template <int NT> struct SwCfg {   // NT = groups of 8 rows
   static constexpr int ROWS = NT * 8;
@@ -342,7 +345,11 @@ template <typename T, int NT> int launch_stream(const Tc5Args& a, cudaStream_t s
   bool* configured = configured_on.slot();
   if (!configured) return B200_ENOTSUP;
   if (!*configured) {
-    if (cudaFuncSetAttribute(gemm_stream_kernel<T, NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, SW_SMEM_MAX) != cudaSuccess) {
+    // The loads in flight land in L1, so shared memory must not take all of an SM (layer of one row 24.6 us at 60 %, 25.5 at
+    // 80, 32.9 at 100); left to itself the driver takes the least that fits, and then every SM is reconfigured between
+    // this kernel and the attention (layer of eight rows with its attention 44.1 us by default, 36.6 at 60 %).
+    if (cudaFuncSetAttribute(gemm_stream_kernel<T, NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, SW_SMEM_MAX) != cudaSuccess ||
+        cudaFuncSetAttribute(gemm_stream_kernel<T, NT>, cudaFuncAttributePreferredSharedMemoryCarveout, SW_CARVEOUT) != cudaSuccess) {
       cudaGetLastError();
       return B200_ENOTSUP;
     }
@@ -386,7 +393,7 @@ template <typename T, int NT> int launch_stream(const Tc5Args& a, cudaStream_t s
 }
 
 template <typename T> int dispatch_stream(const Tc5Args& a, cudaStream_t st) {
-  return a.M <= 8 ? launch_stream<T, 1>(a, st) : launch_stream<T, 2>(a, st);
+  return a.M <= 8 ? launch_stream<T, 1>(a, st) : a.M <= 16 ? launch_stream<T, 2>(a, st) : launch_stream<T, 3>(a, st);
 }
 
 }  // namespace

@@ -61,8 +61,8 @@ int conv_tc5(const Tc5Args& a, const Tc5Conv& g, cudaStream_t stream);
 // operands do not meet the TMA alignment rules (the caller then uses the mma.sync tiles).
 int linear_tc5(const Tc5Args& a, cudaStream_t stream);
 // The same for a few rows (M <= STREAM_MAX_ROWS), all fused forms included; operands as checked by
-// linear_tc5.  B200_ENOTSUP for shapes that are not whole column blocks and chunks.
-constexpr int STREAM_MAX_ROWS = 12;   // decode step over 4352 rows: 12 sequences 1546 -> 1523 us, 16 sequences 1637 -> 1651 (not taken)
+// linear_tc5.  B200_ENOTSUP for shapes that are not whole column blocks and chunks or whose activations do not fit.
+constexpr int STREAM_MAX_ROWS = 24;
 int linear_stream(const Tc5Args& a, cudaStream_t stream);
 bool tc5_enabled();
 // Scratch bytes linear_tc5 needs for (M, N, K): always 0.

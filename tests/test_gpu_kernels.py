@@ -204,7 +204,7 @@ def test_linear_norm_fused_rmsnorm(lib, M, N, K, mode):
     assert code.value == 0
 
 
-@pytest.mark.parametrize("M", [1, 8, 9, 12, 13])
+@pytest.mark.parametrize("M", [1, 8, 9, 16, 17, 24, 25])
 @pytest.mark.parametrize("N,K,shift,ldx", [
     (64, 64, 0, 0),           # one block, one chunk: three of the four warps have none
     (128, 320, 0, 16),        # five chunks, strided rows
@@ -212,6 +212,7 @@ def test_linear_norm_fused_rmsnorm(lib, M, N, K, mode):
     (192, 2112, 8, 0),        # W only 16-byte aligned: the tensor-map kernel
     (64 * 300, 192, 0, 0),    # more blocks than resident CTAs: a CTA walks two
     (64 * 150, 25664, 0, 0),  # no split and rows too long to keep: the tensor-map kernel
+    (64 * 150, 1536, 0, 0),   # no split: two groups of rows fit beside a second CTA, three do not
     (200, 328, 0, 0),         # ragged block and chunk
 ])
 def test_linear_few_rows_edges(lib, M, N, K, shift, ldx):
