@@ -160,10 +160,18 @@ __global__ void __launch_bounds__(480, 1)
               for (int e = 0; e < 8; ++e) any = any || f[e] > MASKED_F;
             }
         } else {
-          for (int q = 0; q < 4; ++q)
-            if (lane + 32 * q < rows_valid)
-              for (int e = 0; e < BKV; ++e)
-                if (key0 + e < p.S && to_f32<T>(m0[static_cast<int64_t>(lane + 32 * q) * p.mask_t + key0 + e]) > MASKED_F) any = true;
+          // the ragged last tile: sixteen predicated loads in flight (one after the other, nine keys of four rows were 20 us)
+          for (int q = 0; q < 4; ++q) {
+            const T* src = m0 + static_cast<int64_t>(lane + 32 * q) * p.mask_t + key0;
+            const int cnt = lane + 32 * q < rows_valid ? static_cast<int>(p.S - key0) : 0;
+            for (int e0 = 0; e0 < cnt; e0 += 16) {
+              float f[16];
+#pragma unroll
+              for (int e = 0; e < 16; ++e) f[e] = e0 + e < cnt ? to_f32<T>(src[e0 + e]) : -INFINITY;
+#pragma unroll
+              for (int e = 0; e < 16; ++e) any = any || f[e] > MASKED_F;
+            }
+          }
         }
         const bool valid = __ballot_sync(0xffffffffu, any) != 0u;
         if (lane == 0) *reinterpret_cast<volatile uint8_t*>(&s_flag[j]) = valid ? 1 : 2;
@@ -403,7 +411,7 @@ int launch_prefill_tc5(const PrefillParams& p, int dtype, cudaStream_t st) {
   mm = mq;
   if (p.mask) {
     const uint64_t dims[3] = {static_cast<uint64_t>(p.S), static_cast<uint64_t>(p.T), static_cast<uint64_t>(p.mask_b == 0 ? 1 : p.B)};
-    const uint64_t str[2] = {st_of(p.mask_t, static_cast<uint64_t>(p.S) * 2), st_of(p.mask_b, static_cast<uint64_t>(p.S) * 2)};
+    const uint64_t str[2] = {static_cast<uint64_t>(p.mask_t) * 2, st_of(p.mask_b, static_cast<uint64_t>(p.mask_t) * 2)};
     const uint32_t box[3] = {64, BQ, 1};
     if (!tma_encode_sw128(&mm, dtype, 3, p.mask, dims, str, box)) return B200_ENOTSUP;
   }

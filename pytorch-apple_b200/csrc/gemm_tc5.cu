@@ -2014,6 +2014,18 @@ int linear_tc5(const Tc5Args& a, cudaStream_t st) {
     return a.dtype == B200_BF16 ? launch<__nv_bfloat16, 128, false, 2>(a, pl, st) : launch<__half, 128, false, 2>(a, pl, st);
   }
   if (const int rc = linear_stream(a, st); rc != B200_ENOTSUP) return rc;
+  // One wave of 128 x 128 tiles where 64-wide tiles would need a second one (reductions of 1024..4095, which the pair
+  // kernel does not split): with a residual on the persistent kernel (residual tile and result are bulk copies), else on
+  // the one-tile kernel.  us before -> after: q/k/v projection (N 2048) 777 tokens 17.4 -> 11.3, 1152 tokens 17.3 -> 12.2;
+  // output projection (N 1536, residual) 777 tokens 16.0 -> 10.9, 1500 16.7 -> 11.7; 1x1 convolution 1024 -> 256 of 32
+  // images 12.5 -> 8.9.  (Kernels the other way round: 13.0 and 16.3 at 777.  Fewer tiles: a prompt of 512 tokens with its
+  // 48 output-projection tiles on the persistent kernel takes 2979 instead of 2923 us.)
+  if (const int64_t tm = ceil_div(a.M, BM); tm > 1 && a.K >= 1024 && a.K < 4096 && !glu && tm * ceil_div(a.N, 128) < 148 &&
+                                            tm * ceil_div(a.N, 64) > 148) {
+    if (a.residual) return dispatch_persistent<false>(128, a, st, nullptr);
+    const Tc5Plan pl = plan_for_bn(128, a.M, a.N, a.K);
+    return a.dtype == B200_BF16 ? launch<__nv_bfloat16, 128, false, 1>(a, pl, st) : launch<__half, 128, false, 1>(a, pl, st);
+  }
   if (pair_shape(a)) {
     const int rc = a.dtype == B200_BF16 ? launch_pair<__nv_bfloat16>(a, st) : launch_pair<__half>(a, st);
     if (rc != B200_ENOTSUP) return rc;

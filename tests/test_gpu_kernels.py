@@ -48,6 +48,10 @@ def close(got, ref, rtol=2e-2, atol=1e-2):
 # ------------------------------------------------------------------ linear
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
 @pytest.mark.parametrize("M,N,K,bias,res,relu,silu", [
+    (777, 2048, 1536, True, False, False, False),   # one wave of 128-wide tiles, ragged last row tile
+    (777, 1536, 1536, False, True, False, False),   # the same with a residual
+    (1537, 700, 1032, True, True, True, False),     # ragged columns and k
+    (900, 1400, 1096, True, False, False, True),
     (1, 1536, 1536, True, False, False, False),
     (1, 1536, 8960, False, True, False, False),
     (8, 8960, 1536, False, False, False, True),
@@ -458,7 +462,7 @@ def test_attn_prefill(lib, B, T):
     assert code.value == 0
 
 
-@pytest.mark.parametrize("B,T,aligned", [(1, 777, True), (1, 777, False), (2, 33, True), (1, 129, True), (1, 65, True)])
+@pytest.mark.parametrize("B,T,aligned", [(1, 777, True), (2, 100, "shared"), (1, 777, False), (2, 33, True), (1, 129, True), (1, 65, True)])
 def test_attn_prefill_ragged_lengths(lib, B, T, aligned):
     """Lengths that are no multiple of eight: mask rows padded to 16 bytes (the tensor-map kernel; the padding is NaN and
     must not be read as a mask) and dense rows (the mma.sync kernel)."""
@@ -466,15 +470,16 @@ def test_attn_prefill_ragged_lengths(lib, B, T, aligned):
 
     dtype, Hq, Hkv, D = torch.bfloat16, 4, 2, 128
     q, k, v = gen((B, Hq, T, D), dtype), gen((B, Hkv, T, D), dtype, 1), gen((B, Hkv, T, D), dtype, 2)
-    mask = mz.causal_mask(B, T, T, 0)
+    shared = aligned == "shared"   # one mask for all sequences: a batch stride of zero
+    mask = mz.causal_mask(1 if shared else B, T, T, 0)
     Tp = -(-T // 8) * 8 if aligned else T
-    M = torch.full((B, 1, T, Tp), float("nan"), dtype=dtype, device="cuda")
+    M = torch.full((1 if shared else B, 1, T, Tp), float("nan"), dtype=dtype, device="cuda")
     M[..., :T] = mask.cuda()
     Q, K, V = q.cuda(), k.cuda(), v.cuda()
     out = torch.full((B, T, Hq, D), float("nan"), dtype=dtype, device="cuda")
     st = lambda t: (C.c_int64 * 3)(*t.stride()[:3])
     ok(lib, lib.b200_attn_prefill(Q.data_ptr(), K.data_ptr(), V.data_ptr(), M.data_ptr(), out.data_ptr(), B, Hq, Hkv, T, T, D,
-                                  st(Q), st(K), st(V), T * Tp, Tp, D ** -0.5, 2, stream()))
+                                  st(Q), st(K), st(V), 0 if shared else T * Tp, Tp, D ** -0.5, 2, stream()))
     close(out, attn_ref(q, k, v, mask, D ** -0.5, dtype).transpose(1, 2), rtol=2e-2, atol=5e-3)
 
 
