@@ -74,7 +74,7 @@ __global__ void __launch_bounds__(480, 1)
   uint8_t* q_s = smem;
   uint8_t* st_s = smem + Q_BYTES;
   uint8_t* p_s = st_s + NST * STAGE;
-  __shared__ __align__(8) uint64_t q_full, kv_full[NST], kv_empty[NST], s_full[2], p_ready, o_full;
+  __shared__ __align__(8) uint64_t q_full, kv_full[NST], kv_empty[NST], s_full[2], p_ready[2], o_full[2];
   __shared__ uint32_t tmem_holder;
   __shared__ uint8_t s_flag[MAX_TILES];   // per key tile: 0 not scanned yet, 1 to be processed, 2 fully masked for these rows
   __shared__ float s_max[2][2][BQ];   // [tile parity][half][row]: the halves' maxima of a tile
@@ -98,8 +98,10 @@ __global__ void __launch_bounds__(480, 1)
     for (int s = 0; s < NST; ++s) { tc5::mbar_init(&kv_full[s], 2); tc5::mbar_init(&kv_empty[s], 1); }
     tc5::mbar_init(&s_full[0], 1);
     tc5::mbar_init(&s_full[1], 1);
-    tc5::mbar_init(&p_ready, 256);
-    tc5::mbar_init(&o_full, 1);
+    tc5::mbar_init(&p_ready[0], 256);
+    tc5::mbar_init(&p_ready[1], 256);
+    tc5::mbar_init(&o_full[0], 1);
+    tc5::mbar_init(&o_full[1], 1);
     tc5::fence_barrier_init();
     tc5::prefetch_tensormap(&map_q);
     tc5::prefetch_tensormap(&map_k);
@@ -238,7 +240,7 @@ __global__ void __launch_bounds__(480, 1)
         // the next tile's scores are computed while the softmax warps work on this one
         const int nxt = next_tile(cur + 1);
         if (nxt == -2 || (nxt >= 0 && !issue_s(n + 1))) { failed = 1; atomicExch(&g_tc5_error, 33); break; }
-        if (!tc5::mbar_wait(&p_ready, n & 1)) { failed = 1; atomicExch(&g_tc5_error, 34); break; }
+        if (!tc5::mbar_wait(&p_ready[n & 1], (n >> 1) & 1)) { failed = 1; atomicExch(&g_tc5_error, 34); break; }
         tc5::tc_fence_after();
         const int st = n % NST;
         const uint32_t v_addr = tc5::smem_addr(st_s + st * STAGE) + K_BYTES;
@@ -248,7 +250,7 @@ __global__ void __launch_bounds__(480, 1)
           const uint64_t db = tc5::umma_desc_sw128_mn(v_addr + k * 2048, BKV * 128, 1024);
           tc5::umma_f16(tm_o, da, db, idesc_o, (n | k) != 0);
         }
-        tc5::umma_commit(&o_full);
+        tc5::umma_commit(&o_full[n & 1]);
         tc5::umma_commit(&kv_empty[st]);
         cur = nxt;
       }
@@ -315,10 +317,9 @@ __global__ void __launch_bounds__(480, 1)
       const float alpha = ex2(m_run - m_use);   // exactly 1 while the max stands; 0 for the first tile
       // Some row's max moved: rescale this warp's half of the 32 rows of O, once the previous product
       // has finished.  (That wait is skipped otherwise: the probabilities are double-buffered, and
-      // S of this tile being complete means the product before the previous one is, so the barrier
-      // is never more than one phase behind when it is looked at again.)
+      // S of this tile being complete means the product before the previous one is.)
       if (n > 0 && __any_sync(0xffffffffu, alpha != 1.f)) {
-        if (!wait_all(&o_full, (n - 1) & 1, 36)) { alive = false; break; }
+        if (!wait_all(&o_full[(n - 1) & 1], ((n - 1) >> 1) & 1, 36)) { alive = false; break; }
         tc5::tc_fence_after();
         {
 #pragma unroll
@@ -347,7 +348,10 @@ __global__ void __launch_bounds__(480, 1)
       }
       tc5::fence_proxy_async();   // the probabilities are read by the tensor core (async proxy)
       tc5::tc_fence_before();     // this thread's tcgen05.ld / st are complete before S and O are touched again
-      mbar_arrive1(&p_ready);
+      // Two barriers in turn, here and for the products: a quarter of the rows that need not rescale may be done with tile
+      // n + 1 (its scores are there already) before another is done with tile n.  On one barrier its arrivals would count
+      // for tile n, and at the end it would take product N - 3 for product N - 1.
+      mbar_arrive1(&p_ready[n & 1]);
       l_run = l_run * alpha + ((sum[0] + sum[1]) + (sum[2] + sum[3]));
       m_run = m_new;
     }
@@ -356,7 +360,7 @@ __global__ void __launch_bounds__(480, 1)
     s_sum[half][r] = l_run;
     asm volatile("bar.sync %0, 64;" ::"r"(1 + quarter) : "memory");
     const float l_all = l_run + s_sum[half ^ 1][r];
-    if (alive && N > 0) alive = wait_all(&o_full, (N - 1) & 1, 37);
+    if (alive && N > 0) alive = wait_all(&o_full[(N - 1) & 1], ((N - 1) >> 1) & 1, 37);
     if (alive) {
       tc5::tc_fence_after();
       const float inv = l_all > 0.f ? 1.f / l_all : 0.f;   // a row whose mask admits no key gives zeros

@@ -483,6 +483,36 @@ def test_attn_prefill_ragged_lengths(lib, B, T, aligned):
     close(out, attn_ref(q, k, v, mask, D ** -0.5, dtype).transpose(1, 2), rtol=2e-2, atol=5e-3)
 
 
+@pytest.mark.parametrize("S", [64, 128, 192, 2048, 4032])
+@pytest.mark.parametrize("slow", [0, 1, 2, 3])
+def test_attn_prefill_row_quarters_out_of_step(lib, slow, S):
+    """The four groups of 32 query rows that share a tile are not kept in step: here one of them has to rescale its sums
+    in every key tile (its scores rise along the keys) and the others never (their largest score is the first key's), so
+    that they run ahead by as much as the barriers let them.  The bound: probabilities and outputs rounded to bf16
+    (eight significant bits: 2^-8 of the magnitudes that are added up, and of the result), the rest is fp32."""
+    dtype, B, Hq, Hkv, T, D = torch.bfloat16, 1, 16, 4, 128, 128
+    q, k, v = gen((B, Hq, T, D), dtype, 0, 0.3), gen((B, Hkv, S, D), dtype, 1, 0.3), gen((B, Hkv, S, D), dtype, 2)
+    rows = torch.arange(T) // 32 == slow
+    q[..., :2] = 0
+    q[:, :, rows, 0] = 8.0
+    q[:, :, ~rows, 1] = 8.0
+    k[..., 0] = (torch.arange(S) // 64) * 0.25      # + 0.18 per key tile in the exponent
+    k[..., 1] = 0
+    k[:, :, 0, 1] = 6.0                             # 4.2 above the others
+    Q, K, V = q.cuda(), k.cuda(), v.cuda()
+    st = lambda t: (C.c_int64 * 3)(*t.stride()[:3])
+    s = (q.double() @ k.double().repeat_interleave(Hq // Hkv, 1).transpose(2, 3)) * D ** -0.5
+    p = s.softmax(-1)
+    vd = v.double().repeat_interleave(Hq // Hkv, 1)
+    want, size = (p @ vd).transpose(1, 2), (p @ vd.abs()).transpose(1, 2)
+    for _ in range(3):
+        out = torch.full((B, T, Hq, D), float("nan"), dtype=dtype, device="cuda")
+        ok(lib, lib.b200_attn_prefill(Q.data_ptr(), K.data_ptr(), V.data_ptr(), None, out.data_ptr(), B, Hq, Hkv, T, S, D,
+                                      st(Q), st(K), st(V), 0, 0, D ** -0.5, 2, stream()))
+        err = (out.double().cpu() - want).abs()
+        assert (err <= (size + want.abs()) * 2.0 ** -8 * 1.01 + 1e-5).all(), float(err.max())
+
+
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
 def test_attn_prefill_arbitrary_masks_and_no_mask(lib, dtype):
     """Nothing in the kernels assumes a causal mask: a per-sequence mask with windows, holes and key
