@@ -133,22 +133,20 @@ __global__ void __launch_bounds__(SW_THREADS, 2) gemm_stream_kernel(const __grid
     }
   }
 
-  if (e.sumsq_in) {   // RMSNorm factor of the input rows; needed in the final pass only
-    for (int m = threadIdx.x >> 2; m < M; m += SW_THREADS / 4) {
-      const float* sp = e.sumsq_in + static_cast<int64_t>(m) * e.sumsq_in_cols;
-      float ss = 0.f;
-      for (int j0 = threadIdx.x & 3; j0 < e.sumsq_in_cols; j0 += 32) {   // eight loads in flight
-        float v[8];
+  // RMSNorm factor of the input rows, needed in the final pass only: the four lanes of a quad request the partials of a row
+  // together, then add them up in index order, as the tensor-map kernel does.  (Decode step of eight sequences, us: 1128;
+  // a sum per lane and two exchanges, in another order, 1137; a thread per row with all loads of its own 1371.)
+  static_assert(STREAM_MAX_ROWS <= SW_THREADS / 4 && NORM_MAX_PARTS % 4 == 0, "a quad per row");
+  if (const int m = threadIdx.x >> 2; e.sumsq_in && m < M) {
+    const float* sp = e.sumsq_in + static_cast<int64_t>(m) * e.sumsq_in_cols + t;
+    float v[NORM_MAX_PARTS / 4];
 #pragma unroll
-        for (int j = 0; j < 8; ++j) v[j] = j0 + 4 * j < e.sumsq_in_cols ? __ldcg(sp + j0 + 4 * j) : 0.f;
+    for (int j = 0; j < NORM_MAX_PARTS / 4; ++j) v[j] = 4 * j + t < e.sumsq_in_cols ? __ldcg(sp + 4 * j) : 0.f;
+    const unsigned quad = 0xfu << (lane & 28);
+    float ss = 0.f;
 #pragma unroll
-        for (int j = 0; j < 8; ++j) ss += v[j];
-      }
-      const unsigned quad = 0xfu << (lane & 28);
-      ss += __shfl_xor_sync(quad, ss, 1);
-      ss += __shfl_xor_sync(quad, ss, 2);
-      if ((threadIdx.x & 3) == 0) s_rinv[m] = 1.0f / sqrtf(ss / static_cast<float>(e.K) + e.norm_eps);
-    }
+    for (int j = 0; j < NORM_MAX_PARTS; ++j) ss += __shfl_sync(quad, v[j >> 2], (lane & 28) + (j & 3));
+    if (t == 0) s_rinv[m] = 1.0f / sqrtf(ss / static_cast<float>(e.K) + e.norm_eps);
   }
   // The final pass: a warp per row, a lane two of its 64 columns (2 lane, 2 lane + 1; gated / rotary: lane and its other
   // half).  It runs once per CTA, so what it costs is instructions fetched: one pair per lane is the shortest code.

@@ -23,7 +23,6 @@ __device__ int g_tc5_error = 0;
 namespace {
 
 constexpr int BM = 128, BK = 64;
-constexpr int NORM_MAX_PARTS = 32;   // row scaling: at most this many sum-of-squares partials per row
 // Kernel modes.
 //   0  compute-bound shapes (several row tiles): two CTAs per SM with a short ring, so that
 //      one CTA's epilogue overlaps the other's main loop;

@@ -63,6 +63,7 @@ int linear_tc5(const Tc5Args& a, cudaStream_t stream);
 // The same for a few rows (M <= STREAM_MAX_ROWS), all fused forms included; operands as checked by
 // linear_tc5.  B200_ENOTSUP for shapes that are not whole column blocks and chunks or whose activations do not fit.
 constexpr int STREAM_MAX_ROWS = 24;
+constexpr int NORM_MAX_PARTS = 32;   // row scaling: at most this many sum-of-squares partials per row
 int linear_stream(const Tc5Args& a, cudaStream_t stream);
 bool tc5_enabled();
 // Scratch bytes linear_tc5 needs for (M, N, K): always 0.

@@ -257,6 +257,34 @@ def test_linear_norm_rejects_shapes_outside_the_fused_kernel(lib):
 def test_bounded_wait_runs_out_and_the_context_survives(lib):
     """A barrier wait that can never be satisfied: the kernel's bounded wait gives up after the probe limit,
     leaves code 99 in the device error word and returns; the next kernels run normally."""
+@pytest.mark.parametrize("M", [1, 9, 24, 25, 64])
+def test_row_scale_adds_its_partials_in_index_order(lib, M):
+    """Every kernel behind b200_linear_norm adds the sum-of-squares partials of a row in index order: 2^24 and then ones
+    is 2^24 that way, and up to 2^24 + 24 in any other (two sums of eight ones and more survive the rounding).  An fp32
+    bias takes the product with the right factor away again, so what is left is the factor's error: a few roundings of
+    2^-24 against 2^-20.4 for the other order."""
+    N, K, parts = 2048, 1536, 32
+    ss = torch.ones(M, parts)
+    ss[:, 0] = 2.0 ** 24
+    ss *= (4.0 ** (torch.arange(M) % 3))[:, None]
+    total = ss[:, 0]                                   # the ones vanish one by one
+    for j in range(1, parts):
+        assert (total + ss[:, j] == total).all()
+    x = torch.zeros(M, K)
+    x[:, 0] = total.div(K).sqrt().bfloat16().float()   # one product per output: its sum is exact in any order
+    w = torch.zeros(N, K)
+    w[:, 0] = gen((N,), seed=3).float()
+    prod = x[:1, 0] * w[:, 0]                          # the bias is shared by the rows, so they all get the first row's product
+    x[:, 0] = x[0, 0] * 2.0 ** (torch.arange(M) % 3)
+    rinv = 1.0 / torch.sqrt(total / K + 1e-6)
+    bias = -(prod * rinv[0])
+    X, W, B, SQ = x.bfloat16().cuda(), w.bfloat16().cuda(), bias.cuda(), ss.cuda()
+    out = torch.full((M, N), float("nan"), dtype=torch.bfloat16, device="cuda")
+    ok(lib, lib.b200_linear_norm(X.data_ptr(), W.data_ptr(), B.data_ptr(), None, out.data_ptr(), M, N, K, K, K, N, 0, 2, 0, 8, 1e-6,
+                                 SQ.data_ptr(), parts, None, stream()))
+    assert (out.float().cpu().abs() <= prod.mul(rinv[0]).abs() * 2.0 ** -22).all()
+
+
     code = C.c_int(-1)
     ok(lib, lib.b200_debug_device_error(C.byref(code), 1))
     assert code.value == 0
