@@ -324,34 +324,34 @@ __global__ void __launch_bounds__(128, STAGES == 2 ? 3 : 2) attn_decode_kernel(c
   }
 }
 
-// Adds up the splits' partial results.  grid = (B*Hq, HD / 32), 256 threads: thread (grp = tid / 8, c4 = tid % 8)
-// owns 4 of the block's 32 dims and every 32nd split, so a 32768-row cache (256 splits) costs a thread eight
-// independent loads; the 32 groups then meet in shared memory.  Bound by the latency of an L2 round trip: 12
-// blocks of one thread per dim, each walking all splits, made the decode step of one sequence over a 32768-row
-// cache with 20000 rows filled 2171 us; this way it takes 1390 us (28 us less per layer).
-constexpr int MRG_GROUPS = 32, MRG_DIMS = 32, MRG_PITCH = MRG_DIMS + 4;
-template <typename T>
-__global__ void __launch_bounds__(256) attn_decode_merge_kernel(const float* __restrict__ part_acc, const float* __restrict__ part_ml,
+// Adds up the splits' partial results.  grid = (B*Hq, HD / DIMS), GROUPS * DIMS / 4 threads: thread (grp, c4) owns 4 of
+// the block's dims and every GROUPS-th split, BATCH of them in flight together; the groups then meet in shared memory.
+// Bound by the latency of an L2 round trip, and by the blocks where there are many heads.  Attention and merge, us:
+// - Many splits (32, 32, 8): a 32768-row cache (256 splits) costs a thread eight independent loads.  One sequence with 20480
+//   rows filled: one thread per dim, each walking all splits, 37.7; this 10.6; one block per head (4, HD, 8) 14.7.
+// - Few splits (4, HD, 4), one block per head: 64 sequences over 448 rows 11.7, over 64 rows 5.6, one over 448 rows 4.5.  With
+//   most of its groups idle the other form costs more than the attention itself (23.2, 17.3, 5.4).
+template <typename T, int GROUPS, int DIMS, int BATCH>
+__global__ void __launch_bounds__(GROUPS * DIMS / 4) attn_decode_merge_kernel(const float* __restrict__ part_acc, const float* __restrict__ part_ml,
                                                                 T* __restrict__ out, int Hq, int Hkv, int G, int splits) {
-  __shared__ __align__(16) float s_acc[MRG_GROUPS][MRG_PITCH];
-  __shared__ float s_m[MRG_GROUPS], s_l[MRG_GROUPS];
+  __shared__ __align__(16) float s_acc[GROUPS][DIMS + 4];
+  __shared__ float s_m[GROUPS], s_l[GROUPS];
   const int64_t bh = blockIdx.x, b = bh / Hq;
   const int h = static_cast<int>(bh % Hq), hk = h / G, r = h % G;
   const int grp = threadIdx.x >> 3, c4 = threadIdx.x & 7;
   pdl_trigger();
   pdl_wait();
   const int64_t base = (b * Hkv + hk) * splits;
-  const int d0 = blockIdx.y * MRG_DIMS + c4 * 4;
-  constexpr int BATCH = 8;   // splits whose loads are in flight together
+  const int d0 = blockIdx.y * DIMS + c4 * 4;
   const bool vec = (reinterpret_cast<uintptr_t>(part_acc) & 15u) == 0;   // the caller's workspace need not be 16-byte aligned
   float m_run = -INFINITY, l = 0.f;
   float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
-  for (int s0 = grp; s0 < splits; s0 += BATCH * MRG_GROUPS) {
+  for (int s0 = grp; s0 < splits; s0 += BATCH * GROUPS) {
     float2 ml[BATCH];
     float4 a[BATCH];
 #pragma unroll
     for (int j = 0; j < BATCH; ++j) {
-      const int s = s0 + j * MRG_GROUPS;
+      const int s = s0 + j * GROUPS;
       const int64_t i = (base + s) * G + r;
       ml[j] = make_float2(-INFINITY, 0.f);   // (max in the log2 domain, sum)
       a[j] = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -378,19 +378,19 @@ __global__ void __launch_bounds__(256) attn_decode_merge_kernel(const float* __r
   *reinterpret_cast<float4*>(&s_acc[grp][c4 * 4]) = acc;
   if (c4 == 0) { s_m[grp] = m_run; s_l[grp] = l; }
   __syncthreads();
-  if (threadIdx.x < MRG_DIMS) {
+  if (threadIdx.x < DIMS) {
     float m_all = -INFINITY;
 #pragma unroll
-    for (int g = 0; g < MRG_GROUPS; ++g) m_all = fmaxf(m_all, s_m[g]);
+    for (int g = 0; g < GROUPS; ++g) m_all = fmaxf(m_all, s_m[g]);
     const float m_use = m_all == -INFINITY ? 0.f : m_all;
     float o = 0.f, lt = 0.f;
 #pragma unroll
-    for (int g = 0; g < MRG_GROUPS; ++g) {
+    for (int g = 0; g < GROUPS; ++g) {
       const float f = ex2_approx(s_m[g] - m_use);
       lt += s_l[g] * f;
       o += s_acc[g][threadIdx.x] * f;
     }
-    out[bh * HD + blockIdx.y * MRG_DIMS + threadIdx.x] = from_f32<T>(lt > 0.f ? o / lt : 0.f);
+    out[bh * HD + blockIdx.y * DIMS + threadIdx.x] = from_f32<T>(lt > 0.f ? o / lt : 0.f);
   }
 }
 
@@ -759,8 +759,13 @@ extern "C" int b200_attn_decode(const void* q, const void* k, const void* v, con
       cudaLaunchKernelEx(&cfg, attn_decode_kernel<T, 2, true>, p);
     } else {
       launch_pdl(attn_decode_kernel<T, 2, false>, grid, dim3(128), 4 * 2 * DEC_STAGE_BYTES, st, p);
-      launch_pdl(attn_decode_merge_kernel<T>, dim3(static_cast<unsigned>(B * Hq), HD / MRG_DIMS), dim3(256), 0, st, static_cast<const float*>(p.part_acc),
-                 static_cast<const float*>(p.part_ml), static_cast<T*>(out), Hq, Hkv, p.G, d.splits);
+      const auto merge = [&](auto kernel, int groups, int dims) {
+        launch_pdl(kernel, dim3(static_cast<unsigned>(B * Hq), HD / dims), dim3(groups * dims / 4), 0, st, static_cast<const float*>(p.part_acc),
+                   static_cast<const float*>(p.part_ml), static_cast<T*>(out), Hq, Hkv, p.G, d.splits);
+      };
+      // (32 splits: two batches of the second form.  No plan has between 8 and 32.)
+      if (d.splits <= 32) merge(attn_decode_merge_kernel<T, 4, HD, 4>, 4, HD);
+      else merge(attn_decode_merge_kernel<T, 32, 32, 8>, 32, 32);
     }
   });
   B200_CHECK_LAUNCH("attn_decode_kernel");

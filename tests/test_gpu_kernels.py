@@ -391,11 +391,12 @@ def test_attn_decode(lib, B, S, valid):
     close(out, attn_ref(q, k, v, None, D ** -0.5, dtype)[:, :, 0], rtol=2e-2, atol=5e-3)
 
 
-@pytest.mark.parametrize("B,S,valid,shift", [(1, 32768, 20001, 0), (1, 32768, 32768, 1), (2, 17000, 1, 0), (3, 448, 447, 0), (1, 16, 5, 1), (1, 64, 64, 0)])
+@pytest.mark.parametrize("B,S,valid,shift", [(1, 32768, 20001, 0), (1, 32768, 32768, 1), (2, 17000, 1, 0), (3, 448, 447, 0), (1, 16, 5, 1), (1, 64, 64, 0),
+                                             (64, 448, 300, 0), (7, 17000, 9000, 1), (6, 17000, 17000, 0), (40, 300, 299, 1)])
 def test_attn_decode_merge_of_workspace_partials(lib, B, S, valid, shift):
     """Caches outside 512..16384 rows leave their splits' partial sums in the workspace for a second kernel: one
-    split, fewer splits than the kernel has groups, 256 of them with the masked ones empty; a workspace that is
-    only 4-byte aligned."""
+    split, fewer splits than the kernel has groups, 256 of them with the masked ones empty; many heads with few and
+    with many splits; a workspace that is only 4-byte aligned."""
     import model_zoo as mz
 
     dtype, Hq, Hkv, D = torch.bfloat16, 12, 2, 128
