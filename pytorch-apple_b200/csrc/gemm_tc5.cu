@@ -1909,13 +1909,16 @@ int persistent_bn(int64_t M, int64_t N, int64_t K, bool glu, bool residual) {
   return 0;
 }
 
+// Whole 16-byte words in the rows of the result and of the residual.
+bool rows16(const Tc5Args& a) {
+  return aligned16(a.out) && a.ldo % 8 == 0 && a.N % 8 == 0 && (!a.residual || (aligned16(a.residual) && a.ldr % 8 == 0));
+}
+
 // The bulk-copy epilogue handles 16-bit outputs with bias, residual and ReLU.
 bool tma_store_ok(const Tc5Args& a) {
   if (a.epilogue & (B200_EPI_GLU | B200_EPI_SILU_MUL)) return false;
   if (a.K > 2048) return false;   // long reductions hide the plain epilogue and prefer the deeper ring
-  if (!aligned16(a.out) || a.ldo % 8 || a.N % 8) return false;
-  if (a.residual && (!aligned16(a.residual) || a.ldr % 8)) return false;
-  return true;
+  return rows16(a);
 }
 
 template <typename T, bool CONV> int dispatch_persistent_t(int bn, bool ts, const Tc5Args& a, cudaStream_t st, const Tc5Conv* g) {
@@ -2013,15 +2016,19 @@ int linear_tc5(const Tc5Args& a, cudaStream_t st) {
     return a.dtype == B200_BF16 ? launch<__nv_bfloat16, 128, false, 2>(a, pl, st) : launch<__half, 128, false, 2>(a, pl, st);
   }
   if (const int rc = linear_stream(a, st); rc != B200_ENOTSUP) return rc;
-  // One wave of 128 x 128 tiles where 64-wide tiles would need a second one (reductions of 1024..4095, which the pair
-  // kernel does not split): with a residual on the persistent kernel (residual tile and result are bulk copies), else on
-  // the one-tile kernel.  us before -> after: q/k/v projection (N 2048) 777 tokens 17.4 -> 11.3, 1152 tokens 17.3 -> 12.2;
-  // output projection (N 1536, residual) 777 tokens 16.0 -> 10.9, 1500 16.7 -> 11.7; 1x1 convolution 1024 -> 256 of 32
-  // images 12.5 -> 8.9.  (Kernels the other way round: 13.0 and 16.3 at 777.  Fewer tiles: a prompt of 512 tokens with its
-  // 48 output-projection tiles on the persistent kernel takes 2979 instead of 2923 us.)
+  // One wave of 128 x 128 tiles where 64-wide tiles would need a second one (75 to 147 tiles; reductions of 1024..4095,
+  // which the pair kernel does not split).  Without a residual, or with rows that are not whole 16-byte words, on the
+  // one-tile kernel, whose staged epilogue writes whole rows with every thread; with a residual of aligned rows on the
+  // persistent kernel (up to K = 2048 residual tile and result are bulk copies).  us, 64-wide tiles -> this:
+  //   no residual    N 2048: 513 rows 15.8 -> 12.0, 777 rows 16.1 -> 12.0, 1152 rows 14.8 -> 12.4, 513 rows of K 4032 32.7 -> 25.7;
+  //                  N 256, K 1024, 9000 rows 12.5 -> 8.9
+  //   residual       N 1536: 777 rows 15.8 -> 12.1 (one-tile kernel 16.3), 1536 rows 16.5 -> 12.6, 777 rows of K 3072 27.6 -> 18.7
+  //   unaligned rows N 716, K 1032, 1537 rows 18.3 -> 16.1 (persistent kernel 22.0); N 1500, 777 rows 24.2 -> 17.7 (22.4)
+  // (Fewer tiles: a prompt of 512 tokens with its 48 output-projection tiles on the persistent kernel takes 2979 instead of
+  // 2923 us.)
   if (const int64_t tm = ceil_div(a.M, BM); tm > 1 && a.K >= 1024 && a.K < 4096 && !glu && tm * ceil_div(a.N, 128) < 148 &&
                                             tm * ceil_div(a.N, 64) > 148) {
-    if (a.residual) return dispatch_persistent<false>(128, a, st, nullptr);
+    if (a.residual && rows16(a)) return dispatch_persistent<false>(128, a, st, nullptr);
     const Tc5Plan pl = plan_for_bn(128, a.M, a.N, a.K);
     return a.dtype == B200_BF16 ? launch<__nv_bfloat16, 128, false, 1>(a, pl, st) : launch<__half, 128, false, 1>(a, pl, st);
   }

@@ -50,7 +50,11 @@ def close(got, ref, rtol=2e-2, atol=1e-2):
 @pytest.mark.parametrize("M,N,K,bias,res,relu,silu", [
     (777, 2048, 1536, True, False, False, False),   # one wave of 128-wide tiles, ragged last row tile
     (777, 1536, 1536, False, True, False, False),   # the same with a residual
-    (1537, 700, 1032, True, True, True, False),     # ragged columns and k
+    (1537, 716, 1032, True, True, True, False),     # the same with ragged columns, rows and k: rows that are no whole 16-byte words
+    (1537, 720, 1032, True, True, True, False),     # ragged columns in whole words: bulk copies
+    (777, 1536, 3080, False, True, False, False),   # a reduction past the bulk copies' limit
+    (777, 1500, 3080, True, True, False, False),
+    (1537, 700, 1032, True, True, True, False),     # 143 64-wide tiles: one wave of them
     (900, 1400, 1096, True, False, False, True),
     (1, 1536, 1536, True, False, False, False),
     (1, 1536, 8960, False, True, False, False),
