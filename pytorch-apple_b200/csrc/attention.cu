@@ -338,7 +338,7 @@ __global__ void __launch_bounds__(GROUPS * DIMS / 4) attn_decode_merge_kernel(co
   __shared__ float s_m[GROUPS], s_l[GROUPS];
   const int64_t bh = blockIdx.x, b = bh / Hq;
   const int h = static_cast<int>(bh % Hq), hk = h / G, r = h % G;
-  const int grp = threadIdx.x >> 3, c4 = threadIdx.x & 7;
+  const int grp = threadIdx.x / (DIMS / 4), c4 = threadIdx.x % (DIMS / 4);
   pdl_trigger();
   pdl_wait();
   const int64_t base = (b * Hkv + hk) * splits;
