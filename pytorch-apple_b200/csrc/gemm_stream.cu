@@ -318,15 +318,23 @@ struct SwPlan { int units, chunks, splits, chunks_per_split; };
 
 // Column blocks are split along K (clusters of up to eight) until about every SM has a CTA or two: the down projection
 // of one row takes 7.2 us with eight splits (192 CTAs), 8.2 with six, 10.5 with four; the short reductions are level
-// from four splits on.  Larger (non-portable) clusters lose: ten 7.9, twelve 9.9 us.
+// from four splits on.  Larger (non-portable) clusters lose: ten 7.9, twelve 9.9 us.  Besides:
+// - One block per SM, no split: four warps do not keep enough loads in flight, and from 9 rows on the tensor-map kernel
+//   was faster; two splits where a half still fills the loads in flight of its warps (us: N 8960, K 1536: 1 row 7.6 -> 5.8,
+//   16 rows 10.0 -> 7.5, tensor-map kernel 9.5; N 9472, K 3584, 8 rows 17.7 -> 12.5, 14.5; with K 512 two splits lose: 2.6 -> 3.3).
+// - Four splits for three where that leaves a warp fewer chunks (K = N = 3584: 1 row 7.1 -> 6.1, 16 rows 9.2 -> 8.0, tensor-map
+//   kernel 8.7; N 3840, K 1536, two chunks per warp either way, loses: 9 rows 4.5 -> 4.9).
 SwPlan plan_stream(int64_t N, int64_t K) {
   SwPlan pl;
   pl.units = static_cast<int>(N / SW_COLS);
   pl.chunks = static_cast<int>(K / SW_CHUNK);
+  const auto per_warp = [&](int splits) { return ceil_div(ceil_div(pl.chunks, splits), SW_WARPS); };
   int s = 192 / pl.units;
   if (s > pl.chunks / SW_WARPS) s = pl.chunks / SW_WARPS;
   if (s > 8) s = 8;
   if (s < 1) s = 1;
+  if (s == 1 && pl.units <= 148 && pl.chunks >= 2 * SW_WARPS * SW_DEPTH) s = 2;
+  if (s == 3 && per_warp(4) < per_warp(3)) s = 4;
   pl.chunks_per_split = static_cast<int>(ceil_div(pl.chunks, s));
   pl.splits = static_cast<int>(ceil_div(pl.chunks, pl.chunks_per_split));
   return pl;

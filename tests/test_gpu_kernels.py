@@ -225,6 +225,11 @@ def test_linear_norm_fused_rmsnorm(lib, M, N, K, mode):
 ])
 def test_linear_few_rows_edges(lib, M, N, K, shift, ldx):
     """Edges of the weight-streaming kernel and of its rule; residual, bias and ReLU in the final pass.  The bound: fp32
+    (64 * 148, 1024, 0, 0),   # one block per SM: two splits
+    (64 * 97, 1088, 0, 0),    # two splits, 9 and 8 chunks
+    (64 * 112, 960, 0, 0),    # one block per SM, all chunks in flight at once: no split
+    (64 * 56, 1792, 0, 0),    # four splits of seven chunks
+    (64 * 56, 1536, 0, 0),    # three splits of eight
     sums in any order (K * 2^-24 of the sum of magnitudes, products exact), and two roundings to bf16
     (eight significant bits: at most 2^-8 of the value each)."""
     lda, ldo = K + ldx, N + ldx
