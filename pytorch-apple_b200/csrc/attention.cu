@@ -85,10 +85,11 @@ __global__ void __launch_bounds__(128, STAGES == 2 ? 3 : 2) attn_decode_kernel(c
   const int n_keys = static_cast<int>(s_end - s_begin);
   const int nblk = (n_keys + 15) / 16;
 
-  // The successor's start: with clusters of 16 the whole grid is resident, and weight loads that begin here compete with
-  // the keys and values, so it is put off to the end (decode layer of eight sequences 45.3 -> 44.2 us, one sequence
-  // 34.1 -> 33.5); a grid of several waves triggers at once (step of 64 sequences 2.742 ms, at the end 2.755).
-  const bool trigger_late = CM && p.splits == 16;
+  // The successor's start: clusters of more than eight are planned only where the whole grid is resident, and weight loads
+  // that begin here compete with the keys and values, so it is put off to the end (decode layer of eight sequences
+  // 45.3 -> 44.2 us, one sequence 34.1 -> 33.5; step of one sequence over 1111 rows, 14 splits, 918 -> 913); a grid of
+  // several waves triggers at once (step of 64 sequences 2.742 ms, at the end 2.755).
+  const bool trigger_late = CM && p.splits > 8;
   if (!trigger_late) pdl_trigger();
   if (CM) tc5::cluster_sync();   // every CTA of the cluster runs before anyone writes into a peer (overlaps the predecessor)
   pdl_wait();   // q, the new cache rows and the mask come from the kernels before this one
