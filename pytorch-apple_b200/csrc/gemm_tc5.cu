@@ -535,7 +535,7 @@ template <int BN, bool TS> struct PCfg {
   static constexpr int W_WARP = TS ? 11 : 6;
   static constexpr int A2_WARP = TS ? 12 : 7;           // second activation producer
   static constexpr int THREADS = (A2_WARP + 1) * 32;
-  static constexpr int W_WARP_GATHER = 10;
+  static constexpr int W_WARP_GATHER = 10, THREADS_GATHER = (W_WARP_GATHER + 1) * 32;
   static constexpr int EPI_WARPS = TS ? 8 : 4;
 };
 
@@ -548,7 +548,7 @@ struct RingPos {
 };
 
 template <typename T, int BN, bool CONV, bool TS, int KPS>
-__global__ void __launch_bounds__(PCfg<BN, TS>::THREADS, 1)
+__global__ void __launch_bounds__(CONV && !TS && KPS == 1 ? PCfg<BN, TS>::THREADS_GATHER : PCfg<BN, TS>::THREADS, 1)
     gemm_tc5p_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_w,
                      const __grid_constant__ CUtensorMap map_r, const __grid_constant__ CUtensorMap map_o, const Tc5Params p,
                      const int tiles_m, const int n_tiles) {
@@ -599,7 +599,7 @@ __global__ void __launch_bounds__(PCfg<BN, TS>::THREADS, 1)
   pdl_trigger();
   auto dead = [&]() { return *reinterpret_cast<volatile int*>(&failed) != 0; };
 
-  const bool gather_variant = CONV && !TS && !p.g.im2col;   // launched with 352 threads
+  const bool gather_variant = CONV && !TS && !p.g.im2col;   // launched with THREADS_GATHER threads, one k-block per stage
   const int a_id = warp == 0 ? 0 : warp == PCfg<BN, TS>::A2_WARP ? 1 : -1;   // producer number among the activation producers (-1: not one)
   if (a_id >= 0 && a_id < p.npa) {
     // ---- activation producers: with two, the k-blocks alternate between them (a 3x3 convolution is bound
@@ -1805,7 +1805,7 @@ int launch_persistent(const Tc5Args& a, cudaStream_t st, const Tc5Conv* g = null
   // own waits, one ring pass back at a time, and a parity wait cannot tell a barrier two phases behind from the
   // phase it expects.  Two is below every ring depth used here.)
   p.npa = CONV && p.g.im2col && ceil_div(a.K, BK) >= 2 ? 2 : 1;
-  const dim3 block((CONV && !TS && !p.g.im2col) ? 352 : PC::THREADS);
+  const dim3 block((CONV && !TS && !p.g.im2col) ? PC::THREADS_GATHER : PC::THREADS);
   if (p.kps == 2)
     launch_pdl(gemm_tc5p_kernel<T, BN, CONV, TS, BN <= 128 ? 2 : 1>, dim3(grid), block, SMEM, st, ma, mw, mr, mo, p, static_cast<int>(tiles_m),
                static_cast<int>(tiles));

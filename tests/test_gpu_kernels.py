@@ -344,6 +344,10 @@ def test_linear_rejects_unaligned(lib):
 ])
 def test_conv2d_nhwc(lib, N, C, H, O, k, s, p, res, relu):
     dtype = torch.float16
+    (1, 64, 40, 64, 3, 9, 1, False, True),     # no im2col map (stride past 8): threads gather the pixels; one tile
+    (2, 192, 100, 200, 3, 9, 1, True, True),   # the same, several ragged tiles, 27 k-blocks, residual
+    (1, 64, 6, 64, 3, 1, 128, False, False),   # no im2col map (padding past 127) and a tile for every SM: the persistent kernel gathers
+    (1, 64, 6, 136, 1, 1, 128, True, True),    # the same, two column tiles, residual
     x = gen((N, C, H, H), dtype)
     w = gen((O, C, k, k), torch.float32, 1, math.sqrt(2.0 / (C * k * k)))
     gamma, beta = torch.rand(O) + 0.5, torch.randn(O) * 0.1
