@@ -54,6 +54,7 @@ FLOAT_DTYPES = ("float32", "float16", "bfloat16")
 DTYPE_BYTES = {"float32": 4, "float16": 2, "bfloat16": 2, "int32": 4, "int64": 8, "bool": 1, "uint8": 1}
 MAX_CHAIN_OPS = 12
 MAX_CHAIN_INPUTS = 4
+MAX_TENSOR_MAP_KEYS = 32768   # keys of the tensor-map prefill attention (a verdict per 64 of them in shared memory)
 
 
 def infer_compute_dtype(graph: IRGraph, requested: str | None) -> str:
@@ -1074,16 +1075,21 @@ class _Lowering:
     def _aligned_mask(self, name: str, T: int) -> str:
         """The mask with rows at multiples of 16 bytes, as tensor maps need them: one copy that all layers of a call
         share.  A 777-token prompt takes the mma.sync attention otherwise (145 us per layer and call; the tensor-map
-        kernel 27); the copy of its 1.2 MB mask is 7 us once."""
+        kernel 27); the copy of its 1.2 MB mask is 7 us once.  A mask that is expanded over the sequences is copied
+        once, not once per sequence; one with more keys than the tensor-map kernel takes is not copied."""
         v = self.view(name)
-        if len(v.shape) < 2 or v.shape[-2] != T or v.strides[-1] != 1 or (v.offset % 8 == 0 and all(s % 8 == 0 for s in v.strides[:-1])):
+        if len(v.shape) < 2 or v.shape[-2] != T or v.strides[-1] != 1 or (v.offset % 8 == 0 and all(s % 8 == 0 for s in v.strides[:-1])) \
+                or v.shape[-1] > MAX_TENSOR_MAP_KEYS:
             return name
         dst = f"{name}__rows16"
         if dst not in self.out.views:
-            padded = v.shape[:-1] + (-(-v.shape[-1] // 8) * 8,)
-            full = self.alloc(dst, padded, v.dtype)
-            self.out.views[dst] = TensorView(dst, 0, v.shape, full.strides, v.dtype)
-            self.copy(name, dst)
+            lead = tuple(1 if st == 0 else n for n, st in zip(v.shape[:-2], v.strides[:-2]))
+            full = self.alloc(dst, lead + (T, -(-v.shape[-1] // 8) * 8), v.dtype)
+            rows = TensorView(dst, 0, lead + v.shape[-2:], full.strides, v.dtype)
+            self.out.views[dst] = V.broadcast_to(rows, v.shape)
+            self.emit(SpecialKernelStep("strided_copy", "mask rows at multiples of 16 bytes", [name], dst,
+                                        params={"op": "strided_copy", "in_view": TensorView(v.buffer, v.offset, rows.shape, v.strides, v.dtype),
+                                                "out_view": rows}), [name, dst])
         return dst
 
     def lower_attention(self, node: OpNode) -> None:

@@ -201,6 +201,45 @@ def test_prefill_mask_rows_are_aligned_once_per_call(fake_native, B, T):
     assert fake_native.calls.count("attn_prefill") == cfg.num_hidden_layers
 
 
+class _ExpandedMaskWrapper(mz.QwenPrefillWrapper):
+    """One mask for all sequences, expanded over the batch inside the graph."""
+
+    def forward(self, input_ids, attention_mask, position_ids, cache_position):
+        return super().forward(input_ids, attention_mask.expand(input_ids.shape[0], -1, -1, -1), position_ids, cache_position)
+
+
+def test_prefill_mask_expanded_over_the_sequences_is_copied_once(fake_native):
+    """The copy with aligned rows is as large as the mask that was given; every sequence reads it (a batch stride of zero)."""
+    from cuda_compiler import compile_subgraph
+    from golden.make_golden import tiny_qwen
+
+    B, T = 3, 9
+    cfg, sd, model = tiny_qwen()
+    ids, _, pos, at = mz.qwen2_example_inputs(cfg, B, T, None, device="cpu")
+    ir = extract_ir(_ExpandedMaskWrapper(model), (ids, mz.causal_mask(1, T, T, 0), pos, at), "p")
+    ids = torch.randint(0, cfg.vocab_size, (B, T), generator=torch.Generator().manual_seed(0))
+    ins = (ids, mz.causal_mask(1, T, T, 0), torch.arange(T)[None].expand(B, T).contiguous(), torch.arange(T))
+    out, _ = run_backend(ir, mz.state_dict_numpy(sd), np_inputs(ir, ins))
+    name = ir["graph_outputs"][0]["name"]
+    ref = IRInterpreter(ir, sd).execute(dict(zip([s["name"] for s in ir["graph_inputs"]], ins)))[name]
+    assert np.abs(to_f32(out[name]) - ref.float().numpy()).max() < 0.1
+    steps = compile_subgraph(ir).steps
+    copies = [st.params["out_view"] for st in steps if getattr(st, "kernel_name", "") == "strided_copy"]
+    assert [v.numel for v in copies] == [T * T]
+    masks = [st.params["mask"] for st in steps if (getattr(st, "params", None) or {}).get("op") == "attention"]
+    assert len(masks) == cfg.num_hidden_layers and all(v.strides[0] == 0 and v.strides[2] == 16 and v.buffer == copies[0].buffer for v in masks)
+
+
+@pytest.mark.parametrize("T,copies", [(32761, 1), (32769, 0)])
+def test_masks_that_the_tensor_map_attention_does_not_take_are_not_copied(T, copies):
+    from cuda_compiler import compile_subgraph
+    from golden.make_golden import TINY_QWEN
+
+    cfg = mz.qwen2_config(num_layers=1, **TINY_QWEN)
+    ir = extract_ir(mz.QwenPrefillWrapper(mz.qwen2_model(cfg)), mz.qwen2_example_inputs(cfg, 1, T, None), "p")
+    assert len([st for st in compile_subgraph(ir).steps if getattr(st, "kernel_name", "") == "strided_copy"]) == copies
+
+
 def test_mixed_partitions_use_the_injected_cpu_executor(fake_native):
     from cuda_compiler import compile_subgraph
     from cuda_runtime import CUDABackend
