@@ -145,7 +145,10 @@ def test_linear_gated_mlp_epilogue(lib, M, I, K):
 
 
 @pytest.mark.parametrize("M,N,K,mode", [(1, 2048, 1536, "bias"), (8, 2048, 1536, "bias"), (64, 2048, 1536, "bias"), (64, 17920, 1536, "glu"),
-                                        (5, 17920, 1536, "glu"), (64, 151936, 1536, "plain"), (33, 1536, 1536, "chain"), (64, 1536, 8960, "chain")])
+                                        (5, 17920, 1536, "glu"), (64, 151936, 1536, "plain"), (33, 1536, 1536, "chain"), (64, 1536, 8960, "chain"),
+                                        *((m, 1536, 1536, "chain") for m in (1, 8, 9, 16, 17, 24, 25)),
+                                        *((m, 1536, 8960, "chain") for m in (1, 9, 16, 17)), *((m, 17920, 1536, "glu") for m in (8, 9, 16, 17)),
+                                        *((m, 2048, 1536, "bias") for m in (9, 17, 24)), (24, 4096, 1536, "glu")])
 def test_linear_norm_fused_rmsnorm(lib, M, N, K, mode):
     """RMSNorm folded into decode GEMMs.  "chain": a residual GEMM that also writes the sum-of-squares
     partials of its output rows, followed by a GEMM over gain-folded weights that scales its output
@@ -212,6 +215,7 @@ def test_linear_norm_fused_rmsnorm(lib, M, N, K, mode):
     assert code.value == 0
 
 
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
 @pytest.mark.parametrize("M", [1, 8, 9, 16, 17, 24, 25])
 @pytest.mark.parametrize("N,K,shift,ldx", [
     (64, 64, 0, 0),           # one block, one chunk: three of the four warps have none
@@ -221,51 +225,54 @@ def test_linear_norm_fused_rmsnorm(lib, M, N, K, mode):
     (64 * 300, 192, 0, 0),    # more blocks than resident CTAs: a CTA walks two
     (64 * 150, 25664, 0, 0),  # no split and rows too long to keep: the tensor-map kernel
     (64 * 150, 1536, 0, 0),   # no split: two groups of rows fit beside a second CTA, three do not
-    (200, 328, 0, 0),         # ragged block and chunk
-])
-def test_linear_few_rows_edges(lib, M, N, K, shift, ldx):
-    """Edges of the weight-streaming kernel and of its rule; residual, bias and ReLU in the final pass.  The bound: fp32
     (64 * 148, 1024, 0, 0),   # one block per SM: two splits
     (64 * 97, 1088, 0, 0),    # two splits, 9 and 8 chunks
     (64 * 112, 960, 0, 0),    # one block per SM, all chunks in flight at once: no split
     (64 * 56, 1792, 0, 0),    # four splits of seven chunks
     (64 * 56, 1536, 0, 0),    # three splits of eight
-    sums in any order (K * 2^-24 of the sum of magnitudes, products exact), and two roundings to bf16
-    (eight significant bits: at most 2^-8 of the value each)."""
+    (200, 328, 0, 0),         # ragged block and chunk
+])
+def test_linear_few_rows_edges(lib, M, N, K, shift, ldx, dtype):
+    """Edges of the weight-streaming kernel and of its rule; residual, bias and ReLU in the final pass.  The bound: fp32
+    sums in any order (K * 2^-24 of the sum of magnitudes, products exact), and two roundings to
+    the activation type (8 or 11 significant bits: at most 2^-8 or 2^-11 of the value each; subnormal halves 2^-25)."""
     lda, ldo = K + ldx, N + ldx
-    A = torch.full((M, lda), float("nan"), dtype=torch.bfloat16, device="cuda")
-    A[:, :K] = gen((M, K)).cuda()
+    A = torch.full((M, lda), float("nan"), dtype=dtype, device="cuda")
+    A[:, :K] = gen((M, K), dtype).cuda()
     g = torch.Generator(device="cuda").manual_seed(1)
-    Wb = torch.randn(N * K + shift, generator=g, device="cuda").mul_(K ** -0.5).bfloat16()
+    Wb = torch.randn(N * K + shift, generator=g, device="cuda").mul_(K ** -0.5).to(dtype)
     W = Wb[shift:].view(N, K)
-    b, r = gen((N,), seed=2).cuda(), torch.zeros(M, ldo, dtype=torch.bfloat16, device="cuda")
-    r[:, :N] = gen((M, N), seed=3).cuda()
-    out = torch.full((M, ldo), 7.0, dtype=torch.bfloat16, device="cuda")
+    b, r = gen((N,), dtype, seed=2).cuda(), torch.zeros(M, ldo, dtype=dtype, device="cuda")
+    r[:, :N] = gen((M, N), dtype, seed=3).cuda()
+    out = torch.full((M, ldo), 7.0, dtype=dtype, device="cuda")
     ws = torch.zeros(1 << 22, dtype=torch.uint8, device="cuda")
-    ok(lib, lib.b200_linear(A.data_ptr(), W.data_ptr(), b.data_ptr(), r.data_ptr(), out.data_ptr(), M, N, K, lda, K, ldo, ldo, 2, 2,
+    ok(lib, lib.b200_linear(A.data_ptr(), W.data_ptr(), b.data_ptr(), r.data_ptr(), out.data_ptr(), M, N, K, lda, K, ldo, ldo, DT[dtype], DT[dtype],
                             1 | 8, None, 0, ws.data_ptr(), ws.numel(), stream()))
     x, w = A[:, :K].double(), W.double()
     lin = x @ w.T + b.double()
     want = (lin + r[:, :N].double()).clamp(min=0)
-    bound = (x.abs() @ w.abs().T) * (K * 2.0 ** -24) + (lin.abs() + want) * 2.0 ** -8 * 1.01 + 1e-6
+    bound = (x.abs() @ w.abs().T) * (K * 2.0 ** -24) + (lin.abs() + want) * (2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -11) * 1.01 + 1e-6
     err = (out[:, :N].double() - want).abs()
     assert (err <= bound).all(), float((err - bound).max())
     assert (out[:, N:] == 7.0).all()
 
 
-def test_linear_norm_rejects_shapes_outside_the_fused_kernel(lib):
-    t = torch.zeros(128 * 1536, dtype=torch.bfloat16, device="cuda")
-    f = torch.zeros(4096, device="cuda")
-    args = lambda M, N, K, cols, sq_out: (t.data_ptr(), t.data_ptr(), None, None, t.data_ptr(), M, N, K, K, K, N, 0, 2, 2, 0, 1e-6,
-                                          f.data_ptr(), cols, f.data_ptr() if sq_out else None, stream())
-    assert lib.b200_linear_norm(*args(100, 64, 128, 1, False)) == -4 and b"M <= 64" in lib.b200_last_error()   # prefill-sized M
-    assert lib.b200_linear_norm(*args(8, 64, 128, 40, False)) == -4                                              # too many partials
-    assert lib.b200_linear_norm(*args(8, 72, 128, 1, True)) == -4                                                # N not a multiple of 64
+@pytest.mark.parametrize("M,N,K,res,kernel", [
+    (1, 1536, 8960, True, "gemm_stream_kernel"), (16, 1536, 8960, True, "gemm_stream_kernel"), (17, 1536, 8960, True, "gemm_tc5_kernel"),
+    (24, 2048, 1536, False, "gemm_stream_kernel"), (25, 2048, 1536, False, "gemm_tc5_kernel"),
+    (16, 17920, 1536, False, "gemm_stream_kernel"), (17, 17920, 1536, False, "gemm_tc5_kernel"), (8, 200, 328, False, "gemm_tc5_kernel"),
+    (777, 2048, 1536, False, "gemm_tc5_kernel"), (777, 1536, 1536, True, "gemm_tc5p_kernel"), (777, 1500, 1536, True, "gemm_tc5_kernel"),
+    (2048, 1536, 1536, True, "gemm_pair_kernel"),
+])
+def test_linear_runs_on_the_kernel_that_its_shape_calls_for(lib, M, N, K, res, kernel):
+    t = torch.zeros(M * K + N * K + 2 * M * N, dtype=torch.bfloat16, device="cuda")
+    a, w, o, r = (t[n:].data_ptr() for n in (0, M * K, M * K + N * K, M * K + N * K + M * N))
+    with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CUDA]) as prof:
+        ok(lib, lib.b200_linear(a, w, None, r if res else None, o, M, N, K, K, K, N, N if res else 0, 2, 2, 8, None, 0, None, 0, stream()))
+    ran = [e.key for e in prof.key_averages() if "gemm" in e.key]
+    assert len(ran) == 1 and kernel + "<" in ran[0], ran
 
 
-def test_bounded_wait_runs_out_and_the_context_survives(lib):
-    """A barrier wait that can never be satisfied: the kernel's bounded wait gives up after the probe limit,
-    leaves code 99 in the device error word and returns; the next kernels run normally."""
 @pytest.mark.parametrize("M", [1, 9, 24, 25, 64])
 def test_row_scale_adds_its_partials_in_index_order(lib, M):
     """Every kernel behind b200_linear_norm adds the sum-of-squares partials of a row in index order: 2^24 and then ones
@@ -294,6 +301,19 @@ def test_row_scale_adds_its_partials_in_index_order(lib, M):
     assert (out.float().cpu().abs() <= prod.mul(rinv[0]).abs() * 2.0 ** -22).all()
 
 
+def test_linear_norm_rejects_shapes_outside_the_fused_kernel(lib):
+    t = torch.zeros(128 * 1536, dtype=torch.bfloat16, device="cuda")
+    f = torch.zeros(4096, device="cuda")
+    args = lambda M, N, K, cols, sq_out: (t.data_ptr(), t.data_ptr(), None, None, t.data_ptr(), M, N, K, K, K, N, 0, 2, 2, 0, 1e-6,
+                                          f.data_ptr(), cols, f.data_ptr() if sq_out else None, stream())
+    assert lib.b200_linear_norm(*args(100, 64, 128, 1, False)) == -4 and b"M <= 64" in lib.b200_last_error()   # prefill-sized M
+    assert lib.b200_linear_norm(*args(8, 64, 128, 40, False)) == -4                                              # too many partials
+    assert lib.b200_linear_norm(*args(8, 72, 128, 1, True)) == -4                                                # N not a multiple of 64
+
+
+def test_bounded_wait_runs_out_and_the_context_survives(lib):
+    """A barrier wait that can never be satisfied: the kernel's bounded wait gives up after the probe limit,
+    leaves code 99 in the device error word and returns; the next kernels run normally."""
     code = C.c_int(-1)
     ok(lib, lib.b200_debug_device_error(C.byref(code), 1))
     assert code.value == 0
@@ -340,14 +360,14 @@ def test_linear_rejects_unaligned(lib):
     (2, 512, 14, 512, 3, 2, 1, False, True),   # 72 k-blocks over eight CTAs: a split starts inside a filter tap
     (3, 192, 9, 72, 3, 2, 1, True, False),     # 27 k-blocks in uneven splits, output channels past a whole tile
     (1, 128, 56, 130, 1, 2, 0, False, True),   # output rows without 8-byte alignment
-    (37, 256, 14, 1024, 1, 1, 0, True, False), # column tiles fastest with eight column tiles (grid trimmed to a multiple of 8)
-])
-def test_conv2d_nhwc(lib, N, C, H, O, k, s, p, res, relu):
-    dtype = torch.float16
     (1, 64, 40, 64, 3, 9, 1, False, True),     # no im2col map (stride past 8): threads gather the pixels; one tile
     (2, 192, 100, 200, 3, 9, 1, True, True),   # the same, several ragged tiles, 27 k-blocks, residual
     (1, 64, 6, 64, 3, 1, 128, False, False),   # no im2col map (padding past 127) and a tile for every SM: the persistent kernel gathers
     (1, 64, 6, 136, 1, 1, 128, True, True),    # the same, two column tiles, residual
+    (37, 256, 14, 1024, 1, 1, 0, True, False), # column tiles fastest with eight column tiles (grid trimmed to a multiple of 8)
+])
+def test_conv2d_nhwc(lib, N, C, H, O, k, s, p, res, relu):
+    dtype = torch.float16
     x = gen((N, C, H, H), dtype)
     w = gen((O, C, k, k), torch.float32, 1, math.sqrt(2.0 / (C * k * k)))
     gamma, beta = torch.rand(O) + 0.5, torch.randn(O) * 0.1
@@ -815,7 +835,8 @@ def test_qkv_rope_cache_fused(lib, B, T):
 
 
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
-@pytest.mark.parametrize("B,norm,pos", [(1, True, 17), (8, True, 4100), (64, True, 4351), (5, False, -3), (64, False, 0)])
+@pytest.mark.parametrize("B,norm,pos", [(1, True, 17), (8, True, 4100), (64, True, 4351), (5, False, -3), (64, False, 0), (9, True, 0),
+                                        (16, True, 4351), (17, False, 5), (19, True, 613), (24, True, -1), (25, True, 3)])
 def test_linear_qkv_rope_equals_the_two_kernels(lib, dtype, B, norm, pos):
     """The merged q/k/v projection whose final pass rotates q and k and writes the cache rows is
     bit-identical to the projection followed by the rope / cache kernel - q, both caches whole."""
