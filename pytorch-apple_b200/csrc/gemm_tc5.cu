@@ -26,7 +26,8 @@ constexpr int BM = 128, BK = 64;
 // Kernel modes.
 //   0  compute-bound shapes (several row tiles): two CTAs per SM with a short ring, so that
 //      one CTA's epilogue overlaps the other's main loop;
-//   1  a single row tile with 64 < M <= 128 (pure weight streaming) and convolutions with few tiles: one CTA per SM, deep ring;
+//   1  a single row tile with 64 < M <= 128 (pure weight streaming), several row tiles with split-K or with one wave of
+//      128-wide tiles, and convolutions with few tiles: one CTA per SM, deep ring, staged epilogue;
 //   2  M <= 64 (decode): the activation tile is loaded 64 rows high (the MMA still reads 128
 //      rows; the upper half is whatever follows in shared memory and only feeds accumulator
 //      rows that are never stored), which halves the stage size; one CTA per SM with a ring of
@@ -60,9 +61,9 @@ __device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(tc5::smem_addr(bar)) : "memory");
 }
 
-// CONV = false: A tiles arrive by TMA.  CONV = true (implicit-GEMM convolution): the four
-// epilogue warps, idle during the main loop, gather the A tile - one output pixel per
-// thread, 128 bytes of channels per k-block - with zero-filling cp.async into the same
+// CONV = false: A tiles arrive by TMA.  CONV = true (implicit-GEMM convolution), MODE 1: by TMA through an im2col map.
+// CONV = true, MODE 0 (geometries without such a map): the four epilogue warps, idle during the main loop, gather the A
+// tile - one output pixel per thread, 128 bytes of channels per k-block - with zero-filling cp.async into the same
 // 128-byte-swizzled layout TMA would produce, and signal the stage's barrier themselves.
 template <typename T, int BN, bool CONV, int MODE>
 __global__ void __launch_bounds__(224, Cfg<BN, MODE>::CTAS) gemm_tc5_kernel(const __grid_constant__ CUtensorMap map_a,
@@ -89,7 +90,7 @@ __global__ void __launch_bounds__(224, Cfg<BN, MODE>::CTAS) gemm_tc5_kernel(cons
   const int nstg = (nkb + KPS - 1) / KPS;                // ring stages this CTA fills
   auto stage_cnt = [&](int i) { return nkb - i * KPS < KPS ? nkb - i * KPS : KPS; };   // k-blocks of stage i
   // single-row-tile shapes and split-K stage the accumulator through shared memory (see the end of the kernel)
-  const bool gather = CONV && MODE == 0 && !p.g.im2col;   // convolution A tile copied by the epilogue warps instead of TMA
+  constexpr bool gather = CONV && MODE == 0;   // convolution without an im2col map: A tile copied by the epilogue warps instead of TMA
   const bool staged = MODE >= 1 || (!CONV && p.splits > 1);   // MODE >= 1: known at compile time, the direct epilogue is dropped
   const bool glu = (p.epilogue & B200_EPI_GLU) != 0;       // host guarantees BN == 128 and N % 128 == 0
   const bool rope = CAN_NORM && BN == 128 && p.rope.cos != nullptr;   // tile = one attention head (host: BN == 128, N % 128 == 0)
@@ -1671,10 +1672,11 @@ int launch(const Tc5Args& a, const Tc5Plan& plan, cudaStream_t st, const Tc5Conv
   Tc5Params p;
   p.x = a.A;
   p.g = g ? *g : Tc5Conv{};
-  if (CONV) {
-    p.g.im2col = make_im2col_map(&ma, a.A, p.g, a.dtype) ? 1 : 0;
-    if (!p.g.im2col && MODE > 0) return B200_ENOTSUP;
-    if (!p.g.im2col) ma = mw;   // unused: the epilogue warps gather the A tile
+  if (CONV && MODE == 0) {
+    ma = mw;   // unused: the epilogue warps gather the A tile
+  } else if (CONV) {
+    if (!make_im2col_map(&ma, a.A, p.g, a.dtype)) return B200_ENOTSUP;
+    p.g.im2col = 1;
   } else if (!make_map(&ma, a.A, a.M, a.K, a.lda, Cfg<BN, MODE>::AROWS, a.dtype)) {
     return B200_ENOTSUP;
   }
@@ -2078,12 +2080,12 @@ int conv_tc5(const Tc5Args& a, const Tc5Conv& g, cudaStream_t st) {
   }
   if (g.C % BK || a.K != static_cast<int64_t>(g.KH) * g.KW * g.C || a.ldw % 8 || !aligned16(a.A) || !aligned16(a.W)) return B200_ENOTSUP;
   if (const int bn = persistent_bn(a.M, a.N, a.K, false, a.residual != nullptr)) return dispatch_persistent<true>(bn, a, st, &g);
-  {   // fewer tiles than SMs; falls through without an im2col map
+  {   // fewer tiles than SMs
     const Tc5Plan sp = plan_conv_split(a.M, a.N, a.K);
     const int rc = a.dtype == B200_BF16 ? launch<__nv_bfloat16, 64, true, 1>(a, sp, st, &g) : launch<__half, 64, true, 1>(a, sp, st, &g);
     if (rc != B200_ENOTSUP) return rc;
   }
-  Tc5Plan pl;
+  Tc5Plan pl;   // no im2col map (stride above 8, padding above 127, filter above 128): threads gather the pixels
   pl.bn = a.N >= 128 ? 128 : 64;
   pl.tiles_n = ceil_div(a.N, pl.bn);
   pl.tiles_m = ceil_div(a.M, BM);

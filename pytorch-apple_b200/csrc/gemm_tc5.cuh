@@ -66,7 +66,7 @@ constexpr int STREAM_MAX_ROWS = 24;
 constexpr int NORM_MAX_PARTS = 32;   // row scaling: at most this many sum-of-squares partials per row
 int linear_stream(const Tc5Args& a, cudaStream_t stream);
 bool tc5_enabled();
-// Scratch bytes linear_tc5 needs for (M, N, K): always 0.
+// Scratch bytes linear_tc5 needs for (M, N, K): the fp32 partial sums of the CTA-pair kernel's split-K, else 0.
 int64_t linear_tc5_workspace_bytes(int64_t M, int64_t N, int64_t K);
 
 }  // namespace b200
