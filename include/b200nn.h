@@ -256,8 +256,8 @@ int b200_conv_weight_prep(const void* w, const void* conv_bias, const void* gamm
  * A, W, out, residual share `dtype` (f16/bf16), fp32 accumulation; bias dtype is
  * `bias_dtype`.  lda/ldw/ldo/ldr are row strides in elements.  Any M.  Operands that
  * meet the TMA rules (16-byte aligned, strides multiples of 8 elements) run on the
- * tcgen05 path (up to 24 rows of whole 64-column blocks and 64-wide chunks: a kernel that streams
- * the weights through registers): one tile per CTA with split-K inside a thread-block cluster (partial sums
+ * tcgen05 path (up to 24 rows of whole 64-column blocks and 64-wide chunks, where the activations of a
+ * K range fit beside a second block: a kernel that streams the weights through registers): one tile per CTA with split-K inside a thread-block cluster (partial sums
  * meet in distributed shared memory, no scratch) for M <= 128 and for shapes with few
  * tiles, a persistent kernel with 128 x 64..256 tiles, or 256 x 256 tiles on pairs of CTAs
  * (cta_group::2) for M > 128, N >= 1024, K >= 1024.  `workspace` (zero-initialised by the

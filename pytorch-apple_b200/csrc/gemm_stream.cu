@@ -2,7 +2,7 @@
 //
 // With a handful of rows the weights are the work: every byte of W is read once and nothing else matters as long
 // as enough of them are in flight, from before the predecessor has finished until the last one has arrived.
-// - The problem is transposed: 16 weight rows are the M side of mma.sync m16n8k16, 8 sequences its N side (6 flop/B
+// - The problem is transposed: 16 weight rows are the M side of mma.sync m16n8k16, 8 sequences its N side (8 flop/B
 //   at 8 rows: the legacy tensor path is far from its limit, and a warp needs no barrier to feed it).
 // - Weights go from memory straight into the registers that are the MMA operands: k is permuted alike in both operands,
 //   so that thread t of a quad owns k = 16t..16t+15 of a 64-wide chunk - one 256-bit load per row, a full 128-byte line
@@ -22,8 +22,10 @@
 //    8 rows   6.6 ->  4.7    5.4 ->  3.5   12.8 -> 10.5    9.8 ->  7.7                       100 -> 76
 //   16 rows   7.7 ->  6.0    5.4 ->  4.0   13.4 -> 13.5    9.8 ->  9.3                        99 -> 84
 // The activations of a CTA's K range stay in shared memory, which bounds the rows that two CTAs per SM can take: 16 for
-// a 1536-wide unsplit row, 24 where K is split (q/k/v and output projection at 19 rows 7.4 -> 6.1 and 5.4 -> 4.1 us); wider
-// unsplit rows and more sequences stay with the tensor-map kernel (gate/up at 19 rows: 13.1 there, 22 here).
+// a 1536-wide unsplit row and for an eighth of 8960, 24 for a sixth of 1536 (q/k/v and output projection at 19 rows 7.4 ->
+// 6.1 and 5.4 -> 4.1 us); other rows stay with the tensor-map kernel (gate/up at 19 rows: 13.1 there, 22 here).
+// The eviction hint on the weights does not cost those that fit L2 and come again: 1536 x 8960, one row, in L2 4.7 us,
+// from memory 7.2 (tensor-map kernel 8.2 and 9.3).
 // Measured and not used: the same loop on a cp.async ring (paced by shared-memory traffic and waits: 28.9 against 24.6 us
 // per layer), prefetching a later part of the weights into L2 (every form slower, by up to 13 us per layer).
 #include "gemm_epilogue.cuh"
