@@ -394,6 +394,18 @@ int b200_attn_prefill(const void* q, const void* k, const void* v, const void* m
                       const int64_t q_strides[3], const int64_t k_strides[3], const int64_t v_strides[3],
                       int64_t mask_b, int64_t mask_t, float scale, int dtype, void* stream);
 
+/* b200_attn_prefill with what b200_mask_tiles found in this mask (mask: the same pointer, strides and sizes; the states
+ * count B = 1 when mask_b is 0).  The layers of a network share one mask: it is then looked through once per call and
+ * not by every head of every layer.  tiles may be NULL (each block looks at its own rows). */
+int b200_attn_prefill_tiles(const void* q, const void* k, const void* v, const void* mask, const void* tiles, void* out,
+                            int64_t B, int Hq, int Hkv, int64_t T, int64_t S, int D, const int64_t q_strides[3],
+                            const int64_t k_strides[3], const int64_t v_strides[3], int64_t mask_b, int64_t mask_t,
+                            float scale, int dtype, void* stream);
+/* One byte per 128 x 128 tile of an additive mask [B, T, S] (element strides mask_b, mask_t, 1), tiles[B][ceil(T/128)][ceil(S/128)]:
+ * 0 no element above -1e30, 1 all elements zero, 2 anything else. */
+int b200_mask_tiles(const void* mask, int64_t B, int64_t T, int64_t S, int64_t mask_b, int64_t mask_t, int dtype,
+                    void* tiles, void* stream);
+
 #ifdef __cplusplus
 }
 #endif

@@ -777,6 +777,13 @@ extern "C" int b200_attn_prefill(const void* q, const void* k, const void* v, co
                                  int Hkv, int64_t T, int64_t S, int D, const int64_t q_strides[3], const int64_t k_strides[3],
                                  const int64_t v_strides[3], int64_t mask_b, int64_t mask_t, float scale, int dtype,
                                  void* stream) {
+  return b200_attn_prefill_tiles(q, k, v, mask, nullptr, out, B, Hq, Hkv, T, S, D, q_strides, k_strides, v_strides, mask_b, mask_t, scale, dtype, stream);
+}
+
+extern "C" int b200_attn_prefill_tiles(const void* q, const void* k, const void* v, const void* mask, const void* tiles, void* out,
+                                       int64_t B, int Hq, int Hkv, int64_t T, int64_t S, int D, const int64_t q_strides[3],
+                                       const int64_t k_strides[3], const int64_t v_strides[3], int64_t mask_b, int64_t mask_t,
+                                       float scale, int dtype, void* stream) {
   B200_CHECK_ARG(q && k && v && out && B >= 0 && Hq > 0 && Hkv > 0 && T >= 0 && S > 0 && q_strides && k_strides && v_strides,
                  "b200_attn_prefill: bad arguments");
   B200_CHECK_ARG(D == HD, "b200_attn_prefill: head_dim %d not supported (128 only)", D);
@@ -789,7 +796,7 @@ extern "C" int b200_attn_prefill(const void* q, const void* k, const void* v, co
   PrefillParams p;
   p.q = q; p.k = k; p.v = v; p.mask = mask; p.out = out; p.B = B; p.T = T; p.S = S; p.Hq = Hq; p.Hkv = Hkv;
   for (int i = 0; i < 3; ++i) { p.qs[i] = q_strides[i]; p.ks[i] = k_strides[i]; p.vs[i] = v_strides[i]; }
-  p.mask_b = mask_b; p.mask_t = mask_t; p.scale = scale; p.mask_dtype = dtype;
+  p.tiles = static_cast<const uint8_t*>(tiles); p.mask_b = mask_b; p.mask_t = mask_t; p.scale = scale; p.mask_dtype = dtype;
   p.mask_staged = (mask && aligned16(mask) && mask_b % 8 == 0 && mask_t % 8 == 0 && S % 8 == 0) ? 1 : 0;   // mask dtype == activation dtype by contract
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   if (tc5_enabled()) {   // tcgen05 kernel first; the mma.sync kernel below takes what it cannot (odd strides, other mask types)

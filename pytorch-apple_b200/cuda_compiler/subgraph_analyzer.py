@@ -54,7 +54,7 @@ FLOAT_DTYPES = ("float32", "float16", "bfloat16")
 DTYPE_BYTES = {"float32": 4, "float16": 2, "bfloat16": 2, "int32": 4, "int64": 8, "bool": 1, "uint8": 1}
 MAX_CHAIN_OPS = 12
 MAX_CHAIN_INPUTS = 4
-MAX_TENSOR_MAP_KEYS = 32768   # keys of the tensor-map prefill attention (a verdict per 64 of them in shared memory)
+MAX_TENSOR_MAP_KEYS = 32768   # keys of the tensor-map prefill attention (a state per 128 of them in shared memory)
 
 
 def infer_compute_dtype(graph: IRGraph, requested: str | None) -> str:

@@ -24,6 +24,8 @@ EPI_SILU_MUL = 2
 EPI_GLU = 4
 EPI_W_STATIC = 8
 
+MASK_TILE = 128   # rows and keys of a tile of b200_mask_tiles
+
 
 class Tensor(C.Structure):
     """``b200_tensor``."""
@@ -77,6 +79,8 @@ SIGNATURES = {
     "b200_attn_decode": (_i, [_vp, _vp, _vp, _vp, _vp, _i64, _i, _i, _i64, _i, _i64, _i64, _i64, _i64, _f, _i, _vp, _i64, _vp]),
     "b200_attn_decode_noalloc": (_i, [_vp, _vp, _vp, _vp, _vp, _i64, _i, _i, _i64, _i, _i64, _i64, _i64, _i64, _f, _i, _vp]),
     "b200_attn_decode_workspace_bytes": (_i64, [_i64, _i, _i, _i64, _i]),
+    "b200_attn_prefill_tiles": (_i, [_vp, _vp, _vp, _vp, _vp, _vp, _i64, _i, _i, _i64, _i64, _i, _I64P, _I64P, _I64P, _i64, _i64, _f, _i, _vp]),
+    "b200_mask_tiles": (_i, [_vp, _i64, _i64, _i64, _i64, _i64, _i, _vp, _vp]),
     "b200_attn_prefill": (_i, [_vp, _vp, _vp, _vp, _vp, _i64, _i, _i, _i64, _i64, _i, _I64P, _I64P, _I64P, _i64, _i64, _f, _i, _vp]),
 }
 

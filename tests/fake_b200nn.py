@@ -431,3 +431,23 @@ class FakeLibrary:
         o = self._attn(Q, K, Vv, M, scale, dt)
         _raw(out, dt, [B, T, Hq, D], [T * Hq * D, Hq * D, D, 1]).copy_(o.transpose(1, 2).to(dt))
         return 0
+
+    def b200_mask_tiles(self, mask, B, T, S, mask_b, mask_t, dtype, tiles, stream):
+        self.calls.append("mask_tiles")
+        M = _raw(mask, _DT[dtype], [B, T, S], [mask_b, mask_t, 1]).float()
+        rows, cols = -(-T // 128), -(-S // 128)
+        out = _raw(tiles, torch.uint8, [B, rows, cols], [rows * cols, cols, 1])
+        for i in range(rows):
+            for j in range(cols):
+                t = M[:, i * 128:(i + 1) * 128, j * 128:(j + 1) * 128].flatten(1)
+                out[:, i, j] = torch.where((t > -1e30).any(1), torch.where((t == 0).all(1), 1, 2), 0).to(torch.uint8)
+        return 0
+
+    def b200_attn_prefill_tiles(self, q, k, v, mask, tiles, out, B, Hq, Hkv, T, S, D, qs, ks, vs, mask_b, mask_t, scale, dtype, stream):
+        if _addr(tiles):   # the states belong to this mask
+            want = torch.empty(B, -(-T // 128), -(-S // 128), dtype=torch.uint8)
+            nb = 1 if mask_b == 0 else B
+            self.b200_mask_tiles(mask, nb, T, S, mask_b, mask_t, dtype, want.data_ptr(), stream)
+            self.calls.pop()
+            assert torch.equal(want[:nb], _raw(tiles, torch.uint8, [nb, *want.shape[1:]], want.stride()))
+        return self.b200_attn_prefill(q, k, v, mask, out, B, Hq, Hkv, T, S, D, qs, ks, vs, mask_b, mask_t, scale, dtype, stream)

@@ -575,6 +575,97 @@ def test_attn_prefill_row_quarters_out_of_step(lib, slow, S):
         assert (err <= (size + want.abs()) * 2.0 ** -8 * 1.01 + 1e-5).all(), float(err.max())
 
 
+def _mask_of(kind, B, T, S, dtype):
+    """[B, T, S] additive masks: all, some or none of the 128 x 128 tiles are masked, zero or mixed."""
+    neg = torch.finfo(dtype).min
+    r, c = torch.arange(T)[:, None], torch.arange(S)[None]
+    m = torch.zeros(B, T, S)
+    if kind == "causal":
+        m[:] = torch.where(c <= r + S - T, 0.0, neg)
+    elif kind == "bias":             # finite values everywhere
+        m[:] = -0.02 * (r - c).abs()
+    elif kind == "holes":            # whole tiles masked, rows without any key, a tile with one key, infinities
+        m[:, :, 128:256] = neg
+        m[:, : T // 2, 256:384] = float("-inf")
+        m[:, T // 3, :] = neg
+        m[0, T - 1, 200 % S] = 0
+    elif kind == "late":             # the first key tile (and more) is not wanted
+        m[:, :, : min(S - 1, 300)] = neg
+    elif kind == "first":            # only the first key tile; the last sequence sees everything but the last key
+        m[:, :, 128:] = neg
+        m[-1, :, :] = 0
+        m[-1, :, S - 1:] = neg
+    return m.to(dtype)
+
+
+@pytest.mark.parametrize("kind", ["causal", "bias", "holes", "first", "late"])
+@pytest.mark.parametrize("B,T,S", [(1, 1, 128), (1, 2, 129), (2, 127, 255), (1, 128, 1), (2, 129, 384), (1, 300, 640), (1, 64, 1111)])
+@pytest.mark.parametrize("rows", ["aligned", "dense", "shared", "one row"])
+def test_attn_prefill_mask_tiles(lib, kind, B, T, S, rows):
+    """Mask tiles that are masked, zero or mixed, in every form of addressing, with the states found beforehand and by the
+    kernel itself: both equal float64 within the rounding of probabilities and outputs to bf16 (2^-8 of what is added up,
+    fp32 elsewhere), and rows that attend to nothing give zeros."""
+    dtype, Hq, Hkv, D = torch.bfloat16, 4, 2, 128
+    q, k, v = gen((B, Hq, T, D), dtype), gen((B, Hkv, S, D), dtype, 1), gen((B, Hkv, S, D), dtype, 2)
+    mask = _mask_of(kind, B, T, S, dtype)
+    pitch = -(-S // 8) * 8 if rows == "aligned" else S
+    if rows == "shared":
+        mask = mask[-1:]
+    if rows == "one row":
+        mask = mask[:, -1:]
+    M = torch.full((mask.shape[0], mask.shape[1], pitch), float("nan"), dtype=dtype, device="cuda")
+    M[..., :S] = mask.cuda()
+    mb, mt = (0 if rows == "shared" else M.stride(0)), (0 if rows == "one row" else pitch)
+    nb = 1 if rows == "shared" else B
+    tiles = torch.full((nb, -(-T // 128), -(-S // 128)), 9, dtype=torch.uint8, device="cuda")
+    ok(lib, lib.b200_mask_tiles(M.data_ptr(), nb, T, S, mb, mt, 2, tiles.data_ptr(), stream()))
+    full = mask.double().expand(B, T, S)
+    for i in range(tiles.shape[1]):
+        for j in range(tiles.shape[2]):
+            t = full[:nb, i * 128:(i + 1) * 128, j * 128:(j + 1) * 128].flatten(1)
+            want = torch.where((t > -1e30).any(1), torch.where((t == 0).all(1), 1, 2), 0)
+            assert tiles[:, i, j].tolist() == want.tolist(), (i, j)
+    s = (q.double() @ k.double().repeat_interleave(Hq // Hkv, 1).transpose(2, 3)) * D ** -0.5 + full[:, None].clamp(min=-1e300)
+    dead = (full <= -1e30).all(-1)
+    p = s.softmax(-1) * ~dead[:, None, :, None]
+    vd = v.double().repeat_interleave(Hq // Hkv, 1)
+    want, size = (p @ vd).transpose(1, 2), (p @ vd.abs()).transpose(1, 2)
+    Q, K, V = q.cuda(), k.cuda(), v.cuda()
+    st = lambda t: (C.c_int64 * 3)(*t.stride()[:3])
+    got = []
+    for states in (None, tiles.data_ptr()):
+        out = torch.full((B, T, Hq, D), float("nan"), dtype=dtype, device="cuda")
+        ok(lib, lib.b200_attn_prefill_tiles(Q.data_ptr(), K.data_ptr(), V.data_ptr(), M.data_ptr(), states, out.data_ptr(), B, Hq, Hkv, T, S, D,
+                                            st(Q), st(K), st(V), mb, mt, D ** -0.5, 2, stream()))
+        err = (out.double().cpu() - want).abs()
+        assert (err <= (size + want.abs()) * 2.0 ** -8 * 1.01 + 1e-5).all(), float(err.max())
+        got.append(out)
+    assert torch.equal(*got)
+    code = C.c_int(0)
+    ok(lib, lib.b200_debug_device_error(C.byref(code), 1))
+    assert code.value == 0
+
+
+@pytest.mark.parametrize("T", [128, 400])
+def test_attn_prefill_many_launches_in_a_row(lib, T):
+    """The first key tile is requested before it is known to be wanted, so its scores may be complete before the producer
+    looks at the stage again: a few hundred launches, all equal, no wait that runs out."""
+    dtype, Hq, Hkv, D = torch.bfloat16, 12, 2, 128
+    Q, K, V = gen((1, Hq, T, D), dtype).cuda(), gen((1, Hkv, T, D), dtype, 1).cuda(), gen((1, Hkv, T, D), dtype, 2).cuda()
+    M = _mask_of("causal", 1, T, T, dtype).cuda()
+    tiles = torch.empty(1, -(-T // 128), -(-T // 128), dtype=torch.uint8, device="cuda")
+    ok(lib, lib.b200_mask_tiles(M.data_ptr(), 1, T, T, 0, T, 2, tiles.data_ptr(), stream()))
+    st = lambda t: (C.c_int64 * 3)(*t.stride()[:3])
+    outs = [torch.empty((1, T, Hq, D), dtype=dtype, device="cuda") for _ in range(200)]
+    for out in outs:
+        ok(lib, lib.b200_attn_prefill_tiles(Q.data_ptr(), K.data_ptr(), V.data_ptr(), M.data_ptr(), tiles.data_ptr(), out.data_ptr(), 1, Hq, Hkv,
+                                            T, T, D, st(Q), st(K), st(V), 0, T, D ** -0.5, 2, stream()))
+    assert all(torch.equal(outs[0], out) for out in outs[1:])
+    code = C.c_int(0)
+    ok(lib, lib.b200_debug_device_error(C.byref(code), 1))
+    assert code.value == 0
+
+
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
 def test_attn_prefill_arbitrary_masks_and_no_mask(lib, dtype):
     """Nothing in the kernels assumes a causal mask: a per-sequence mask with windows, holes and key
