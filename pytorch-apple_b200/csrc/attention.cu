@@ -69,10 +69,16 @@ constexpr int DEC_ACC_PITCH = HD + 4;          // row pitch of the cross-warp ac
 // CTA stores head h's partial (accumulator, max, sum) into the receive buffer of cluster rank h
 // (distributed shared memory); after one cluster barrier every rank combines the splits of the
 // heads it owns (head h belongs to rank h % splits) and writes the final output.  2 <= splits <= 16.
-template <typename T, int STAGES, bool CM>
-__global__ void __launch_bounds__(128, STAGES == 2 ? 3 : 2) attn_decode_kernel(const __grid_constant__ DecodeParams p) {
+//
+// NW = 8 warps instead of 4, one CTA per SM, where all clusters are resident even so (up to three sequences) and a split has
+// more than four blocks: what a warp does with its blocks one after the other is then half as long.  us, one sequence: 4097 keys
+// 7.7 -> 6.3, 8000 keys 9.9 -> 7.2, 16000 keys 16.8 -> 11.0, 1111 keys (80 per split) 4.6 -> 4.3, 790 keys (64 per split) would
+// lose, 3.9 -> 4.2; three sequences of 4097 8.3 -> 7.4.  With a second wave of clusters it loses (four: 13.6), and a third ring
+// stage for four warps gains nothing (7.8, 8.6): this is not the memory's latency.
+template <typename T, int STAGES, bool CM, int NW = 4>
+__global__ void __launch_bounds__(NW * 32, NW == 8 ? 1 : STAGES == 2 ? 3 : 2) attn_decode_kernel(const __grid_constant__ DecodeParams p) {
   extern __shared__ __align__(1024) uint8_t dsm[];
-  __shared__ float s_m[4][8], s_l[4][8];
+  __shared__ float s_m[NW][8], s_l[NW][8];
   // partials of the heads this CTA owns (head h belongs to cluster rank h % splits), by [owned head * splits + source rank]
   __shared__ __align__(16) float recv_acc[CM ? 16 : 1][HD];
   __shared__ float recv_ml[CM ? 16 : 1][2];
@@ -136,27 +142,27 @@ __global__ void __launch_bounds__(128, STAGES == 2 ? 3 : 2) attn_decode_kernel(c
   if (cur >= 0) issue(cur, 0);
   cp_async_commit();
   if (STAGES > 2) {
-    nxt = warp + 4 < nblk ? warp + 4 : -1;
+    nxt = warp + NW < nblk ? warp + NW : -1;
     if (nxt >= 0) issue(nxt, 1);
     cp_async_commit();
   }
 
-  // ---- which of this warp's blocks have an unmasked key: bit j <-> block warp + 4j ----
+  // ---- which of this warp's blocks have an unmasked key: bit j <-> block warp + NW j ----
   const char* mask_row = p.mask ? static_cast<const char*>(p.mask) : nullptr;
   const int64_t mask_base = b * p.mask_bs + s_begin;
   uint32_t vbits = 0;
 #pragma unroll
-  for (int i = 0; i < DEC_MAX_SPLIT / 128; ++i) {
-    if (i * 128 >= n_keys) break;   // (uniform) every pass covers 128 keys of the split
-    const int idx = i * 32 + lane, blk = warp + 4 * (idx >> 4), key = blk * 16 + (idx & 15);
+  for (int i = 0; i < DEC_MAX_SPLIT / (NW * 32); ++i) {
+    if (i * NW * 32 >= n_keys) break;   // (uniform) every pass covers NW * 32 keys of the split
+    const int idx = i * 32 + lane, blk = warp + NW * (idx >> 4), key = blk * 16 + (idx & 15);
     float mv = -INFINITY;
     if (key < n_keys) mv = mask_row ? load_as_f32(mask_row, mask_base + key, p.mask_dtype) : 0.f;
     const uint32_t bal = __ballot_sync(0xffffffffu, mv > MASKED);
     vbits |= ((bal & 0xffffu) ? 1u : 0u) << (2 * i) | ((bal >> 16) ? 1u : 0u) << (2 * i + 1);
   }
-  auto is_valid = [&](int blk) { return ((vbits >> ((blk - warp) >> 2)) & 1u) != 0u; };
-  auto next_valid = [&](int blk) {  // first valid block of this warp at or after blk (stride 4)
-    while (blk < nblk && !is_valid(blk)) blk += 4;
+  auto is_valid = [&](int blk) { return ((vbits >> ((blk - warp) / NW)) & 1u) != 0u; };
+  auto next_valid = [&](int blk) {  // first valid block of this warp at or after blk (stride NW)
+    while (blk < nblk && !is_valid(blk)) blk += NW;
     return blk;
   };
 
@@ -183,7 +189,7 @@ __global__ void __launch_bounds__(128, STAGES == 2 ? 3 : 2) attn_decode_kernel(c
     return mask_row ? load_as_f32(mask_row, mask_base + key, p.mask_dtype) * LOG2E : 0.f;
   };
 
-  int fetch = next_valid(warp + (STAGES > 2 ? 8 : 4));   // next block to copy
+  int fetch = next_valid(warp + (STAGES > 2 ? 2 * NW : NW));   // next block to copy
   int st_fetch = STAGES > 2 ? 2 : 1, st_use = 0;
   while (cur >= 0) {
     int fetched = -1;
@@ -193,7 +199,7 @@ __global__ void __launch_bounds__(128, STAGES == 2 ? 3 : 2) attn_decode_kernel(c
       if (fetch < nblk) {
         issue(fetch, st_fetch);
         fetched = fetch;
-        fetch = next_valid(fetch + 4);
+        fetch = next_valid(fetch + NW);
       }
       cp_async_commit();
       st_fetch = (st_fetch + 1) % STAGES;
@@ -202,7 +208,7 @@ __global__ void __launch_bounds__(128, STAGES == 2 ? 3 : 2) attn_decode_kernel(c
       if (fetch < nblk) {
         issue(fetch, st_fetch);
         fetched = fetch;
-        fetch = next_valid(fetch + 4);
+        fetch = next_valid(fetch + NW);
       }
       cp_async_commit();
       st_fetch ^= 1;
@@ -279,14 +285,16 @@ __global__ void __launch_bounds__(128, STAGES == 2 ? 3 : 2) attn_decode_kernel(c
   if (g == 0) { s_m[warp][2 * t] = m0; s_m[warp][2 * t + 1] = m1; s_l[warp][2 * t] = l0; s_l[warp][2 * t + 1] = l1; }
   __syncthreads();
   const int64_t pidx = ((b * p.Hkv + hk) * p.splits + split) * p.G;
-  const int d = threadIdx.x;
+  const int d = threadIdx.x & (HD - 1), part = threadIdx.x / HD;   // (with eight warps the heads are dealt to two threads per dim)
 #pragma unroll 1
-  for (int h = 0; h < p.G; ++h) {
-    const float ma = fmaxf(fmaxf(s_m[0][h], s_m[1][h]), fmaxf(s_m[2][h], s_m[3][h]));
+  for (int h = part; h < p.G; h += NW / 4) {
+    float ma = s_m[0][h];
+#pragma unroll
+    for (int wi = 1; wi < NW; ++wi) ma = fmaxf(ma, s_m[wi][h]);
     const float mu = ma == -INFINITY ? 0.f : ma;
     float acc = 0.f, lr = 0.f;
 #pragma unroll
-    for (int wi = 0; wi < 4; ++wi) {
+    for (int wi = 0; wi < NW; ++wi) {
       const float f = ex2_approx(s_m[wi][h] - mu);
       acc += reinterpret_cast<const float*>(dsm + wi * (STAGES * DEC_STAGE_BYTES))[h * DEC_ACC_PITCH + d] * f;
       lr += s_l[wi][h] * f;
@@ -309,7 +317,7 @@ __global__ void __launch_bounds__(128, STAGES == 2 ? 3 : 2) attn_decode_kernel(c
   }
   if (CM) {
     tc5::cluster_sync();   // all partials have landed; nobody touches a peer's memory afterwards
-    for (int h = split; h < p.G; h += p.splits) {   // the heads this CTA owns
+    for (int h = split + part * p.splits; h < p.G; h += p.splits * (NW / 4)) {   // the heads this CTA owns
       const int base = (h / p.splits) * p.splits;
       float m_all = -INFINITY;
       for (int r = 0; r < p.splits; ++r) m_all = fmaxf(m_all, recv_ml[base + r][0]);
@@ -682,37 +690,37 @@ extern "C" int b200_attn_decode(const void* q, const void* k, const void* v, con
   if (B == 0) return B200_OK;
   if (!(aligned16(q) && aligned16(k) && aligned16(v) && q_batch_stride % 8 == 0 && kv_batch_stride % 8 == 0 && kv_head_stride % 8 == 0))
     B200_FAIL(B200_EALIGN, "b200_attn_decode: operands must be 16-byte aligned with strides multiple of 8");
-  // clusters of 16 CTAs are a non-portable size: how many the device keeps resident at once is asked once per device
-  // (0 = not asked yet, -1 = not available)
-  static PerDevice<int> resident16_on;
-  int* resident16 = resident16_on.slot();
+  // clusters of 16 CTAs are a non-portable size: how many the device keeps resident at once, with four and with eight warps
+  // per CTA, is asked once per device (0 = not asked yet, -1 = not available)
+  struct Resident16 { int n4, n8; };
+  static PerDevice<Resident16> resident16_on;
+  Resident16* resident16 = resident16_on.slot();
   if (!resident16) B200_FAIL(B200_ELAUNCH, "attn_decode_kernel: no current device");
-  if (*resident16 == 0) {
-    *resident16 = -1;
-    int n16 = 0;
-    bool ok16 = true;
-    // (the attribute is per kernel instantiation: both activation types get it, whichever asks first)
-    ok16 = cudaFuncSetAttribute(attn_decode_kernel<__nv_bfloat16, 2, true>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess &&
-           cudaFuncSetAttribute(attn_decode_kernel<__half, 2, true>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess;
-    B200_DISPATCH_HALF(dtype, T, {
-      ok16 = ok16 && cudaFuncSetAttribute(attn_decode_kernel<T, 2, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 4 * 2 * DEC_STAGE_BYTES) == cudaSuccess;
-      if (ok16) {
-        cudaLaunchConfig_t qc = {};
-        qc.gridDim = dim3(16, 1, 1);
-        qc.blockDim = dim3(128);
-        qc.dynamicSmemBytes = 4 * 2 * DEC_STAGE_BYTES;
-        cudaLaunchAttribute ca;
-        ca.id = cudaLaunchAttributeClusterDimension;
-        ca.val.clusterDim.x = 16; ca.val.clusterDim.y = 1; ca.val.clusterDim.z = 1;
-        qc.attrs = &ca;
-        qc.numAttrs = 1;
-        ok16 = cudaOccupancyMaxActiveClusters(&n16, attn_decode_kernel<T, 2, true>, &qc) == cudaSuccess && n16 >= 1;
-      }
-    });
+  if (resident16->n4 == 0) {
+    // (the attributes are per kernel instantiation: both activation types get them, whichever asks first)
+    const auto ask = [](auto kernel, auto other, int warps) {
+      for (const void* f : {reinterpret_cast<const void*>(kernel), reinterpret_cast<const void*>(other)})
+        if (cudaFuncSetAttribute(f, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess ||
+            cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, warps * 2 * DEC_STAGE_BYTES) != cudaSuccess)
+          return -1;
+      cudaLaunchConfig_t qc = {};
+      qc.gridDim = dim3(16, 1, 1);
+      qc.blockDim = dim3(static_cast<unsigned>(warps) * 32);
+      qc.dynamicSmemBytes = warps * 2 * DEC_STAGE_BYTES;
+      cudaLaunchAttribute ca;
+      ca.id = cudaLaunchAttributeClusterDimension;
+      ca.val.clusterDim.x = 16; ca.val.clusterDim.y = 1; ca.val.clusterDim.z = 1;
+      qc.attrs = &ca;
+      qc.numAttrs = 1;
+      int n = 0;
+      return cudaOccupancyMaxActiveClusters(&n, kernel, &qc) == cudaSuccess && n >= 1 ? n : -1;
+    };
+    resident16->n8 = ask(attn_decode_kernel<__nv_bfloat16, 2, true, 8>, attn_decode_kernel<__half, 2, true, 8>, 8);
+    resident16->n4 = ask(attn_decode_kernel<__nv_bfloat16, 2, true>, attn_decode_kernel<__half, 2, true>, 4);
     cudaGetLastError();
-    if (ok16) *resident16 = n16;
   }
-  const DecodePlan d = plan_decode(B, Hkv, S, Hq / Hkv, *resident16);
+  const DecodePlan d = plan_decode(B, Hkv, S, Hq / Hkv, resident16->n4);
+  const bool eight_warps = d.cluster && d.splits > 8 && d.split_len > 64 && B * Hkv <= resident16->n8;
   const int64_t need = b200_attn_decode_workspace_bytes(B, Hq, Hkv, S, D);
   if (need > 0 && (!workspace || workspace_bytes < need))
     B200_FAIL(B200_EINVAL, "b200_attn_decode: workspace of %lld bytes required (got %lld)", (long long)need, (long long)workspace_bytes);
@@ -740,8 +748,9 @@ extern "C" int b200_attn_decode(const void* q, const void* k, const void* v, con
     if (d.cluster) {   // one kernel: the splits of a (sequence, KV head) are a cluster along x and merge in shared memory
       cudaLaunchConfig_t cfg = {};
       cfg.gridDim = grid;
-      cfg.blockDim = dim3(128);
-      cfg.dynamicSmemBytes = 4 * 2 * DEC_STAGE_BYTES;
+      const int warps = eight_warps ? 8 : 4;
+      cfg.blockDim = dim3(static_cast<unsigned>(warps) * 32);
+      cfg.dynamicSmemBytes = warps * 2 * DEC_STAGE_BYTES;
       cfg.stream = st;
       cudaLaunchAttribute attrs[2];
       int n_attrs = 0;
@@ -757,7 +766,8 @@ extern "C" int b200_attn_decode(const void* q, const void* k, const void* v, con
       }
       cfg.attrs = attrs;
       cfg.numAttrs = n_attrs;
-      cudaLaunchKernelEx(&cfg, attn_decode_kernel<T, 2, true>, p);
+      if (eight_warps) cudaLaunchKernelEx(&cfg, attn_decode_kernel<T, 2, true, 8>, p);
+      else cudaLaunchKernelEx(&cfg, attn_decode_kernel<T, 2, true>, p);
     } else {
       launch_pdl(attn_decode_kernel<T, 2, false>, grid, dim3(128), 4 * 2 * DEC_STAGE_BYTES, st, p);
       const auto merge = [&](auto kernel, int groups, int dims) {

@@ -466,6 +466,36 @@ def test_attn_decode_small_batches_in_both_dtypes(lib, dtype, B):
     close(out, ref, rtol=2e-2, atol=5e-3)
 
 
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("Hq,Hkv", [(12, 2), (7, 7), (8, 1)])
+@pytest.mark.parametrize("B,S", [(1, 1024), (1, 1040), (3, 1111), (1, 4352), (4, 2048), (1, 16383)])
+def test_attn_decode_eight_warps(lib, dtype, Hq, Hkv, B, S):
+    """Few sequences with more than 64 keys per split take eight warps per CTA: on both sides of that line and of the number
+    of clusters that fit, masks with a filled prefix, with holes, with one key; against float64 within the rounding
+    of probabilities and outputs (2^-8 of what is added up in bf16, 2^-11 in fp16; fp32 elsewhere)."""
+    D, neg = 128, torch.finfo(dtype).min
+    q, k, v = gen((B, Hq, 1, D), dtype), gen((B, Hkv, S, D), dtype, 1), gen((B, Hkv, S, D), dtype, 2)
+    g = torch.Generator().manual_seed(S)
+    mask = torch.zeros(B, 1, 1, S)
+    mask[0, ..., (3 * S) // 4:] = neg
+    if B > 1:
+        mask[1] = torch.where(torch.rand(S, generator=g) < 0.3, 0.0, neg)
+    if B > 2:
+        mask[2] = neg
+        mask[2, ..., S - 1] = 0
+    mask = mask.to(dtype)
+    s = (q.double() @ k.double().repeat_interleave(Hq // Hkv, 1).transpose(2, 3)) * D ** -0.5 + mask.double()
+    p, vd = s.softmax(-1), v.double().repeat_interleave(Hq // Hkv, 1)
+    want, size = (p @ vd)[:, :, 0], (p @ vd.abs())[:, :, 0]
+    Q, K, V, M = q.cuda(), k.cuda(), v.cuda(), mask.cuda()
+    out = torch.full((B, Hq, D), float("nan"), dtype=dtype, device="cuda")
+    ok(lib, lib.b200_attn_decode(Q.data_ptr(), K.data_ptr(), V.data_ptr(), M.data_ptr(), out.data_ptr(), B, Hq, Hkv, S, D, Hq * D,
+                                 Hkv * S * D, S * D, S, D ** -0.5, DT[dtype], None, 0, stream()))
+    eps = 2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -11
+    err = (out.double().cpu() - want).abs()
+    assert (err <= (size + want.abs()) * eps * 1.01 + 1e-5).all(), float(err.max())
+
+
 @pytest.mark.parametrize("B,S,Hq,Hkv", [(40, 2048, 12, 2), (64, 4352, 12, 2), (33, 1000, 8, 1), (130, 640, 4, 4)])
 def test_attn_decode_many_sequences_ragged_masks(lib, B, S, Hq, Hkv):
     """Batches large enough for the balanced kernel (every CTA gets the same number of unmasked 16-key
