@@ -1481,8 +1481,8 @@ bool make_map(CUtensorMap* map, const void* base, int64_t rows, int64_t K, int64
 
 // Tiled tensor map of up to five dimensions with a 128-byte swizzle (dims / box innermost first,
 // strides in bytes for dimensions 1..rank-1).  Used by kernels outside this file.
-bool tma_encode_sw128(CUtensorMap* map, int dtype, int rank, const void* base, const uint64_t* dims, const uint64_t* strides_bytes,
-                      const uint32_t* box) {
+static bool tma_encode(CUtensorMap* map, int dtype, int rank, const void* base, const uint64_t* dims, const uint64_t* strides_bytes,
+                       const uint32_t* box, CUtensorMapSwizzle swizzle) {
   EncodeTiledFn fn = encode_fn();
   if (!fn || rank < 1 || rank > 5) return false;
   cuuint64_t d[5], st[4];
@@ -1491,7 +1491,15 @@ bool tma_encode_sw128(CUtensorMap* map, int dtype, int rank, const void* base, c
   for (int i = 0; i + 1 < rank; ++i) st[i] = strides_bytes[i];
   const CUtensorMapDataType dt = dtype == B200_BF16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16;
   return fn(map, dt, static_cast<cuuint32_t>(rank), const_cast<void*>(base), d, st, bx, es, CU_TENSOR_MAP_INTERLEAVE_NONE,
-            CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+            swizzle, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+bool tma_encode_sw128(CUtensorMap* map, int dtype, int rank, const void* base, const uint64_t* dims, const uint64_t* strides_bytes,
+                      const uint32_t* box) {
+  return tma_encode(map, dtype, rank, base, dims, strides_bytes, box, CU_TENSOR_MAP_SWIZZLE_128B);
+}
+bool tma_encode_plain(CUtensorMap* map, int dtype, int rank, const void* base, const uint64_t* dims, const uint64_t* strides_bytes,
+                      const uint32_t* box) {
+  return tma_encode(map, dtype, rank, base, dims, strides_bytes, box, CU_TENSOR_MAP_SWIZZLE_NONE);
 }
 
 namespace {
@@ -2118,8 +2126,8 @@ extern "C" int b200_debug_device_error(int* code, int clear) {
   int v = 0;
   cudaError_t e = cudaMemcpyFromSymbol(&v, b200::g_tc5_error, sizeof(int));
   if (e != cudaSuccess) B200_FAIL(B200_ELAUNCH, "b200_debug_device_error: %s", cudaGetErrorString(e));
-  const int att = b200::attn_prefill_tc5_error(clear != 0);
-  if (code) *code = v ? v : (att > 0 ? att : 0);
+  const int att = b200::attn_prefill_tc5_error(clear != 0), stem = b200::conv_stem_error(clear != 0);
+  if (code) *code = v ? v : att > 0 ? att : stem > 0 ? stem : 0;
   if (clear && v) {
     v = 0;
     cudaMemcpyToSymbol(b200::g_tc5_error, &v, sizeof(int));

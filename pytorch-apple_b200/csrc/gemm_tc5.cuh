@@ -56,6 +56,8 @@ struct Tc5Conv {
 // (stem convolution after channel padding) with O <= 64.
 // Args: A = x [N,H,W,C], W = packed weights [O, KH*KW*C], M = N*Ho*Wo, N = O, K = KH*KW*C.
 int conv_tc5(const Tc5Args& a, const Tc5Conv& g, cudaStream_t stream);
+// code left by a bounded wait of the stem + pooling kernel (conv_stem.cu) that ran out (0 = none); optionally cleared
+int conv_stem_error(bool clear);
 
 // out = epi(A W^T + bias + residual) on the tcgen05 path.  Returns B200_ENOTSUP when the
 // operands do not meet the TMA alignment rules (the caller then uses the mma.sync tiles).

@@ -11,6 +11,8 @@ namespace b200 {
 // host: tiled tensor map with 128-byte swizzle (implemented in gemm_tc5.cu)
 bool tma_encode_sw128(CUtensorMap* map, int dtype, int rank, const void* base, const uint64_t* dims, const uint64_t* strides_bytes,
                       const uint32_t* box);
+bool tma_encode_plain(CUtensorMap* map, int dtype, int rank, const void* base, const uint64_t* dims, const uint64_t* strides_bytes,
+                      const uint32_t* box);   // the same without swizzle
 
 namespace tc5 {
 

@@ -49,6 +49,59 @@ def _mask_key(m: TensorView) -> tuple:
     return (m.buffer, m.offset, 1 if m.strides[0] == 0 else B, T, S, m.strides[0], m.strides[2])
 
 
+def _views_of(value):
+    """Every TensorView in a step's parameters."""
+    if isinstance(value, TensorView):
+        yield value
+    elif isinstance(value, dict):
+        for v in value.values():
+            yield from _views_of(v)
+    elif isinstance(value, (list, tuple)):
+        for v in value:
+            yield from _views_of(v)
+
+
+def _find_stems(program: CUDAProgram, lib) -> dict[int, tuple | None]:
+    """Heads of convolution networks that run as one kernel: the repack of a planar graph input to channels-last, a convolution
+    of it, and a 3x3 / 2 max-pooling of the result, with nothing else reading what lies in between (256 images of a
+    ResNet: 600 us as three kernels, 173 as one).  {index of the pooling step: (repack, convolution, pooling) parameters, other two: None}."""
+    steps = [(i, s.params) for i, s in enumerate(program.steps) if getattr(s, "params", None)]
+    users: dict[str, list[int]] = {}
+    for i, p in steps:
+        for name in {v.buffer for v in _views_of(p)}:
+            users.setdefault(name, []).append(i)
+    for spec in program.output_specs:
+        view = program.views.get(spec.name)
+        if view is not None:
+            users.setdefault(view.buffer, []).append(-1)
+    inputs = {s.name for s in program.input_specs}
+    params, found = dict(steps), {}
+    for i, copy in steps:
+        if copy.get("op") != "strided_copy" or copy["in_view"].buffer not in inputs or len(copy["in_view"].shape) != 4:
+            continue
+        x, mid = copy["in_view"], copy["out_view"].buffer
+        others = [j for j in users[mid] if j != i]
+        conv = params.get(others[0]) if len(others) == 1 else None
+        if conv is None or conv.get("op") != "conv2d" or conv["x"].buffer != mid or conv["residual"] is not None:
+            continue
+        y = conv["y"]
+        others = [j for j in users[y.buffer] if j != others[0]] + [others[0]]
+        pool = params.get(others[0]) if len(others) == 2 else None
+        if pool is None or pool.get("op") != "max_pool2d" or pool["x"].buffer != y.buffer or pool["y"].buffer == y.buffer:
+            continue
+        N, Cn, H, W = x.shape
+        O, PH, PW = y.shape[1], (y.shape[2] - 1) // 2 + 1, (y.shape[3] - 1) // 2 + 1
+        cv = [conv[k] for k in ("c_pad", "out_channels", "kernel_h", "kernel_w", "stride_h", "stride_w", "pad_h", "pad_w")]
+        if (x.dtype == y.dtype == pool["y"].dtype and tuple(x.strides) == (Cn * H * W, H * W, W, 1) and tuple(copy["out_view"].shape) == tuple(x.shape)
+                and conv["x"].offset == copy["out_view"].offset and tuple(pool["x"].shape) == tuple(y.shape)
+                and tuple(pool["x"].strides) == tuple(y.strides) and pool["x"].offset == y.offset
+                and [pool[k] for k in ("kernel_h", "kernel_w", "stride_h", "stride_w", "pad_h", "pad_w")] == [3, 3, 2, 2, 1, 1]
+                and tuple(pool["y"].shape) == (N, O, PH, PW) and tuple(pool["y"].strides) == (PH * PW * O, 1, PW * O, O)
+                and pool["y"].offset % 8 == 0 and lib.b200_conv_stem_pool_supported(Cn, H, W, *cv, DTYPE_CODES[y.dtype])):
+            found.update({i: None, others[1]: None, others[0]: (copy, conv, pool)})
+    return found
+
+
 class _Plan:
     """Launch list bound to one set of buffer addresses."""
 
@@ -96,6 +149,7 @@ class CUDAExecutor:
                 key = _mask_key(p["mask"])
                 if key not in self._tiles:
                     self._tiles[key] = torch.empty(key[2] * -(-key[3] // MASK_TILE) * -(-key[4] // MASK_TILE), dtype=torch.uint8, device=self._device)
+        self._stems = _find_stems(program, self._lib)
         # split-K partial sums must start at zero; the kernel restores zeros before it exits
         self._ws = {"__ws_splitk": torch.zeros(max(ws_lin, 256), dtype=torch.uint8, device=self._device),
                     "__ws_attn": torch.empty(max(ws_att, 256), dtype=torch.uint8, device=self._device)}
@@ -378,11 +432,15 @@ class CUDAExecutor:
         self._cur_inputs = inputs
         self._cur_plan = plan
         self._staged: dict[str, Any] = {}
-        for step in self._program.steps:
+        for i, step in enumerate(self._program.steps):
             if isinstance(step, AliasStep):
                 continue
             p = step.params
-            getattr(self, "_bind_" + p["op"])(plan, step, p)
+            stem = self._stems.get(i, p)
+            if stem is p:
+                getattr(self, "_bind_" + p["op"])(plan, step, p)
+            elif stem is not None:
+                self._bind_stem_pool(plan, *stem)
         # every library call is one kernel, except decode attention when its splits are merged by a
         # second kernel (the library then asks for a workspace; with in-kernel merging it asks for none)
         def _two_kernels(q) -> bool:
@@ -633,6 +691,13 @@ class CUDAExecutor:
             self._ptr(x), self._prepared[p["w_prepared"]].data_ptr(), self._prepared[p["bias_prepared"]].data_ptr(), self._ptr(res),
             self._ptr(y), p["batch"], p["in_h"], p["in_w"], p["c_pad"], p["c_pad"], p["out_channels"], p["kernel_h"], p["kernel_w"],
             p["stride_h"], p["stride_w"], p["pad_h"], p["pad_w"], p["out_h"], p["out_w"], DTYPE_CODES[y.dtype], epi)))
+
+    def _bind_stem_pool(self, plan, copy, conv, pool):
+        x = copy["in_view"]
+        plan.launches.append((self._lib.b200_conv_stem_pool, (
+            self._ptr(x), self._prepared[conv["w_prepared"]].data_ptr(), self._prepared[conv["bias_prepared"]].data_ptr(), self._ptr(pool["y"]),
+            *x.shape, conv["c_pad"], conv["out_channels"], conv["kernel_h"], conv["kernel_w"], conv["stride_h"], conv["stride_w"], conv["pad_h"],
+            conv["pad_w"], DTYPE_CODES[x.dtype], native.EPI_RELU if conv["relu"] else 0)))
 
     def _bind_attention(self, plan, step, p):
         q, k, v, m, y = p["q"], p["k"], p["v"], p["mask"], p["y"]

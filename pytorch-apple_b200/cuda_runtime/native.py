@@ -76,6 +76,8 @@ SIGNATURES = {
                                   _vp]),
     "b200_matmul_strided": (_i, [_vp, _vp, _vp, _i64, _i64, _i64, _i64, _i64, _I64P, _I64P, _I64P, _i, _vp]),
     "b200_conv2d_nhwc": (_i, [_vp, _vp, _vp, _vp, _vp] + [_i] * 16 + [_vp]),
+    "b200_conv_stem_pool": (_i, [_vp, _vp, _vp, _vp] + [_i] * 14 + [_vp]),
+    "b200_conv_stem_pool_supported": (_i, [_i] * 12),
     "b200_attn_decode": (_i, [_vp, _vp, _vp, _vp, _vp, _i64, _i, _i, _i64, _i, _i64, _i64, _i64, _i64, _f, _i, _vp, _i64, _vp]),
     "b200_attn_decode_noalloc": (_i, [_vp, _vp, _vp, _vp, _vp, _i64, _i, _i, _i64, _i, _i64, _i64, _i64, _i64, _f, _i, _vp]),
     "b200_attn_decode_workspace_bytes": (_i64, [_i64, _i, _i, _i64, _i]),

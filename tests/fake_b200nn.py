@@ -451,3 +451,18 @@ class FakeLibrary:
             self.calls.pop()
             assert torch.equal(want[:nb], _raw(tiles, torch.uint8, [nb, *want.shape[1:]], want.stride()))
         return self.b200_attn_prefill(q, k, v, mask, out, B, Hq, Hkv, T, S, D, qs, ks, vs, mask_b, mask_t, scale, dtype, stream)
+
+    def b200_conv_stem_pool_supported(self, Cn, H, W, C_pad, O, KH, KW, sh, sw, ph, pw, dtype):
+        return int(1 <= Cn <= 4 and C_pad == 8 and 8 <= O <= 64 and O % 8 == 0 and 2 <= KH <= 8 and KW == 7 and sh == sw == 2 and pw == 3
+                   and 0 <= ph < KH and (W - 1) // 2 + 1 <= 128 and H + 2 * ph >= KH and dtype in (1, 2))
+
+    def b200_conv_stem_pool(self, x, w, bias, y, N, Cn, H, W, C_pad, O, KH, KW, sh, sw, ph, pw, dtype, epilogue, stream):
+        self.calls += ["conv2d", "max_pool2d"]
+        dt = _DT[dtype]
+        X = _raw(x, dt, [N, Cn, H, W], [Cn * H * W, H * W, W, 1]).float()
+        Wt = _raw(w, dt, [O, C_pad, KH, KW], [KH * KW * C_pad, 1, KW * C_pad, C_pad]).float()[:, :Cn]
+        r = torch.nn.functional.conv2d(X, Wt, _flat(bias, 0, O) if _addr(bias) else None, (sh, sw), (ph, pw))
+        r = torch.nn.functional.max_pool2d((torch.relu(r) if epilogue & 1 else r).to(dt).float(), 3, 2, 1)
+        PH, PW = r.shape[2:]
+        _raw(y, dt, [N, O, PH, PW], [PH * PW * O, 1, PW * O, O]).copy_(r.to(dt))
+        return 0

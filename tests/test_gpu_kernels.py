@@ -1109,3 +1109,41 @@ def test_argmax_rows_matches_and_breaks_ties_low(lib):
     ok(lib, lib.b200_argmax_rows(X.data_ptr(), out.data_ptr(), 9, 151936, 151936, 2, stream()))
     ref = torch.tensor([int(np.flatnonzero(r == r.max())[0]) for r in x.float().numpy()])
     assert torch.equal(out.cpu(), ref) and out[3] == 77
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("N,Cn,H,W,O,KH,ph,relu", [
+    (1, 3, 224, 224, 64, 7, 3, True), (5, 3, 224, 224, 64, 7, 3, True),        # one pooled row per CTA; windows that cross images
+    (40, 3, 64, 64, 64, 7, 3, True), (7, 3, 65, 71, 48, 7, 3, True),           # several images per CTA; odd sizes, rows that are no whole words
+    (3, 4, 32, 256, 8, 7, 3, False), (2, 1, 30, 250, 16, 8, 3, False),         # widest rows, one and four planes, no ReLU, eight filter rows
+    (300, 2, 7, 9, 24, 7, 0, True), (4, 3, 1, 8, 64, 3, 1, True), (33, 3, 5, 16, 64, 5, 2, False)])   # images of one or two output rows
+def test_conv_stem_pool(lib, dtype, N, Cn, H, W, O, KH, ph, relu):
+    """Convolution, bias, ReLU and max-pooling from the planar image in one kernel.  Bound: each convolution output is rounded to the
+    activation type once (2^-11 in fp16, 2^-8 in bf16, of its value) after an fp32 sum of at most KH * 28 products (2^-22 of their
+    magnitudes); a maximum errs by no more than the largest error under it."""
+    x, w = gen((N, Cn, H, W), dtype), gen((O, Cn, KH, 7), dtype, 1, 0.2)
+    bias = gen((O,), torch.float32, 2)
+    packed = torch.zeros(O, KH, 7, 8, dtype=dtype)
+    packed[..., :Cn] = w.permute(0, 2, 3, 1)
+    conv = lambda a, b: torch.nn.functional.conv2d(a, b, None, 2, (ph, 3))
+    ref, size = conv(x.double(), w.double()) + bias.double()[None, :, None, None], conv(x.double().abs(), w.double().abs()) + bias.double().abs()[None, :, None, None]
+    ref = torch.relu(ref) if relu else ref
+    pool = lambda t: torch.nn.functional.max_pool2d(t, 3, 2, 1)
+    want, slack = pool(ref).permute(0, 2, 3, 1), pool(ref.abs() * (2.0 ** -11 if dtype == torch.float16 else 2.0 ** -8) + size * 2.0 ** -20 + 1e-7).permute(0, 2, 3, 1)
+    X, Wd, Bd = x.cuda(), packed.cuda(), bias.cuda()
+    y = torch.full(want.shape, float("nan"), dtype=dtype, device="cuda")
+    code = DT[dtype]
+    assert lib.b200_conv_stem_pool_supported(Cn, H, W, 8, O, KH, 7, 2, 2, ph, 3, code)
+    for _ in range(2):
+        ok(lib, lib.b200_conv_stem_pool(X.data_ptr(), Wd.data_ptr(), Bd.data_ptr(), y.data_ptr(), N, Cn, H, W, 8, O, KH, 7, 2, 2, ph, 3, code, int(relu), stream()))
+    err = (y.double().cpu() - want).abs()
+    assert (err <= slack).all(), float((err / slack).max())
+    c = C.c_int(0)
+    ok(lib, lib.b200_debug_device_error(C.byref(c), 1))
+    assert c.value == 0
+
+
+def test_conv_stem_pool_shapes_it_does_not_take(lib):
+    for bad in [(5, 32, 32, 8, 64, 7, 7, 2, 2, 3, 3, 1), (3, 32, 258, 8, 64, 7, 7, 2, 2, 3, 3, 1), (3, 32, 32, 8, 72, 7, 7, 2, 2, 3, 3, 1), (3, 32, 32, 8, 64, 9, 7, 2, 2, 3, 3, 1),
+                (3, 32, 32, 8, 64, 7, 7, 1, 1, 3, 3, 1), (3, 32, 32, 8, 64, 7, 5, 2, 2, 3, 3, 1), (3, 32, 32, 8, 64, 7, 7, 2, 2, 3, 3, 0)]:
+        assert lib.b200_conv_stem_pool_supported(*bad) == 0
