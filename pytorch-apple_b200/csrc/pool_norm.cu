@@ -119,6 +119,51 @@ __global__ void __launch_bounds__(256) adaptive_avg_pool2d_kernel(const __grid_c
                  sum / static_cast<float>((h1 - h0) * (w1 - w0)));
 }
 
+// Channels-last: a block owns 256 channels (8 per thread, 16-byte loads) of one output pixel, its eight warps every eighth
+// input pixel of the window; the warps' fp32 sums meet in shared memory and are added in warp order.  Bound by the memory for many
+// images, by launch and one round trip for few.  us, 7x7 x 2048 channels, a thread per output and two-byte loads one after the
+// other -> this: one image 7.1 -> 2.8, 32 images 7.6 -> 4.2, 256 images 24.8 -> 13.6.
+constexpr int AVG_WARPS = 8;
+template <typename T>
+__global__ void __launch_bounds__(AVG_WARPS * 32) adaptive_avg_pool2d_cl8_kernel(const __grid_constant__ Pool4D p) {
+  __shared__ float part[AVG_WARPS][8][32];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int64_t c = (static_cast<int64_t>(blockIdx.x) * 32 + lane) * 8;
+  const int64_t px = blockIdx.y;   // output pixel: (n, oh, ow)
+  const int ow = static_cast<int>(px % p.OW), oh = static_cast<int>(px / p.OW % p.OH);
+  const int64_t n = px / p.OW / p.OH;
+  const int h0 = static_cast<int>(oh * p.H / p.OH), h1 = static_cast<int>(((oh + 1) * p.H + p.OH - 1) / p.OH);
+  const int w0 = static_cast<int>(ow * p.W / p.OW), w1 = static_cast<int>(((ow + 1) * p.W + p.OW - 1) / p.OW);
+  const int ww = w1 - w0, count = (h1 - h0) * ww;
+  pdl_trigger();
+  pdl_wait();
+  float sum[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+  if (c < p.C) {
+    const T* x = static_cast<const T*>(p.x) + n * p.xs[0] + c;
+#pragma unroll 4
+    for (int i = warp; i < count; i += AVG_WARPS) {
+      const int ih = h0 + i / ww, iw = w0 + i % ww;
+      float v[8];
+      unpack8<T>(ld_global_nc_v4(x + ih * p.xs[2] + iw * p.xs[3]), v);
+#pragma unroll
+      for (int k = 0; k < 8; ++k) sum[k] += v[k];
+    }
+  }
+#pragma unroll
+  for (int k = 0; k < 8; ++k) part[warp][k][lane] = sum[k];
+  __syncthreads();
+  if (warp != 0 || c >= p.C) return;
+  const float n_px = static_cast<float>(count);
+#pragma unroll
+  for (int k = 0; k < 8; ++k) {
+    float t = part[0][k][lane];
+#pragma unroll
+    for (int w = 1; w < AVG_WARPS; ++w) t += part[w][k][lane];
+    sum[k] = t / n_px;
+  }
+  *reinterpret_cast<uint4*>(static_cast<T*>(p.y) + n * p.ys[0] + oh * p.ys[2] + ow * p.ys[3] + c) = pack8<T>(sum);
+}
+
 __global__ void __launch_bounds__(256) batch_norm_kernel(const __grid_constant__ Pool4D p, const void* gamma, const void* beta,
                                                          const void* mean, const void* var, float eps, int param_dtype,
                                                          int relu) {
@@ -180,6 +225,13 @@ static int fill_pool(Pool4D* p, const b200_tensor* x, const b200_tensor* y) {
 
 using namespace b200;
 
+// 16-bit channels-last operands whose pixels are whole 16-byte words of channels
+static bool words_of_channels(const Pool4D& p) {
+  return p.x_dtype == p.y_dtype && (p.x_dtype == B200_F16 || p.x_dtype == B200_BF16) && p.channels_last && p.C % 8 == 0 && p.xs[1] == 1 &&
+         p.ys[1] == 1 && aligned16(p.x) && aligned16(p.y) && p.xs[0] % 8 == 0 && p.xs[2] % 8 == 0 && p.xs[3] % 8 == 0 && p.ys[0] % 8 == 0 &&
+         p.ys[2] % 8 == 0 && p.ys[3] % 8 == 0;
+}
+
 extern "C" int b200_max_pool2d(const b200_tensor* x, const b200_tensor* y, int kh, int kw, int sh, int sw, int ph, int pw,
                                void* stream) {
   Pool4D p;
@@ -187,9 +239,7 @@ extern "C" int b200_max_pool2d(const b200_tensor* x, const b200_tensor* y, int k
   p.kh = kh; p.kw = kw; p.sh = sh; p.sw = sw; p.ph = ph; p.pw = pw;
   const int64_t total = p.N * p.C * p.OH * p.OW;
   if (total == 0) return B200_OK;
-  const bool half_types = p.x_dtype == p.y_dtype && (p.x_dtype == B200_F16 || p.x_dtype == B200_BF16);
-  if (half_types && p.channels_last && p.C % 8 == 0 && p.xs[1] == 1 && p.ys[1] == 1 && aligned16(p.x) && aligned16(p.y) &&
-      p.xs[0] % 8 == 0 && p.xs[2] % 8 == 0 && p.xs[3] % 8 == 0 && p.ys[0] % 8 == 0 && p.ys[2] % 8 == 0 && p.ys[3] % 8 == 0) {
+  if (words_of_channels(p)) {
     const unsigned blocks = static_cast<unsigned>(ceil_div(total / 8, 256));
     if (p.x_dtype == B200_F16) max_pool2d_cl8_kernel<__half><<<blocks, 256, 0, static_cast<cudaStream_t>(stream)>>>(p);
     else max_pool2d_cl8_kernel<__nv_bfloat16><<<blocks, 256, 0, static_cast<cudaStream_t>(stream)>>>(p);
@@ -206,6 +256,14 @@ extern "C" int b200_adaptive_avg_pool2d(const b200_tensor* x, const b200_tensor*
   B200_CHECK_ARG(fill_pool(&p, x, y) == 0 && p.OH > 0 && p.OW > 0, "b200_adaptive_avg_pool2d: bad arguments");
   const int64_t total = p.N * p.C * p.OH * p.OW;
   if (total == 0) return B200_OK;
+  // (the windows are counted in 32 bits; grid.y holds the output pixels)
+  if (words_of_channels(p) && p.N * p.OH * p.OW <= 65535 && p.H < (1 << 15) && p.W < (1 << 15) && p.OH < (1 << 15) && p.OW < (1 << 15)) {
+    const dim3 grid(static_cast<unsigned>(ceil_div(p.C, 256)), static_cast<unsigned>(p.N * p.OH * p.OW));
+    if (p.x_dtype == B200_F16) launch_pdl(adaptive_avg_pool2d_cl8_kernel<__half>, grid, dim3(AVG_WARPS * 32), 0, static_cast<cudaStream_t>(stream), p);
+    else launch_pdl(adaptive_avg_pool2d_cl8_kernel<__nv_bfloat16>, grid, dim3(AVG_WARPS * 32), 0, static_cast<cudaStream_t>(stream), p);
+    B200_CHECK_LAUNCH("adaptive_avg_pool2d_cl8_kernel");
+    return B200_OK;
+  }
   adaptive_avg_pool2d_kernel<<<static_cast<unsigned>(ceil_div(total, 256)), 256, 0, static_cast<cudaStream_t>(stream)>>>(p);
   B200_CHECK_LAUNCH("adaptive_avg_pool2d_kernel");
   return B200_OK;

@@ -1147,3 +1147,19 @@ def test_conv_stem_pool_shapes_it_does_not_take(lib):
     for bad in [(5, 32, 32, 8, 64, 7, 7, 2, 2, 3, 3, 1), (3, 32, 258, 8, 64, 7, 7, 2, 2, 3, 3, 1), (3, 32, 32, 8, 72, 7, 7, 2, 2, 3, 3, 1), (3, 32, 32, 8, 64, 9, 7, 2, 2, 3, 3, 1),
                 (3, 32, 32, 8, 64, 7, 7, 1, 1, 3, 3, 1), (3, 32, 32, 8, 64, 7, 5, 2, 2, 3, 3, 1), (3, 32, 32, 8, 64, 7, 7, 2, 2, 3, 3, 0)]:
         assert lib.b200_conv_stem_pool_supported(*bad) == 0
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("N,Cn,H,W,OH,OW", [(1, 8, 1, 1, 1, 1), (2, 248, 7, 7, 1, 1), (1, 264, 9, 5, 1, 1), (3, 2048, 7, 7, 1, 1), (2, 64, 13, 11, 4, 3), (2, 20, 7, 7, 1, 1)])
+def test_adaptive_avg_pool_channels_last(lib, dtype, N, Cn, H, W, OH, OW):
+    """Channels that end inside a block, windows of unequal size, and channels that are no whole words (the general kernel).  One
+    rounding of an fp32 mean: 2^-11 in fp16 and 2^-8 in bf16 of the result, 2^-20 of the mean magnitude for the sum."""
+    x = gen((N, Cn, H, W), dtype)
+    want = torch.nn.functional.adaptive_avg_pool2d(x.double(), (OH, OW))
+    size = torch.nn.functional.adaptive_avg_pool2d(x.double().abs(), (OH, OW))
+    X = x.cuda().contiguous(memory_format=torch.channels_last)
+    Y = torch.full((N, OH, OW, Cn), float("nan"), dtype=dtype, device="cuda").permute(0, 3, 1, 2)
+    a, b = bt(X), bt(Y)
+    ok(lib, lib.b200_adaptive_avg_pool2d(C.byref(a), C.byref(b), stream()))
+    err = (Y.double().cpu() - want).abs()
+    assert (err <= want.abs() * (2.0 ** -11 if dtype == torch.float16 else 2.0 ** -8) + size * 2.0 ** -20 + 6e-8).all(), float(err.max())
