@@ -2087,7 +2087,10 @@ int conv_tc5(const Tc5Args& a, const Tc5Conv& g, cudaStream_t st) {
     return a.dtype == B200_BF16 ? launch_persistent<__nv_bfloat16, 64, true, true>(a, st, &g8) : launch_persistent<__half, 64, true, true>(a, st, &g8);
   }
   if (g.C % BK || a.K != static_cast<int64_t>(g.KH) * g.KW * g.C || a.ldw % 8 || !aligned16(a.A) || !aligned16(a.W)) return B200_ENOTSUP;
-  if (const int bn = persistent_bn(a.M, a.N, a.K, false, a.residual != nullptr)) return dispatch_persistent<true>(bn, a, st, &g);
+  if (const int bn = persistent_bn(a.M, a.N, a.K, false, a.residual != nullptr)) {
+    if (const int rc = conv_rows(a, g, bn, st); rc != B200_ENOTSUP) return rc;
+    return dispatch_persistent<true>(bn, a, st, &g);
+  }
   {   // fewer tiles than SMs
     const Tc5Plan sp = plan_conv_split(a.M, a.N, a.K);
     const int rc = a.dtype == B200_BF16 ? launch<__nv_bfloat16, 64, true, 1>(a, sp, st, &g) : launch<__half, 64, true, 1>(a, sp, st, &g);
@@ -2126,8 +2129,9 @@ extern "C" int b200_debug_device_error(int* code, int clear) {
   int v = 0;
   cudaError_t e = cudaMemcpyFromSymbol(&v, b200::g_tc5_error, sizeof(int));
   if (e != cudaSuccess) B200_FAIL(B200_ELAUNCH, "b200_debug_device_error: %s", cudaGetErrorString(e));
-  const int att = b200::attn_prefill_tc5_error(clear != 0), stem = b200::conv_stem_error(clear != 0);
-  if (code) *code = v ? v : att > 0 ? att : stem > 0 ? stem : 0;
+  const int att = b200::attn_prefill_tc5_error(clear != 0), stem = b200::conv_stem_error(clear != 0),
+            rows = b200::conv_rows_error(clear != 0);
+  if (code) *code = v ? v : att > 0 ? att : stem > 0 ? stem : rows > 0 ? rows : 0;
   if (clear && v) {
     v = 0;
     cudaMemcpyToSymbol(b200::g_tc5_error, &v, sizeof(int));

@@ -56,6 +56,10 @@ struct Tc5Conv {
 // (stem convolution after channel padding) with O <= 64.
 // Args: A = x [N,H,W,C], W = packed weights [O, KH*KW*C], M = N*Ho*Wo, N = O, K = KH*KW*C.
 int conv_tc5(const Tc5Args& a, const Tc5Conv& g, cudaStream_t stream);
+// 3x3 / stride-1 / padding-1 convolutions whose input rows stay in shared memory (conv_rows.cu), arguments as conv_tc5.
+// B200_ENOTSUP for other geometries and for shapes that the im2col route with tiles of im2col_bn columns serves better.
+int conv_rows(const Tc5Args& a, const Tc5Conv& g, int im2col_bn, cudaStream_t stream);
+int conv_rows_error(bool clear);
 // code left by a bounded wait of the stem + pooling kernel (conv_stem.cu) that ran out (0 = none); optionally cleared
 int conv_stem_error(bool clear);
 

@@ -1163,3 +1163,52 @@ def test_adaptive_avg_pool_channels_last(lib, dtype, N, Cn, H, W, OH, OW):
     ok(lib, lib.b200_adaptive_avg_pool2d(C.byref(a), C.byref(b), stream()))
     err = (Y.double().cpu() - want).abs()
     assert (err <= want.abs() * (2.0 ** -11 if dtype == torch.float16 else 2.0 ** -8) + size * 2.0 ** -20 + 6e-8).all(), float(err.max())
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("N,H,W,Cn,O,res,relu", [
+    (7, 56, 56, 64, 64, False, True), (12, 56, 56, 64, 64, True, True),      # weights resident, two issuing threads; with residual
+    (20, 31, 30, 64, 64, False, False), (9, 57, 55, 64, 40, True, False),    # last tiles of an image shorter, fewer channels than a tile
+    (3, 90, 126, 64, 64, False, True), (25, 28, 28, 128, 128, True, True),   # one row per tile; weights streamed, one tile per unit
+    (127, 28, 28, 128, 128, False, True), (20, 28, 28, 64, 200, True, True),  # two tiles per unit, an odd number of tiles; two column tiles
+    (35, 14, 14, 256, 256, True, True), (40, 14, 14, 192, 136, False, True), (300, 7, 15, 64, 128, False, True),   # tiles of eight rows; a whole image per tile
+    (48, 14, 14, 256, 256, True, True)])                                     # (the im2col route)
+def test_conv3x3_rows(lib, dtype, N, H, W, Cn, O, res, relu):
+    """3x3 / 1 / 1 convolutions over enough pixels for the kernel that keeps input rows in shared memory.  Bound: fp32 sums of 9 C
+    products (2^-20 of their magnitudes), rounded to the activation type, the sum with the residual rounded once more."""
+    x, w = gen((N, H, W, Cn), dtype).cuda(), gen((O, 3, 3, Cn), dtype, 1, 0.05).cuda()
+    bias = gen((O,), torch.float32, 2).cuda()
+    r = gen((N, H, W, O), dtype, 3).cuda() if res else None
+    conv = lambda a, b: torch.nn.functional.conv2d(a.permute(0, 3, 1, 2), b.permute(0, 3, 1, 2), None, 1, 1).permute(0, 2, 3, 1)
+    eps = 2.0 ** -11 if dtype == torch.float16 else 2.0 ** -8
+    want = conv(x.double(), w.double()) + bias.double()
+    slack = want.abs() * eps + (conv(x.double().abs(), w.double().abs()) + bias.double().abs()) * 2.0 ** -20 + 1e-7
+    if res:
+        want = want + r.double()
+        slack = slack + want.abs() * eps
+    want = torch.relu(want) if relu else want
+    y = torch.full((N, H, W, O), float("nan"), dtype=dtype, device="cuda")
+    for _ in range(2):
+        ok(lib, lib.b200_conv2d_nhwc(x.data_ptr(), w.data_ptr(), bias.data_ptr(), r.data_ptr() if res else None, y.data_ptr(), N, H, W, Cn, Cn, O, 3, 3, 1, 1, 1, 1,
+                                     H, W, DT[dtype], int(relu), stream()))
+        err = (y.double() - want).abs()
+        assert (err <= slack * 1.01).all(), float((err / slack).max())
+    code = C.c_int(0)
+    ok(lib, lib.b200_debug_device_error(C.byref(code), 1))
+    assert code.value == 0
+
+
+@pytest.mark.parametrize("N,H,Cn,O,kernel", [(20, 56, 64, 64, "conv_rows_kernel"), (127, 28, 128, 128, "conv_rows_kernel"), (20, 28, 128, 128, "conv_rows_kernel"),
+                                             (48, 14, 256, 256, "gemm_tc5p_kernel"), (256, 14, 256, 256, "gemm_tc5p_kernel"), (20, 56, 128, 64, "gemm_tc5p_kernel"),
+                                             (2, 56, 64, 64, "gemm_tc5_kernel")])
+def test_conv3x3_runs_on_the_kernel_that_its_shape_calls_for(lib, N, H, Cn, O, kernel):
+    x, w = torch.zeros(N, H, H, Cn, dtype=torch.float16, device="cuda"), torch.zeros(O, 3, 3, Cn, dtype=torch.float16, device="cuda")
+    y = torch.empty(N, H, H, O, dtype=torch.float16, device="cuda")
+    call = lambda: ok(lib, lib.b200_conv2d_nhwc(x.data_ptr(), w.data_ptr(), None, None, y.data_ptr(), N, H, H, Cn, Cn, O, 3, 3, 1, 1, 1, 1, H, H, 1, 0, stream()))
+    names = []
+    for _ in range(3):   # (a profiling session now and then reports nothing)
+        with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CUDA]) as prof:
+            call()
+            torch.cuda.synchronize()
+        names = names or [e.key for e in prof.key_averages() if "_kernel" in e.key]
+    assert len(names) == 1 and kernel in names[0], names
