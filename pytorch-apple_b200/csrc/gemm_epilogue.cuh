@@ -30,6 +30,10 @@ struct Tc5Params {
   Tc5Args::Rope rope;
 };
 
+// The CTA-pair kernel (gemm_pair.cu): tiles of 256 weight rows x up to 256 tokens; p.splits > 1: partial sums to p.partial.
+int gemm_pair(const Tc5Args& a, const Tc5Params& p, cudaStream_t st);
+int gemm_pair_error(bool clear);
+
 template <typename T> struct AbFormat;
 template <> struct AbFormat<__half> { static constexpr int value = 0; };
 template <> struct AbFormat<__nv_bfloat16> { static constexpr int value = 1; };

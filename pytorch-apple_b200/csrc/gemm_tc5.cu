@@ -956,221 +956,6 @@ __global__ void __launch_bounds__(CONV && !TS && KPS == 1 ? PCfg<BN, TS>::THREAD
   if (warp == 1) { tc5::tc_fence_after(); tc5::tmem_dealloc(tmem_base, 2 * BN); }
 }
 
-// ---- CTA-pair kernel: 256 x 256 tiles on two SMs (cta_group::2) ------------------------------------
-// A 128 x 256 tile per CTA needs 48 KB of operands per 4.2 MFLOP; at the rate the L2 feeds the SMs
-// (measured ~11 TB/s over all SMs) that bounds the persistent kernel at ~1 PFLOP/s.  Here the two CTAs
-// of a cluster share one 256 x 256 tile: each loads its own 128 rows of A and its own 128 of the 256 B
-// rows (32 KB per k-block and CTA for the same 4.2 MFLOP), rank 0 issues M = 256 MMAs that read both
-// CTAs' shared memory and write both CTAs' tensor memory.  Linear layers only; the epilogue is the plain
-// one (accumulator rows -> registers -> global), overlapped with the next tile through the two accumulators.
-// warps: 0 / 7 activation producers, 6 / 8 weight producers, 1 MMA (rank 0) and TMEM, 2-5 epilogue of columns
-// 0..127, 9-12 epilogue of columns 128..255 (a tile that nothing follows - the last of a CTA, every split-K unit -
-// is drained in half the time).
-constexpr int PAIR_BN = 256, PAIR_ST = 6, PAIR_THREADS = 416;
-constexpr int PAIR_A_STAGE = BM * BK * 2, PAIR_B_STAGE = (PAIR_BN / 2) * BK * 2, PAIR_STAGE = PAIR_A_STAGE + PAIR_B_STAGE;
-constexpr int PAIR_SMEM = PAIR_ST * PAIR_STAGE + 1024;
-
-template <typename T>
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PAIR_THREADS, 1)
-    gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_w, const Tc5Params p, const int tiles_m,
-                     const int n_tiles) {
-  constexpr int ST = PAIR_ST, BN = PAIR_BN;
-  extern __shared__ uint8_t smem_raw[];
-  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
-  // full_bar / acc_empty are used in rank 0 only (its MMA thread waits on them); empty_bar / acc_full in both
-  __shared__ __align__(8) uint64_t full_bar[ST], empty_bar[ST], acc_full[2], acc_empty[2];
-  __shared__ uint32_t tmem_holder;
-  __shared__ int failed;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const uint32_t rank = tc5::cluster_ctarank();
-  const int pair = blockIdx.x >> 1, n_pairs = gridDim.x >> 1;
-  const int KB = static_cast<int>((p.K + BK - 1) / BK);
-  // Work units: (tile, split).  With split-K (few tiles, long reduction) a unit covers p.kb_per_split
-  // k-blocks of its tile and leaves fp32 partial sums in p.partial; a second kernel adds them up.
-  const int n_units = n_tiles * p.splits;
-  auto unit_kb0 = [&](int unit) { return (unit / n_tiles) * p.kb_per_split; };
-  auto unit_nkb = [&](int unit) { const int k0 = unit_kb0(unit); return (KB - k0 < p.kb_per_split ? KB - k0 : p.kb_per_split); };
-  if (threadIdx.x == 0) {
-    failed = 0;
-    for (int s = 0; s < ST; ++s) { tc5::mbar_init(&full_bar[s], 2); tc5::mbar_init(&empty_bar[s], 1); }   // full: rank 0's two producers of the k-block
-    for (int b = 0; b < 2; ++b) { tc5::mbar_init(&acc_full[b], 1); tc5::mbar_init(&acc_empty[b], 16); }    // empty: eight epilogue warps of each CTA
-    tc5::fence_barrier_init();
-    tc5::prefetch_tensormap(&map_a);
-    tc5::prefetch_tensormap(&map_w);
-  }
-  if (warp == 1) { tc5::tmem_alloc_pair(&tmem_holder, 2 * BN); tc5::tmem_relinquish_pair(); }
-  tc5::tc_fence_before();
-  __syncthreads();
-  tc5::cluster_sync();   // the peer's barriers exist before anything arrives on them
-  tc5::tc_fence_after();
-  const uint32_t tmem_base = tmem_holder;
-  pdl_trigger();
-  auto dead = [&]() { return *reinterpret_cast<volatile int*>(&failed) != 0; };
-  const uint32_t ring_addr = tc5::smem_addr(smem), full0 = tc5::smem_addr(&full_bar[0]), empty0 = tc5::smem_addr(&empty_bar[0]);
-
-  const int a_id = warp == 0 ? 0 : warp == 7 ? 1 : -1, b_id = warp == 6 ? 0 : warp == 8 ? 1 : -1;
-  if (a_id >= 0 || b_id >= 0) {
-    // ---- producers: k-blocks alternate between the two threads of an operand (2 <= ring depth) ----
-    if (lane == 0) {
-      const bool is_a = a_id >= 0;
-      const int mine = is_a ? a_id : b_id;
-      if (is_a || !(p.epilogue & B200_EPI_W_STATIC)) pdl_wait();
-      const CUtensorMap* map = is_a ? &map_a : &map_w;
-      const uint32_t lead_full0 = tc5::map_to_rank(full0, 0);
-      int it = 0, s = 0;
-      uint32_t ph = 0, dst = ring_addr + (is_a ? 0 : PAIR_A_STAGE);
-      const uint32_t dst0 = dst;
-      bool alive = true;
-      for (int unit = pair; unit < n_units && alive && !dead(); unit += n_pairs) {
-        const int tile = unit % n_tiles;
-        const int row0 = (is_a ? (tile % tiles_m) : (tile / tiles_m)) * 256 + static_cast<int>(rank) * 128;   // this CTA's half
-        const int kb0 = unit_kb0(unit), kb1 = kb0 + unit_nkb(unit);
-        for (int kb = kb0; kb < kb1; ++kb, ++it) {
-          if ((it & 1) == mine) {
-            if (!tc5::mbar_wait_a(empty0 + 8u * s, ph ^ 1u)) { failed = 1; atomicExch(&g_tc5_error, 40); alive = false; break; }
-            if (rank == 0) tc5::mbar_arrive_expect_tx_a(full0 + 8u * s, 2 * PAIR_A_STAGE);   // both CTAs' halves of this operand
-            tc5::tma_load_2d_pair(dst, map, lead_full0 + 8u * s, kb * BK, row0);
-          }
-          dst += PAIR_STAGE;
-          if (++s == ST) { s = 0; ph ^= 1u; dst = dst0; }
-        }
-      }
-    }
-  } else if (warp == 1) {
-    if (lane == 0 && rank == 0) {
-      // ---- MMA issuer (rank 0 only) ----
-      constexpr uint32_t idesc = tc5::umma_idesc(256, BN, AbFormat<T>::value);
-      const uint32_t ring_lo = tc5::desc_sw128_lo(ring_addr);
-      const uint32_t acc_full0 = tc5::smem_addr(&acc_full[0]), acc_empty0 = tc5::smem_addr(&acc_empty[0]);
-      int ti = 0, s = 0;
-      uint32_t ph = 0, a_lo = ring_lo;
-      bool alive = true;
-      for (int unit = pair; unit < n_units && alive && !dead(); unit += n_pairs, ++ti) {
-        const int b = ti & 1;
-        if (!tc5::mbar_wait_a(acc_empty0 + 8u * b, ((ti >> 1) & 1) ^ 1)) { failed = 1; atomicExch(&g_tc5_error, 41); break; }
-        tc5::tc_fence_after();
-        const uint32_t acc = tmem_base + b * BN;
-        const int nkb = unit_nkb(unit);
-        for (int kb = 0; kb < nkb; ++kb) {
-          if (!tc5::mbar_wait_a(full0 + 8u * s, ph)) { failed = 1; atomicExch(&g_tc5_error, 42); alive = false; break; }
-          tc5::umma_f16_kblock_pair(acc, a_lo, a_lo + (PAIR_A_STAGE >> 4), idesc, kb);
-          tc5::umma_commit_pair(empty0 + 8u * s);   // frees the stage in both CTAs
-          a_lo += PAIR_STAGE >> 4;
-          if (++s == ST) { s = 0; ph ^= 1u; a_lo = ring_lo; }
-        }
-        if (!alive) break;
-        tc5::umma_commit_pair(acc_full0 + 8u * b);
-      }
-    }
-  } else {
-    // ---- epilogue (warps 2-5 and 9-12): this CTA's 128 accumulator rows, columns c_lo .. c_lo + 127 ----
-    const int q = warp & 3;
-    const int c_lo = warp >= 9 ? BN / 2 : 0, c_hi = c_lo + BN / 2;
-    pdl_wait();
-    const bool glu = (p.epilogue & B200_EPI_GLU) != 0;
-    const bool res_fast = p.splits == 1 && !glu && p.residual && !(p.epilogue & B200_EPI_SILU_MUL) && p.ldr % 8 == 0 && p.N % 8 == 0 &&
-                          (reinterpret_cast<uintptr_t>(p.residual) & 15u) == 0;
-    const uint32_t lead_acc_empty0 = tc5::map_to_rank(tc5::smem_addr(&acc_empty[0]), 0);
-    int ti = 0;
-    for (int unit = pair; unit < n_units; unit += n_pairs, ++ti) {
-      const int b = ti & 1;
-      const int tile = unit % n_tiles;
-      const int64_t m = static_cast<int64_t>(tile % tiles_m) * 256 + rank * 128 + q * 32 + lane;
-      const int64_t n0 = static_cast<int64_t>(tile / tiles_m) * BN;
-      // Residual rows are read 32 columns (four 16-byte words) at a time, one step ahead of their use and the
-      // first step before the accumulator is waited for: a load per step issued and consumed in place would
-      // put an L2 round trip between any two steps of this thread's row.
-      uint4 rc[4], rn[4];
-      const T* rrow = res_fast && m < p.M ? static_cast<const T*>(p.residual) + m * p.ldr + n0 : nullptr;
-      auto fetch = [&](int c, uint4 (&r)[4]) {
-#pragma unroll
-        for (int j = 0; j < 4; ++j)
-          r[j] = (rrow && n0 + c + 8 * j < p.N) ? __ldg(reinterpret_cast<const uint4*>(rrow + c) + j) : make_uint4(0u, 0u, 0u, 0u);
-      };
-      if (res_fast) fetch(c_lo, rc);
-      bool ok = true;
-      if (lane == 0) ok = tc5::mbar_wait(&acc_full[b], (ti >> 1) & 1);
-      ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
-      if (!ok && lane == 0) { failed = 1; atomicExch(&g_tc5_error, 43); }
-      ok = __all_sync(0xffffffffu, ok && !dead());
-      if (!ok) break;
-      tc5::tc_fence_after();
-      const uint32_t t_row = tmem_base + b * BN + (static_cast<uint32_t>(q * 32) << 16);
-      if (res_fast) {
-        float va[16], vb[16];
-#pragma unroll 1
-        for (int c = c_lo; c < c_hi; c += 32) {
-          __syncwarp();
-          tc5::tmem_ld_32x16(t_row + c, va);
-          tc5::tmem_ld_32x16(t_row + c + 16, vb);
-          if (c + 32 < c_hi) fetch(c + 32, rn);
-          tc5::tmem_ld_wait();
-          if (m < p.M && n0 + c < p.N) finish_cols_res<T>(p, va, m, n0 + c, rc[0], rc[1]);
-          if (m < p.M && n0 + c + 16 < p.N) finish_cols_res<T>(p, vb, m, n0 + c + 16, rc[2], rc[3]);
-#pragma unroll
-          for (int j = 0; j < 4; ++j) rc[j] = rn[j];
-        }
-      } else if (p.splits > 1) {
-        // raw partial sums of this unit's k-range (N % 8 == 0: 32-byte units stay inside the row); two 16-column
-        // units in flight, 256-bit stores (a lane's store is one whole sector)
-        float* dst = p.partial + (static_cast<int64_t>(unit / n_tiles) * p.M + m) * p.N + n0;
-        float va[16], vb[16];
-        __syncwarp();
-        tc5::tmem_ld_32x16(t_row + c_lo, va);
-#pragma unroll 1
-        for (int c = c_lo; c < c_hi; c += 32) {
-          tc5::tmem_ld_wait();
-          tc5::tmem_ld_32x16(t_row + c + 16, vb);
-          if (m < p.M) {
-            if (n0 + c < p.N) tc5::st_global_f8(dst + c, va);
-            if (n0 + c + 8 < p.N) tc5::st_global_f8(dst + c + 8, va + 8);
-          }
-          __syncwarp();
-          tc5::tmem_ld_wait();
-          if (c + 32 < c_hi) tc5::tmem_ld_32x16(t_row + c + 32, va);
-          if (m < p.M) {
-            if (n0 + c + 16 < p.N) tc5::st_global_f8(dst + c + 16, vb);
-            if (n0 + c + 24 < p.N) tc5::st_global_f8(dst + c + 24, vb + 8);
-          }
-          __syncwarp();
-        }
-      } else if (glu) {
-#pragma unroll 1
-        for (int c = c_lo / 2; c < c_hi / 2; c += 16) {   // c counts gate columns: block c / 64 of 128 merged columns
-          float vg[16], vu[16];
-          const int col = (c >> 6) * 128 + (c & 63);
-          __syncwarp();
-          tc5::tmem_ld_32x16(t_row + col, vg);
-          tc5::tmem_ld_32x16(t_row + col + 64, vu);
-          tc5::tmem_ld_wait();
-          const int64_t nm = n0 + col;
-          if (m < p.M && nm < p.N) finish_glu_cols<T, 16>(p, vg, vu, m, nm, (n0 + (c >> 6) * 128) / 2 + (c & 63));
-        }
-      } else {
-        float va[16], vb[16];   // two units in flight: the next tcgen05.ld runs under the current unit's math
-        __syncwarp();
-        tc5::tmem_ld_32x16(t_row + c_lo, va);
-#pragma unroll 1
-        for (int c = c_lo; c < c_hi; c += 32) {
-          tc5::tmem_ld_wait();
-          tc5::tmem_ld_32x16(t_row + c + 16, vb);
-          if (m < p.M && n0 + c < p.N) finish_cols<T, 16>(p, va, m, n0 + c);
-          tc5::tmem_ld_wait();
-          if (c + 32 < c_hi) tc5::tmem_ld_32x16(t_row + c + 32, va);
-          if (m < p.M && n0 + c + 16 < p.N) finish_cols<T, 16>(p, vb, m, n0 + c + 16);
-        }
-      }
-      tc5::tc_fence_before();
-      __syncwarp();
-      if (lane == 0) tc5::mbar_arrive_cluster(lead_acc_empty0 + 8u * b);   // this warp has drained its quarter of the accumulator
-    }
-  }
-  tc5::tc_fence_before();
-  __syncthreads();
-  tc5::cluster_sync();   // neither CTA leaves while the other may still signal its barriers or read its shared memory
-  if (warp == 1) { tc5::tc_fence_after(); tc5::tmem_dealloc_pair(tmem_base, 2 * BN); }
-}
-
 // Second half of the pair kernel's split-K: out = epilogue(sum over splits of the fp32 partial sums), eight
 // consecutive columns per thread.  The partial sums of all splits (at most PAIR_MAX_SPLITS) are requested before
 // the first is used - one memory round trip per output instead of one per split, which is what this kernel's
@@ -1825,12 +1610,13 @@ int launch_persistent(const Tc5Args& a, cudaStream_t st, const Tc5Conv* g = null
   return B200_OK;
 }
 
-// The CTA-pair kernel takes a linear layer when its 256 x 256 tiles give at least half of the 74 pairs a tile
-// (even half empty it beats 128-wide tiles on every SM) and the reduction is long enough to hide the plain epilogue.
+// The CTA-pair kernel takes a linear layer when its tiles (256 columns x up to 256 rows) give at least half of the 74 pairs a tile
+// (even half empty it beats 128-wide tiles on every SM; with one tile of rows from 65 on: gate/up of 128 rows 16.1 -> 13.9 us,
+// of 65 rows 15.0 -> 14.7, vocabulary 92 -> 86) and the reduction is long enough to hide the plain epilogue.
 bool pair_shape(const Tc5Args& a) {
   // (N >= 1024: a tall activation matrix against one or two column tiles - the 1x1 convolutions 1024 -> 256 / 512
   // over 50176 pixels - measured slower here than with the bulk-copy epilogue of the persistent kernel)
-  if (a.M <= 128 || a.N < 1024 || a.K < 1024) return false;
+  if (a.M <= 64 || a.N < 1024 || a.K < 1024) return false;
   return ceil_div(a.M, 256) * ceil_div(a.N, 256) >= 37;
 }
 
@@ -1853,18 +1639,6 @@ int pair_splits(int64_t M, int64_t N, int64_t K) {
 int64_t pair_splitk_bytes(int64_t M, int64_t N, int splits) { return splits > 1 ? splits * M * N * 4 : 0; }
 
 template <typename T> int launch_pair(const Tc5Args& a, cudaStream_t st, int splits = 1) {
-  static PerDevice<bool> configured_on;
-  bool* configured = configured_on.slot();
-  if (!configured) return B200_ENOTSUP;
-  if (!*configured) {
-    if (cudaFuncSetAttribute(gemm_pair_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, PAIR_SMEM) != cudaSuccess) {
-      cudaGetLastError();
-      return B200_ENOTSUP;
-    }
-    *configured = true;
-  }
-  CUtensorMap ma, mw;
-  if (!make_map(&ma, a.A, a.M, a.K, a.lda, BM, a.dtype) || !make_map(&mw, a.W, a.N, a.K, a.ldw, PAIR_BN / 2, a.dtype)) return B200_ENOTSUP;
   Tc5Params p = {};
   p.bias = a.bias; p.residual = a.residual; p.aux = a.aux; p.out = a.out;
   p.M = a.M; p.N = a.N; p.K = a.K; p.ldo = a.ldo; p.ldr = a.ldr; p.ldaux = a.ldaux;
@@ -1872,13 +1646,10 @@ template <typename T> int launch_pair(const Tc5Args& a, cudaStream_t st, int spl
   p.splits = splits; p.kb_per_split = static_cast<int>(ceil_div(ceil_div(a.K, BK), splits));
   p.partial = static_cast<float*>(a.workspace);
   p.x = a.A;
-  const int64_t tiles_m = ceil_div(a.M, 256), tiles = tiles_m * ceil_div(a.N, PAIR_BN), units = tiles * splits;
-  if (units >= (1ll << 30) || splits > PAIR_MAX_SPLITS) return B200_ENOTSUP;
+  if (splits > PAIR_MAX_SPLITS) return B200_ENOTSUP;
   if (splits > 1 && (!a.workspace || a.workspace_bytes < pair_splitk_bytes(a.M, a.N, splits) || (reinterpret_cast<uintptr_t>(a.workspace) & 31u)))   // 256-bit accesses
     return B200_ENOTSUP;
-  const int pairs = static_cast<int>(units < sm_count() / 2 ? units : sm_count() / 2);
-  launch_pdl(gemm_pair_kernel<T>, dim3(2 * pairs), dim3(PAIR_THREADS), PAIR_SMEM, st, ma, mw, p, static_cast<int>(tiles_m), static_cast<int>(tiles));
-  B200_CHECK_LAUNCH("gemm_pair_kernel");
+  if (const int rc = gemm_pair(a, p, st); rc != B200_OK) return rc;
   if (splits > 1) {
     const Tc5Args::NormTail& t = a.norm_tail;
     const bool tail = t.out && t.gain && t.done && a.N <= 2048 && a.M < (1ll << 31) && t.ld % 8 == 0 && aligned16(t.out) && aligned16(t.gain) &&
@@ -2130,8 +1901,8 @@ extern "C" int b200_debug_device_error(int* code, int clear) {
   cudaError_t e = cudaMemcpyFromSymbol(&v, b200::g_tc5_error, sizeof(int));
   if (e != cudaSuccess) B200_FAIL(B200_ELAUNCH, "b200_debug_device_error: %s", cudaGetErrorString(e));
   const int att = b200::attn_prefill_tc5_error(clear != 0), stem = b200::conv_stem_error(clear != 0),
-            rows = b200::conv_rows_error(clear != 0);
-  if (code) *code = v ? v : att > 0 ? att : stem > 0 ? stem : rows > 0 ? rows : 0;
+            rows = b200::conv_rows_error(clear != 0), pair = b200::gemm_pair_error(clear != 0);
+  if (code) *code = v ? v : att > 0 ? att : stem > 0 ? stem : rows > 0 ? rows : pair > 0 ? pair : 0;
   if (clear && v) {
     v = 0;
     cudaMemcpyToSymbol(b200::g_tc5_error, &v, sizeof(int));

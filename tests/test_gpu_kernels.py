@@ -1198,17 +1198,50 @@ def test_conv3x3_rows(lib, dtype, N, H, W, Cn, O, res, relu):
     assert code.value == 0
 
 
-@pytest.mark.parametrize("N,H,Cn,O,kernel", [(20, 56, 64, 64, "conv_rows_kernel"), (127, 28, 128, 128, "conv_rows_kernel"), (20, 28, 128, 128, "conv_rows_kernel"),
-                                             (48, 14, 256, 256, "gemm_tc5p_kernel"), (256, 14, 256, 256, "gemm_tc5p_kernel"), (20, 56, 128, 64, "gemm_tc5p_kernel"),
-                                             (2, 56, 64, 64, "gemm_tc5_kernel")])
-def test_conv3x3_runs_on_the_kernel_that_its_shape_calls_for(lib, N, H, Cn, O, kernel):
-    x, w = torch.zeros(N, H, H, Cn, dtype=torch.float16, device="cuda"), torch.zeros(O, 3, 3, Cn, dtype=torch.float16, device="cuda")
-    y = torch.empty(N, H, H, O, dtype=torch.float16, device="cuda")
-    call = lambda: ok(lib, lib.b200_conv2d_nhwc(x.data_ptr(), w.data_ptr(), None, None, y.data_ptr(), N, H, H, Cn, Cn, O, 3, 3, 1, 1, 1, 1, H, H, 1, 0, stream()))
-    names = []
-    for _ in range(3):   # (a profiling session now and then reports nothing)
-        with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CUDA]) as prof:
-            call()
-            torch.cuda.synchronize()
-        names = names or [e.key for e in prof.key_averages() if "_kernel" in e.key]
-    assert len(names) == 1 and kernel in names[0], names
+@pytest.mark.parametrize("M", [65, 80, 128, 129, 250, 257, 273, 500, 777])
+@pytest.mark.parametrize("form", ["plain", "residual", "residual unaligned", "gated", "silu mul", "split"])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+def test_linear_pair_token_tiles(lib, M, form, dtype):
+    """Token tiles of every width (multiples of 16, a last one that is short), each epilogue, partial sums; columns that end inside a
+    block.  Bound: fp32 sums of K products (2^-20 of their magnitudes), each rounding to the activation type 2^-8 (bf16) or 2^-11."""
+    N, K = (9600, 1032) if form != "split" else (1536, 4104)
+    if form in ("residual unaligned", "silu mul"):
+        N = 9500
+    if form == "split" and M <= 256:
+        pytest.skip("too few tiles to split")
+    a, w, bias = gen((M, K), dtype).cuda(), gen((N, K), dtype, 1, 0.05).cuda(), gen((N,), torch.float32, 2).cuda()
+    eps = 2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -11
+    s, size = a.double() @ w.double().T + bias.double(), a.double().abs() @ w.double().abs().T + bias.double().abs()
+    slack = s.abs() * eps + size * 2.0 ** -20 + 1e-6
+    epi, res, aux, out_cols = 0, None, None, N
+    if form == "gated":
+        epi, out_cols = 4, N // 2
+        blocks, sb = s.view(M, N // 128, 2, 64), slack.view(M, N // 128, 2, 64)
+        gate, up = blocks[:, :, 0], blocks[:, :, 1]
+        act = gate * torch.sigmoid(gate)
+        want = (act * up).reshape(M, -1)
+        slack = ((sb[:, :, 0] * 1.1 + act.abs() * (eps + 1e-5)) * up.abs() + act.abs() * sb[:, :, 1] + 2 * sb[:, :, 0] * sb[:, :, 1]).reshape(M, -1) + want.abs() * eps + 1e-6
+    elif form == "silu mul":
+        epi, aux = 2, gen((M, N), dtype, 3).cuda()
+        act = s * torch.sigmoid(s)
+        want = act * aux.double()
+        slack = (slack * 1.1 + act.abs() * (eps + 1e-5)) * aux.double().abs() + want.abs() * eps + 1e-6
+    elif form == "plain":
+        want = s
+    else:
+        res = gen((M, N), dtype, 3).cuda()
+        want = s + res.double()
+        slack = slack + want.abs() * eps
+    out = torch.full((M, out_cols), float("nan"), dtype=dtype, device="cuda")
+    need = lib.b200_linear_workspace_bytes(M, N, K)
+    assert (need > 0) == (form == "split")
+    ws = torch.zeros(max(need, 16), dtype=torch.uint8, device="cuda")
+    for _ in range(2):
+        ok(lib, lib.b200_linear(a.data_ptr(), w.data_ptr(), bias.data_ptr(), res.data_ptr() if res is not None else None, out.data_ptr(), M, N, K, K, K, out_cols,
+                                N if res is not None else 0, DT[dtype], 0, epi, aux.data_ptr() if aux is not None else None, N if aux is not None else 0,
+                                ws.data_ptr(), need, stream()))
+        err = (out.double() - want).abs()
+        assert (err <= slack * 1.01).all(), float((err / slack).max())
+    code = C.c_int(0)
+    ok(lib, lib.b200_debug_device_error(C.byref(code), 1))
+    assert code.value == 0
