@@ -8,7 +8,7 @@
 // - a producer thread brings new input rows in pairs, planar as they are, by TMA (rows and pixels outside the image
 //   arrive as zeros) into a ring; images whose rows are no whole 16-byte words are copied there by the loaders themselves;
 // - loaders (128 threads, one per column) write them to a window of 16 row slots as sliding windows: per plane, 16 bytes for
-//   output column p hold its pixels 2p - 4 .. 2p + 3 - the eight taps of a filter row, the first of which has no weight.  That
+//   output column p hold its pixels 2p - 4 .. 2p + 3 - the eight taps of a filter row, the first of which is no tap and zero.  That
 //   is the unswizzled K-major core-matrix layout (8 columns x 16 bytes, every core matrix a 128-byte line), and the MMA reads its A
 //   operand in place: two instructions (K = 16: the taps of two planes) per filter row.  (Windows that overlap in memory instead of
 //   being written out need no copies, but core matrices that straddle two lines: 143 cycles per MMA instead of 85.);
@@ -273,7 +273,8 @@ __global__ void __launch_bounds__(SP_THREADS, 1) conv_stem_pool_kernel(const __g
           for (int ch = 0; ch < 4; ++ch)
             if (ch < p.C) {
               const uint32_t* px = reinterpret_cast<const uint32_t*>(src + (ch * 2 + j) * pitch + 4 * t + 8);   // pixel 2t - 4
-              *reinterpret_cast<uint4*>(slot + ch * SP_PLANE) = make_uint4(px[0], px[1], px[2], px[3]);
+              // (pixel 2t - 4 belongs to no tap: an infinity there times the zero weight would be a NaN)
+              *reinterpret_cast<uint4*>(slot + ch * SP_PLANE) = make_uint4(px[0] & 0xffff0000u, px[1], px[2], px[3]);
             }
         }
         if (p.tma) arrive(&raw_empty[s]);

@@ -1143,6 +1143,31 @@ def test_conv_stem_pool(lib, dtype, N, Cn, H, W, O, KH, ph, relu):
     assert c.value == 0
 
 
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("W", [64, 71])
+@pytest.mark.parametrize("relu", [True, False])
+def test_conv_stem_pool_infinite_pixel(lib, dtype, W, relu):
+    """One infinite pixel reaches the outputs whose filter covers it and no other.  Bound of the finite ones as above."""
+    x, w = gen((2, 3, 33, W), dtype), gen((64, 3, 7, 7), dtype, 1, 0.2)
+    packed = torch.zeros(64, 7, 7, 8, dtype=dtype)
+    packed[..., :3] = w.permute(0, 2, 3, 1)
+    conv = lambda a, b: torch.nn.functional.conv2d(a, b, None, 2, 3)
+    pool = lambda t: torch.nn.functional.max_pool2d(t, 3, 2, 1).permute(0, 2, 3, 1)
+    size = conv(x.double().abs(), w.double().abs())
+    for at in (0, 12, 13, W - 1):
+        bad = x.clone()
+        bad[1, 2, 16, at] = float("inf")
+        ref = conv(bad.double(), w.double())
+        ref = torch.relu(ref) if relu else ref
+        want, X, Wd = pool(ref), bad.cuda(), packed.cuda()
+        slack = pool(size) * ((2.0 ** -11 if dtype == torch.float16 else 2.0 ** -8) + 2.0 ** -20) + 1e-7
+        y = torch.empty(want.shape, dtype=dtype, device="cuda")
+        ok(lib, lib.b200_conv_stem_pool(X.data_ptr(), Wd.data_ptr(), None, y.data_ptr(), 2, 3, 33, W, 8, 64, 7, 7, 2, 2, 3, 3, DT[dtype], int(relu), stream()))
+        got, finite = y.double().cpu(), want.isfinite()
+        assert torch.equal(got[~finite], want[~finite])
+        assert got[finite].isfinite().all() and ((got - want).abs()[finite] <= slack[finite]).all()
+
+
 def test_conv_stem_pool_shapes_it_does_not_take(lib):
     for bad in [(5, 32, 32, 8, 64, 7, 7, 2, 2, 3, 3, 1), (3, 32, 258, 8, 64, 7, 7, 2, 2, 3, 3, 1), (3, 32, 32, 8, 72, 7, 7, 2, 2, 3, 3, 1), (3, 32, 32, 8, 64, 9, 7, 2, 2, 3, 3, 1),
                 (3, 32, 32, 8, 64, 7, 7, 1, 1, 3, 3, 1), (3, 32, 32, 8, 64, 7, 5, 2, 2, 3, 3, 1), (3, 32, 32, 8, 64, 7, 7, 2, 2, 3, 3, 0)]:
