@@ -41,6 +41,7 @@ except ImportError:  # pragma: no cover
 
 
 _HANDLE = operator.attrgetter("native_handle")
+_CONTIGUOUS = operator.methodcaller("is_contiguous")
 
 
 def _mask_key(m: TensorView) -> tuple:
@@ -183,6 +184,8 @@ class CUDAExecutor:
         self._check_weights(weights)
         tensors = self._input_tensors(inputs)
         key = tuple((n, t.data_ptr(), t.dtype) for n, t in tensors.items())
+        if not all(map(_CONTIGUOUS, tensors.values())):   # not the plan of a contiguous tensor that had this address: binding refuses it
+            key += tuple(n for n, t in tensors.items() if not t.is_contiguous())
         plan = self._plans.get(key)
         if plan is None:
             if len(self._plans) >= 8:
@@ -472,9 +475,9 @@ class CUDAExecutor:
             have = str(t.dtype).replace("torch.", "")
             if have == "bool":
                 have = "uint8"
+            if not t.is_contiguous():   # views are strides of the declared shape, and a conversion takes the elements as they lie
+                raise RuntimeError(f"graph input '{name}' must be contiguous")
             if have == view.dtype or any_dtype:
-                if not t.is_contiguous():
-                    raise RuntimeError(f"graph input '{name}' must be contiguous")
                 return t.data_ptr(), have
             staged = self._staged.get(name)
             if staged is None:  # per-run conversion into the dtype the kernels expect

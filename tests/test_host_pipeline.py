@@ -146,6 +146,48 @@ def test_resnet18_golden(fake_native):
     assert fake_native.calls.count("conv2d") == 20 and "batch_norm" not in fake_native.calls
 
 
+def _network_head(stages, size=32, compute_dtype="float16"):
+    """IR of ``stages`` over two images, and an executor of it: execute({"x": buffer})."""
+    from functools import partial
+
+    from cuda_compiler import compile_subgraph, is_cuda_op_supported
+    from cuda_runtime import CUDABackend
+    from npu_compiler import partition
+    from npu_runtime import DAGExecutor
+
+    torch.manual_seed(0)
+    model = torch.nn.Sequential(*stages).eval()
+    ir = extract_ir(model, (torch.zeros(2, 3, size, size),), "head")
+    dag = DAGExecutor(partition(ir, is_cuda_op_supported), CUDABackend(), partial(compile_subgraph, compute_dtype=compute_dtype))
+    dag.load_weights(mz.state_dict_numpy(model.state_dict()))
+    return model, ir, dag
+
+
+def _stem():
+    return [torch.nn.Conv2d(3, 16, 7, 2, 3), torch.nn.ReLU(), torch.nn.MaxPool2d(3, 2, 1)]
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.float32, torch.uint8])
+@pytest.mark.parametrize("layout", ["channels_last", "sliced", "transposed", "permuted"])
+def test_images_that_are_not_contiguous_are_refused(fake_native, dtype, layout):
+    """In the compute dtype or to be converted to it, at a new address or at that of a contiguous image seen before."""
+    from cuda_runtime import CUDABuffer
+
+    model, ir, dag = _network_head(_stem())
+    name = ir["graph_inputs"][0]["name"]
+    base = (torch.rand(2, 3, 32, 32, generator=torch.Generator().manual_seed(1)) * 4).to(dtype)
+    run = lambda t: to_f32(dag.execute({name: CUDABuffer(t)})[ir["graph_outputs"][0]["name"]])
+    np.testing.assert_allclose(run(base), model(base.float()).detach().numpy(), rtol=2e-3, atol=2e-3)
+    wide = torch.zeros(2, 3, 32, 40, dtype=dtype)
+    wide[..., :32] = base
+    bad = {"channels_last": base.contiguous(memory_format=torch.channels_last), "sliced": wide[..., :32], "transposed": base.transpose(2, 3),
+           "permuted": base.permute(0, 2, 3, 1).contiguous().permute(0, 3, 1, 2)}[layout]
+    assert not bad.is_contiguous()
+    with pytest.raises(RuntimeError, match="contiguous"):
+        run(bad)
+    np.testing.assert_allclose(run(base), model(base.float()).detach().numpy(), rtol=2e-3, atol=2e-3)
+
+
 def test_qwen_tiny_golden_prefill_then_decode(fake_native):
     from golden.make_golden import tiny_qwen
 
