@@ -234,7 +234,8 @@ __global__ void __launch_bounds__(PF5_THREADS, 1)
   if (warp == 9) {
     if (lane == 0) {   // ---- TMA producer: one instruction per tile (the maps split the head dimension into (64, 2): two panels) ----
       int n = 0;
-      if (missed && (!tc5::mbar_wait(&k_full[0], 0) || !tc5::mbar_wait(&v_full[0], 0))) { failed = 1; atomicExch(&g_tc5_error, 29); }
+      // (with no tile at all nobody else looks for Q: every copy has landed before the CTA leaves)
+      if (missed && !(tc5::mbar_wait(&k_full[0], 0) & tc5::mbar_wait(&v_full[0], 0) & tc5::mbar_wait(&q_full, 0))) { failed = 1; atomicExch(&g_tc5_error, 29); }
       uint32_t masks = 0;   // mixed tiles so far of each buffer, 16 bits each
       for (; n < N; ++n) {
         const int st = n & 1, j = s_tile[n] & (MIXED - 1);

@@ -696,6 +696,36 @@ def test_attn_prefill_many_launches_in_a_row(lib, T):
     assert code.value == 0
 
 
+@pytest.mark.parametrize("known", [True, False])
+def test_attn_prefill_row_blocks_without_keys(lib, known):
+    """Blocks of 128 rows whose mask admits no key have only their copies to wait for: next to blocks that work, and in
+    launches that follow at once and use the same shared memory, with states found beforehand and by the kernel itself."""
+    dtype, Hq, Hkv, D, T, S = torch.bfloat16, 12, 2, 128, 1700, 300
+    q, k, v = gen((1, Hq, T, D), dtype), gen((1, Hkv, S, D), dtype, 1), gen((1, Hkv, S, D), dtype, 2)
+    mask = torch.full((1, T, 304), torch.finfo(dtype).min, dtype=dtype)
+    mask[:, 128 * 3:128 * 5, :S] = 0
+    Q, K, V, M = q.cuda(), k.cuda(), v.cuda(), mask.cuda()
+    tiles = torch.empty(1, -(-T // 128), -(-S // 128), dtype=torch.uint8, device="cuda")
+    ok(lib, lib.b200_mask_tiles(M.data_ptr(), 1, T, S, 0, 304, 2, tiles.data_ptr(), stream()))
+    st = lambda t: (C.c_int64 * 3)(*t.stride()[:3])
+    outs = [torch.full((1, T, Hq, D), float("nan"), dtype=dtype, device="cuda") for _ in range(50)]
+    for out in outs:
+        ok(lib, lib.b200_attn_prefill_tiles(Q.data_ptr(), K.data_ptr(), V.data_ptr(), M.data_ptr(), tiles.data_ptr() if known else None, out.data_ptr(), 1, Hq, Hkv,
+                                            T, S, D, st(Q), st(K), st(V), 0, 304, D ** -0.5, 2, stream()))
+    rows = slice(128 * 3, 128 * 5)
+    p = ((q[:, :, rows].double() @ k.double().repeat_interleave(6, 1).transpose(2, 3)) * D ** -0.5).softmax(-1)
+    vd = v.double().repeat_interleave(6, 1)
+    want, size = (p @ vd).transpose(1, 2), (p @ vd.abs()).transpose(1, 2)
+    for out in outs:
+        got = out.double().cpu()
+        assert ((got[:, rows] - want).abs() <= (size + want.abs()) * 2.0 ** -8 * 1.01 + 1e-5).all()
+        got[:, rows] = 0
+        assert not got.any()
+    code = C.c_int(0)
+    ok(lib, lib.b200_debug_device_error(C.byref(code), 1))
+    assert code.value == 0
+
+
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
 def test_attn_prefill_arbitrary_masks_and_no_mask(lib, dtype):
     """Nothing in the kernels assumes a causal mask: a per-sequence mask with windows, holes and key
