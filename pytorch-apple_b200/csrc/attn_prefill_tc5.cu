@@ -360,10 +360,10 @@ __global__ void __launch_bounds__(PF5_THREADS, 1)
           }
         }
         to_log2 = 1.f;
-      } else if (c < 0.f) {
+      } else if (c <= 0.f) {   // (with the factor left for later the maximum would be the minimum, and 0 times an absent key's -infinity no number)
 #pragma unroll
-        for (int e = 0; e < 64; ++e) u[e] = -u[e];
-        to_log2 = -c;
+        for (int e = 0; e < 64; e += 2) tc5::mul2(u[e], u[e + 1], c);
+        to_log2 = 1.f;
       }
       if (left < 64) {   // keys past the end
 #pragma unroll

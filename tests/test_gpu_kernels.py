@@ -696,6 +696,31 @@ def test_attn_prefill_many_launches_in_a_row(lib, T):
     assert code.value == 0
 
 
+@pytest.mark.parametrize("scale", [0.0, -0.07])
+@pytest.mark.parametrize("S", [100, 129, 200, 256])
+@pytest.mark.parametrize("masked", [None, "zero", "causal"])
+def test_attn_prefill_scales_that_are_not_positive(lib, masked, S, scale):
+    """Scale 0 weighs all keys alike and a negative one turns their order round, also where the last key tile, or half of it,
+    lies past the end.  Bound as for any mask: 2^-8 of what is added up."""
+    dtype, Hq, Hkv, D, T = torch.bfloat16, 4, 2, 128, 130
+    q, k, v = gen((1, Hq, T, D), dtype), gen((1, Hkv, S, D), dtype, 1), gen((1, Hkv, S, D), dtype, 2)
+    mask = torch.zeros(1, T, S).to(dtype) if masked == "zero" else _mask_of("causal", 1, T, S, dtype) if masked else None
+    s = (q.double() @ k.double().repeat_interleave(2, 1).transpose(2, 3)) * scale + (mask.double()[:, None] if masked else 0)
+    dead = (mask.double() <= -1e30).all(-1)[:, None, :, None] if masked else torch.zeros((), dtype=torch.bool)
+    p, vd = s.softmax(-1) * ~dead, v.double().repeat_interleave(2, 1)
+    want, size = (p @ vd).transpose(1, 2), (p @ vd.abs()).transpose(1, 2)
+    pitch = -(-S // 8) * 8
+    Q, K, V, M = q.cuda(), k.cuda(), v.cuda(), torch.zeros(1, T, pitch, dtype=dtype, device="cuda")
+    if masked:
+        M[..., :S] = mask.cuda()
+    st = lambda t: (C.c_int64 * 3)(*t.stride()[:3])
+    out = torch.full((1, T, Hq, D), float("nan"), dtype=dtype, device="cuda")
+    ok(lib, lib.b200_attn_prefill(Q.data_ptr(), K.data_ptr(), V.data_ptr(), M.data_ptr() if masked else None, out.data_ptr(), 1, Hq, Hkv, T, S, D,
+                                  st(Q), st(K), st(V), 0, pitch if masked else 0, scale, 2, stream()))
+    err = (out.double().cpu() - want).abs()
+    assert (err <= (size + want.abs()) * 2.0 ** -8 * 1.01 + 1e-5).all(), float(err.max())
+
+
 @pytest.mark.parametrize("known", [True, False])
 def test_attn_prefill_row_blocks_without_keys(lib, known):
     """Blocks of 128 rows whose mask admits no key have only their copies to wait for: next to blocks that work, and in
