@@ -120,6 +120,7 @@ __global__ void __launch_bounds__(SP_THREADS, 1) conv_stem_pool_kernel(const __g
 
   // Epilogue and pooler warps prepare what stays, while the first input rows are on their way
   if ((warp >= 1 && warp < 5) || (warp >= 9 && warp < 13)) {
+    pdl_wait();   // (the kernel before this one may be the one that prepares the weights)
     const int t = threadIdx.x - (warp < 5 ? 32 : 5 * 32);
     // weights [O][KH][7][8] -> [two filter rows][O][row, plane, tap + 1] with the 128-byte swizzle; tap 0 and absent output channels are zero
     for (int i = t; i < p.KH * 4 * SP_BN; i += 256) {
@@ -286,7 +287,6 @@ __global__ void __launch_bounds__(SP_THREADS, 1) conv_stem_pool_kernel(const __g
   } else if (warp < 13) {
     // ---- poolers: pixel pw, eight channels per thread and step ----
     const int t = threadIdx.x - 9 * 32, k8 = t & 7;
-    pdl_wait();   // the output may still be read by the kernel before this one
     for (int k = 0; k < count; ++k) {
       const int row = first + k;
       const bool ok = __all_sync(0xffffffffu, tc5::mbar_wait(&v_ready[k & 1], (k >> 1) & 1));

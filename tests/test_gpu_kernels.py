@@ -1223,6 +1223,31 @@ def test_conv_stem_pool_infinite_pixel(lib, dtype, W, relu):
         assert got[finite].isfinite().all() and ((got - want).abs()[finite] <= slack[finite]).all()
 
 
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+def test_conv_stem_pool_behind_the_kernel_that_prepares_its_weights(lib, dtype):
+    """Weights and bias written by the launch before, over and over: each call sees its own, bit for bit."""
+    N, H, W, O = 4, 64, 64, 64
+    x = gen((N, 3, H, W), dtype).cuda()
+    sets = [(gen((O, 3, 7, 7), torch.float32, s, 0.1).cuda(), gen((O,), torch.float32, s + 50).cuda()) for s in range(24)]
+    packed, bias = torch.empty(O, 7, 7, 8, dtype=dtype, device="cuda"), torch.empty(O, dtype=torch.float32, device="cuda")
+    outs = [torch.full((N, 16, 16, O), float("nan"), dtype=dtype, device="cuda") for _ in range(2 * len(sets))]
+
+    def call(i, out, wait):
+        w, b = sets[i]
+        ok(lib, lib.b200_conv_weight_prep(w.data_ptr(), b.data_ptr(), None, None, None, None, packed.data_ptr(), bias.data_ptr(), O, 3, 7, 7, 8, 0.0, 0, 0, DT[dtype], stream()))
+        if wait:
+            torch.cuda.synchronize()
+        ok(lib, lib.b200_conv_stem_pool(x.data_ptr(), packed.data_ptr(), bias.data_ptr(), out.data_ptr(), N, 3, H, W, 8, O, 7, 7, 2, 2, 3, 3, DT[dtype], 1, stream()))
+
+    for i in range(len(sets)):
+        call(i, outs[i], False)
+    for i in range(len(sets)):
+        call(i, outs[len(sets) + i], True)
+    for i in range(len(sets)):
+        assert torch.equal(outs[i], outs[len(sets) + i]) and outs[i].isfinite().all()
+    assert not torch.equal(outs[0], outs[1])
+
+
 def test_conv_stem_pool_shapes_it_does_not_take(lib):
     for bad in [(5, 32, 32, 8, 64, 7, 7, 2, 2, 3, 3, 1), (3, 32, 258, 8, 64, 7, 7, 2, 2, 3, 3, 1), (3, 32, 32, 8, 72, 7, 7, 2, 2, 3, 3, 1), (3, 32, 32, 8, 64, 9, 7, 2, 2, 3, 3, 1),
                 (3, 32, 32, 8, 64, 7, 7, 1, 1, 3, 3, 1), (3, 32, 32, 8, 64, 7, 5, 2, 2, 3, 3, 1), (3, 32, 32, 8, 64, 7, 7, 2, 2, 3, 3, 0)]:
