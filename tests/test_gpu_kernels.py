@@ -1275,7 +1275,9 @@ def test_adaptive_avg_pool_channels_last(lib, dtype, N, Cn, H, W, OH, OW):
     (7, 56, 56, 64, 64, False, True), (12, 56, 56, 64, 64, True, True),      # weights resident, two issuing threads; with residual
     (20, 31, 30, 64, 64, False, False), (9, 57, 55, 64, 40, True, False),    # last tiles of an image shorter, fewer channels than a tile
     (3, 90, 126, 64, 64, False, True), (25, 28, 28, 128, 128, True, True),   # one row per tile; weights streamed, one tile per unit
-    (127, 28, 28, 128, 128, False, True), (20, 28, 28, 64, 200, True, True),  # two tiles per unit, an odd number of tiles; two column tiles
+    (127, 28, 28, 128, 128, False, True), (20, 28, 28, 64, 200, True, True),  # one tile per unit; two, and two column tiles
+    (125, 28, 28, 128, 128, False, True), (125, 28, 28, 128, 128, True, False),   # two tiles per unit, an odd number of tiles
+    (21, 28, 28, 64, 200, True, True), (41, 28, 28, 64, 200, False, False),      # the same in each of two column tiles
     (35, 14, 14, 256, 256, True, True), (40, 14, 14, 192, 136, False, True), (300, 7, 15, 64, 128, False, True),   # tiles of eight rows; a whole image per tile
     (48, 14, 14, 256, 256, True, True)])                                     # (the im2col route)
 def test_conv3x3_rows(lib, dtype, N, H, W, Cn, O, res, relu):
@@ -1301,6 +1303,24 @@ def test_conv3x3_rows(lib, dtype, N, H, W, Cn, O, res, relu):
     code = C.c_int(0)
     ok(lib, lib.b200_debug_device_error(C.byref(code), 1))
     assert code.value == 0
+
+
+@pytest.mark.parametrize("N,H,Cn,O,kernel", [(20, 56, 64, 64, "conv_rows_kernel<__half, 64, 1, true>"), (127, 28, 128, 128, "conv_rows_kernel<__half, 128, 1, false>"),
+                                             (20, 28, 128, 128, "conv_rows_kernel<__half, 128, 1, false>"), (125, 28, 128, 128, "conv_rows_kernel<__half, 128, 2, false>"),
+                                             (20, 28, 64, 200, "conv_rows_kernel<__half, 128, 2, false>"), (21, 28, 64, 200, "conv_rows_kernel<__half, 128, 2, false>"),
+                                             (48, 14, 256, 256, "gemm_tc5p_kernel"), (256, 14, 256, 256, "gemm_tc5p_kernel"), (20, 56, 128, 64, "gemm_tc5p_kernel"),
+                                             (2, 56, 64, 64, "gemm_tc5_kernel")])
+def test_conv3x3_runs_on_the_kernel_that_its_shape_calls_for(lib, N, H, Cn, O, kernel):
+    x, w = torch.zeros(N, H, H, Cn, dtype=torch.float16, device="cuda"), torch.zeros(O, 3, 3, Cn, dtype=torch.float16, device="cuda")
+    y = torch.empty(N, H, H, O, dtype=torch.float16, device="cuda")
+    call = lambda: ok(lib, lib.b200_conv2d_nhwc(x.data_ptr(), w.data_ptr(), None, None, y.data_ptr(), N, H, H, Cn, Cn, O, 3, 3, 1, 1, 1, 1, H, H, 1, 0, stream()))
+    names = []
+    for _ in range(3):   # (a profiling session now and then reports nothing)
+        with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CUDA]) as prof:
+            call()
+            torch.cuda.synchronize()
+        names = names or [e.key for e in prof.key_averages() if "_kernel" in e.key]
+    assert len(names) == 1 and kernel in names[0], names
 
 
 @pytest.mark.parametrize("M", [65, 80, 128, 129, 250, 257, 273, 500, 777])
