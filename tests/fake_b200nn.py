@@ -457,7 +457,7 @@ class FakeLibrary:
                    and 0 <= ph < KH and (W - 1) // 2 + 1 <= 128 and H + 2 * ph >= KH and dtype in (1, 2))
 
     def b200_conv_stem_pool(self, x, w, bias, y, N, Cn, H, W, C_pad, O, KH, KW, sh, sw, ph, pw, dtype, epilogue, stream):
-        self.calls += ["conv2d", "max_pool2d"]
+        self.calls += ["conv_stem_pool", "conv2d", "max_pool2d"]   # (itself and the operators that it stands for)
         dt = _DT[dtype]
         X = _raw(x, dt, [N, Cn, H, W], [Cn * H * W, H * W, W, 1]).float()
         Wt = _raw(w, dt, [O, C_pad, KH, KW], [KH * KW * C_pad, 1, KW * C_pad, C_pad]).float()[:, :Cn]

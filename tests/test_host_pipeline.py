@@ -144,10 +144,11 @@ def test_resnet18_golden(fake_native):
     np.testing.assert_allclose(got, fx["logits"], rtol=0, atol=1e-1)  # the reference's ResNet-18 tolerance
     assert (np.argsort(-got, 1)[:, :5] == np.argsort(-fx["logits"], 1)[:, :5]).all()
     assert fake_native.calls.count("conv2d") == 20 and "batch_norm" not in fake_native.calls
+    assert fake_native.calls.count("conv_stem_pool") == 1
 
 
-def _network_head(stages, size=32, compute_dtype="float16"):
-    """IR of ``stages`` over two images, and an executor of it: execute({"x": buffer})."""
+def _network_head(stages, size=32):
+    """A model of ``stages`` over two images, its IR, and a DAGExecutor with its weights that computes in fp16."""
     from functools import partial
 
     from cuda_compiler import compile_subgraph, is_cuda_op_supported
@@ -158,7 +159,7 @@ def _network_head(stages, size=32, compute_dtype="float16"):
     torch.manual_seed(0)
     model = torch.nn.Sequential(*stages).eval()
     ir = extract_ir(model, (torch.zeros(2, 3, size, size),), "head")
-    dag = DAGExecutor(partition(ir, is_cuda_op_supported), CUDABackend(), partial(compile_subgraph, compute_dtype=compute_dtype))
+    dag = DAGExecutor(partition(ir, is_cuda_op_supported), CUDABackend(), partial(compile_subgraph, compute_dtype="float16"))
     dag.load_weights(mz.state_dict_numpy(model.state_dict()))
     return model, ir, dag
 
@@ -186,6 +187,53 @@ def test_images_that_are_not_contiguous_are_refused(fake_native, dtype, layout):
     with pytest.raises(RuntimeError, match="contiguous"):
         run(bad)
     np.testing.assert_allclose(run(base), model(base.float()).detach().numpy(), rtol=2e-3, atol=2e-3)
+
+
+class _Head(torch.nn.Module):
+    """7x7 / 2 convolution, ReLU and pooling, in the ways that have to stay three kernels (or, "plain" and "slice", one)."""
+
+    def __init__(self, kind):
+        super().__init__()
+        self.kind = kind
+        self.conv, self.other = torch.nn.Conv2d(3, 16, 7, 2, 3), torch.nn.Conv2d(3, 16, 7, 2, 3)
+        self.pool = {"window": torch.nn.MaxPool2d(2, 2), "padding": torch.nn.MaxPool2d(3, 2, 0), "stride": torch.nn.MaxPool2d(3, 1, 1)}.get(
+            kind, torch.nn.MaxPool2d(3, 2, 1))
+
+    def forward(self, x):
+        if self.kind == "slice":        # planar, but not the start of its buffer
+            x = x[1:]
+        if self.kind == "computed":     # no graph input
+            x = x * 2.0
+        y = self.conv(x)
+        if self.kind == "residual":
+            y = y + self.other(x)
+        y = torch.relu(y)
+        p = self.pool(y)
+        if self.kind == "conv is a result":
+            return p, y
+        if self.kind == "conv is read again":
+            return p, y * 2.0
+        if self.kind == "image is read again":
+            return p, self.other(x)
+        if self.kind == "pooled twice":
+            return p, self.pool(y * 0.5)
+        return p
+
+
+@pytest.mark.parametrize("kind,fused", [("plain", True), ("slice", True), ("computed", False), ("conv is a result", False), ("conv is read again", False),
+                                        ("image is read again", False), ("pooled twice", False), ("residual", False), ("window", False), ("padding", False),
+                                        ("stride", False)])
+def test_network_heads_that_are_one_kernel_and_those_that_are_not(fake_native, kind, fused):
+    from cuda_runtime import CUDABuffer
+
+    model, ir, dag = _network_head([_Head(kind)])
+    x = torch.randn(2, 3, 32, 32, generator=torch.Generator().manual_seed(1)).half()
+    for scale in (1.0, -0.5):   # (the second call replays a launch list)
+        out = dag.execute({ir["graph_inputs"][0]["name"]: CUDABuffer(x * scale)})
+        want = model((x * scale).float())
+        for spec, ref in zip(ir["graph_outputs"], want if isinstance(want, tuple) else (want,)):
+            np.testing.assert_allclose(to_f32(out[spec["name"]]), ref.detach().numpy(), rtol=4e-3, atol=4e-3)
+    assert fake_native.calls.count("conv_stem_pool") == (2 if fused else 0)
 
 
 def test_qwen_tiny_golden_prefill_then_decode(fake_native):
