@@ -126,30 +126,6 @@ __device__ __forceinline__ void finish_cols(const Tc5Params& p, float (&v)[CNT],
   store_cols<T, CNT>(static_cast<T*>(p.out) + m * p.ldo + n, v, cnt);
 }
 
-// finish_cols with the residual already in registers (16 values as two 16-byte words); no silu_mul term
-template <typename T>
-__device__ __forceinline__ void finish_cols_res(const Tc5Params& p, float (&v)[16], int64_t m, int64_t n, const uint4& r0, const uint4& r1) {
-  const int cnt = static_cast<int>(p.N - n < 16 ? p.N - n : 16);
-  add_bias<16>(p, v, n, cnt);
-  float r[16], t[8];
-  unpack8<T>(r0, t);
-#pragma unroll
-  for (int i = 0; i < 8; ++i) r[i] = t[i];
-  unpack8<T>(r1, t);
-#pragma unroll
-  for (int i = 0; i < 8; ++i) r[8 + i] = t[i];
-#pragma unroll
-  for (int i = 0; i < 16; i += 2) {
-    round2<T>(v[i], v[i + 1]);
-    v[i] += r[i]; v[i + 1] += r[i + 1];
-  }
-  if (p.epilogue & B200_EPI_RELU) {
-#pragma unroll
-    for (int i = 0; i < 16; ++i) v[i] = fmaxf(v[i], 0.f);
-  }
-  store_cols<T, 16>(static_cast<T*>(p.out) + m * p.ldo + n, v, cnt);
-}
-
 // gated-MLP epilogue: CNT gate accumulators (merged columns n_merged..) and the matching up
 // accumulators (merged columns n_merged + 64 ..) of row m -> CNT outputs starting at column n_out
 template <typename T, int CNT>

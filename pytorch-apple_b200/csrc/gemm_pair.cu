@@ -185,72 +185,72 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PR_THREADS, 1)
         tc5::tmem_ld_32x32_async(t_row + PR_CHUNK * g, v);
 #pragma unroll 1
         for (int c = PR_CHUNK * g; c < nt; c += 2 * PR_CHUNK) {
-        const int cnt = nt - c < PR_CHUNK ? nt - c : PR_CHUNK;
-        const int tokens = static_cast<int>(p.M - m0 - c < cnt ? (p.M - m0 - c < 0 ? 0 : p.M - m0 - c) : cnt);   // that exist
-        // 16-byte words of the result that this thread finishes: token i / 16, columns 8 (i % 16) .. (gated: i / 8, i % 8); residual requested now
-        uint4 r[4];
-        if (res_vec) {
+          const int cnt = nt - c < PR_CHUNK ? nt - c : PR_CHUNK;
+          const int tokens = static_cast<int>(p.M - m0 - c < cnt ? (p.M - m0 - c < 0 ? 0 : p.M - m0 - c) : cnt);   // that exist
+          // 16-byte words of the result that this thread finishes: token i / 16, columns 8 (i % 16) .. (gated: i / 8, i % 8); residual requested now
+          uint4 r[4];
+          if (res_vec) {
 #pragma unroll
-          for (int k = 0; k < 4; ++k) {
-            const int i = t + 128 * k, j = i >> 4;
-            const int64_t n = n0 + 8 * (i & 15);
-            r[k] = j < tokens && n < p.N ? __ldg(reinterpret_cast<const uint4*>(res + (m0 + c + j) * p.ldr + n)) : make_uint4(0u, 0u, 0u, 0u);
+            for (int k = 0; k < 4; ++k) {
+              const int i = t + 128 * k, j = i >> 4;
+              const int64_t n = n0 + 8 * (i & 15);
+              r[k] = j < tokens && n < p.N ? __ldg(reinterpret_cast<const uint4*>(res + (m0 + c + j) * p.ldr + n)) : make_uint4(0u, 0u, 0u, 0u);
+            }
           }
-        }
-        T* const turn = reinterpret_cast<T*>(buf + (round & 1) * PR_BUF);
-        ++round;
-        tc5::tmem_ld_wait();
+          T* const turn = reinterpret_cast<T*>(buf + (round & 1) * PR_BUF);
+          ++round;
+          tc5::tmem_ld_wait();
 #pragma unroll
-        for (int j = 0; j < PR_CHUNK; ++j) turn[j * 128 + t] = from_f32<T>(v[j] + bias);
-        if (c + 2 * PR_CHUNK < nt) tc5::tmem_ld_32x32_async(t_row + c + 2 * PR_CHUNK, v);   // the next 32 tokens, while these are finished
-        // (two buffers: whoever writes one again has passed the barrier behind which everybody had read it)
-        asm volatile("bar.sync %0, 128;" ::"r"(1 + g) : "memory");
-        if (glu) {
+          for (int j = 0; j < PR_CHUNK; ++j) turn[j * 128 + t] = from_f32<T>(v[j] + bias);
+          if (c + 2 * PR_CHUNK < nt) tc5::tmem_ld_32x32_async(t_row + c + 2 * PR_CHUNK, v);   // the next 32 tokens, while these are finished
+          // (two buffers: whoever writes one again has passed the barrier behind which everybody had read it)
+          asm volatile("bar.sync %0, 128;" ::"r"(1 + g) : "memory");
+          if (glu) {
 #pragma unroll
-          for (int k = 0; k < 2; ++k) {
-            const int i = t + 128 * k, j = i >> 3, cc = 8 * (i & 7);
-            if (j < tokens && n0 < p.N) {   // (N is a multiple of 128: the block is whole)
-              float gt[8], up[8];
-              unpack8<T>(*reinterpret_cast<const uint4*>(turn + j * 128 + cc), gt);
-              unpack8<T>(*reinterpret_cast<const uint4*>(turn + j * 128 + 64 + cc), up);
+            for (int k = 0; k < 2; ++k) {
+              const int i = t + 128 * k, j = i >> 3, cc = 8 * (i & 7);
+              if (j < tokens && n0 < p.N) {   // (N is a multiple of 128: the block is whole)
+                float gt[8], up[8];
+                unpack8<T>(*reinterpret_cast<const uint4*>(turn + j * 128 + cc), gt);
+                unpack8<T>(*reinterpret_cast<const uint4*>(turn + j * 128 + 64 + cc), up);
 #pragma unroll
-              for (int e = 0; e < 8; e += 2) {
-                float a = silu_f32(gt[e]), d = silu_f32(gt[e + 1]);
-                round2<T>(a, d);
-                gt[e] = a * up[e]; gt[e + 1] = d * up[e + 1];
+                for (int e = 0; e < 8; e += 2) {
+                  float a = silu_f32(gt[e]), d = silu_f32(gt[e + 1]);
+                  round2<T>(a, d);
+                  gt[e] = a * up[e]; gt[e + 1] = d * up[e + 1];
+                }
+                store_cols<T, 8>(static_cast<T*>(p.out) + (m0 + c + j) * p.ldo + n0 / 2 + cc, gt, 8);
               }
-              store_cols<T, 8>(static_cast<T*>(p.out) + (m0 + c + j) * p.ldo + n0 / 2 + cc, gt, 8);
+            }
+          } else {
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+              const int i = t + 128 * k, j = i >> 4;
+              const int64_t n = n0 + 8 * (i & 15), m = m0 + c + j;
+              if (j >= tokens || n >= p.N) continue;
+              const int left = static_cast<int>(p.N - n < 8 ? p.N - n : 8);
+              float f[8];
+              unpack8<T>(*reinterpret_cast<const uint4*>(turn + j * 128 + 8 * (i & 15)), f);
+              if (res) {
+                float rf[8];
+                if (res_vec) unpack8<T>(r[k], rf);
+                else load_cols<T, 8>(res, p.ldr, m, n, left, rf);
+#pragma unroll
+                for (int e = 0; e < 8; ++e) f[e] += rf[e];
+              }
+              if (relu) {
+#pragma unroll
+                for (int e = 0; e < 8; ++e) f[e] = fmaxf(f[e], 0.f);
+              }
+              if (silu) {
+                float x[8];
+                load_cols<T, 8>(static_cast<const T*>(p.aux), p.ldaux, m, n, left, x);
+#pragma unroll
+                for (int e = 0; e < 8; ++e) f[e] = round_as<T>(silu_f32(round_as<T>(f[e]))) * x[e];
+              }
+              store_cols<T, 8>(static_cast<T*>(p.out) + m * p.ldo + n, f, left);
             }
           }
-        } else {
-#pragma unroll
-          for (int k = 0; k < 4; ++k) {
-            const int i = t + 128 * k, j = i >> 4;
-            const int64_t n = n0 + 8 * (i & 15), m = m0 + c + j;
-            if (j >= tokens || n >= p.N) continue;
-            const int left = static_cast<int>(p.N - n < 8 ? p.N - n : 8);
-            float f[8];
-            unpack8<T>(*reinterpret_cast<const uint4*>(turn + j * 128 + 8 * (i & 15)), f);
-            if (res) {
-              float rf[8];
-              if (res_vec) unpack8<T>(r[k], rf);
-              else load_cols<T, 8>(res, p.ldr, m, n, left, rf);
-#pragma unroll
-              for (int e = 0; e < 8; ++e) f[e] += rf[e];
-            }
-            if (relu) {
-#pragma unroll
-              for (int e = 0; e < 8; ++e) f[e] = fmaxf(f[e], 0.f);
-            }
-            if (silu) {
-              float x[8];
-              load_cols<T, 8>(static_cast<const T*>(p.aux), p.ldaux, m, n, left, x);
-#pragma unroll
-              for (int e = 0; e < 8; ++e) f[e] = round_as<T>(silu_f32(round_as<T>(f[e]))) * x[e];
-            }
-            store_cols<T, 8>(static_cast<T*>(p.out) + m * p.ldo + n, f, left);
-          }
-        }
           __syncwarp();
         }
       }
