@@ -6,7 +6,9 @@
 // A persistent CTA owns consecutive pooled rows and walks the convolution rows that they need (two per pooled row, three
 // for the first one of a CTA or an image); nothing between the image and the pooled row leaves the SM:
 // - a producer thread brings new input rows in pairs, planar as they are, by TMA (rows and pixels outside the image
-//   arrive as zeros) into a ring; images whose rows are no whole 16-byte words are copied there by the loaders themselves;
+//   arrive as zeros) into a ring; images whose rows are no whole 16-byte words, or wider than one box, are copied there by the loaders
+//   themselves, element by element, which is slower than the three kernels (256 wide, 128 images: 798 us against 360): the executor
+//   keeps those for such images;
 // - loaders (128 threads, one per column) write them to a window of 16 row slots as sliding windows: per plane, 16 bytes for
 //   output column p hold its pixels 2p - 4 .. 2p + 3 - the eight taps of a filter row, the first of which is no tap and zero.  That
 //   is the unswizzled K-major core-matrix layout (8 columns x 16 bytes, every core matrix a 128-byte line), and the MMA reads its A

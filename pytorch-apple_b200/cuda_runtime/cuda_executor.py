@@ -32,7 +32,7 @@ from typing import Any
 from cuda_compiler.cuda_codegen import EW_OPCODES
 from cuda_compiler.cuda_program import AliasStep, CUDAProgram, TensorView
 from cuda_runtime import native
-from cuda_runtime.native import DTYPE_BYTES, DTYPE_CODES, MASK_TILE
+from cuda_runtime.native import DTYPE_BYTES, DTYPE_CODES, MASK_TILE, STEM_TMA_WIDTH
 
 try:
     import torch
@@ -62,10 +62,14 @@ def _views_of(value):
             yield from _views_of(v)
 
 
-def _find_stems(program: CUDAProgram, lib) -> dict[int, tuple | None]:
+def _find_stems(program: CUDAProgram, lib) -> list[tuple[int, int, int]]:
     """Heads of convolution networks that run as one kernel: the repack of a planar graph input to channels-last, a convolution
     of it, and a 3x3 / 2 max-pooling of the result, with nothing else reading what lies in between (256 images of a
-    ResNet: 600 us as three kernels, 173 as one).  {index of the pooling step: (repack, convolution, pooling) parameters, other two: None}."""
+    ResNet: 584 us as three kernels, 172 as one).  Indices of the three steps.
+
+    Only images whose rows TMA can copy: others the kernel copies element by element (us, three kernels against one: 8 / 128
+    images 223 wide 32 against 42 / 301 against 583, 256 wide 35 against 44 / 360 against 798, 33 wide 15 against 16 / 41
+    against 50; 200 wide, by TMA, 30 against 12 / 259 against 81)."""
     steps = [(i, s.params) for i, s in enumerate(program.steps) if getattr(s, "params", None)]
     users: dict[str, list[int]] = {}
     for i, p in steps:
@@ -76,7 +80,7 @@ def _find_stems(program: CUDAProgram, lib) -> dict[int, tuple | None]:
         if view is not None:
             users.setdefault(view.buffer, []).append(-1)
     inputs = {s.name for s in program.input_specs}
-    params, found = dict(steps), {}
+    params, found = dict(steps), []
     for i, copy in steps:
         if copy.get("op") != "strided_copy" or copy["in_view"].buffer not in inputs or len(copy["in_view"].shape) != 4:
             continue
@@ -93,13 +97,13 @@ def _find_stems(program: CUDAProgram, lib) -> dict[int, tuple | None]:
         N, Cn, H, W = x.shape
         O, PH, PW = y.shape[1], (y.shape[2] - 1) // 2 + 1, (y.shape[3] - 1) // 2 + 1
         cv = [conv[k] for k in ("c_pad", "out_channels", "kernel_h", "kernel_w", "stride_h", "stride_w", "pad_h", "pad_w")]
-        if (x.dtype == y.dtype == pool["y"].dtype and tuple(x.strides) == (Cn * H * W, H * W, W, 1) and tuple(copy["out_view"].shape) == tuple(x.shape)
+        if (W % 8 == 0 and W <= STEM_TMA_WIDTH and x.dtype == y.dtype == pool["y"].dtype and tuple(x.strides) == (Cn * H * W, H * W, W, 1) and tuple(copy["out_view"].shape) == tuple(x.shape)
                 and conv["x"].offset == copy["out_view"].offset and tuple(pool["x"].shape) == tuple(y.shape)
                 and tuple(pool["x"].strides) == tuple(y.strides) and pool["x"].offset == y.offset
                 and [pool[k] for k in ("kernel_h", "kernel_w", "stride_h", "stride_w", "pad_h", "pad_w")] == [3, 3, 2, 2, 1, 1]
                 and tuple(pool["y"].shape) == (N, O, PH, PW) and tuple(pool["y"].strides) == (PH * PW * O, 1, PW * O, O)
                 and pool["y"].offset % 8 == 0 and lib.b200_conv_stem_pool_supported(Cn, H, W, *cv, DTYPE_CODES[y.dtype])):
-            found.update({i: None, others[1]: None, others[0]: (copy, conv, pool)})
+            found.append((i, others[1], others[0]))
     return found
 
 
@@ -435,15 +439,19 @@ class CUDAExecutor:
         self._cur_inputs = inputs
         self._cur_plan = plan
         self._staged: dict[str, Any] = {}
+        merged = {}   # steps that one kernel stands for: nothing to bind, except at the last of them
+        for at in self._stems:
+            copy, conv, pool = (self._program.steps[i].params for i in at)
+            if self._ptr(copy["in_view"]) % 16 == 0:   # TMA: a slice of a larger tensor may start anywhere
+                merged.update({at[0]: None, at[1]: None, at[2]: (copy, conv, pool)})
         for i, step in enumerate(self._program.steps):
             if isinstance(step, AliasStep):
                 continue
             p = step.params
-            stem = self._stems.get(i, p)
-            if stem is p:
+            if i not in merged:
                 getattr(self, "_bind_" + p["op"])(plan, step, p)
-            elif stem is not None:
-                self._bind_stem_pool(plan, *stem)
+            elif merged[i] is not None:
+                self._bind_stem_pool(plan, *merged[i])
         # every library call is one kernel, except decode attention when its splits are merged by a
         # second kernel (the library then asks for a workspace; with in-kernel merging it asks for none)
         def _two_kernels(q) -> bool:

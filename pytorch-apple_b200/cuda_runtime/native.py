@@ -25,6 +25,7 @@ EPI_GLU = 4
 EPI_W_STATIC = 8
 
 MASK_TILE = 128   # rows and keys of a tile of b200_mask_tiles
+STEM_TMA_WIDTH = 240   # widest image that b200_conv_stem_pool brings in by TMA (rows of whole 16-byte words)
 
 
 class Tensor(C.Structure):

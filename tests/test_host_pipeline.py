@@ -189,6 +189,20 @@ def test_images_that_are_not_contiguous_are_refused(fake_native, dtype, layout):
     np.testing.assert_allclose(run(base), model(base.float()).detach().numpy(), rtol=2e-3, atol=2e-3)
 
 
+@pytest.mark.parametrize("size,shift,fused", [(32, 0, True), (240, 0, True), (240, 8, True), (32, 1, False), (30, 0, False), (33, 0, False), (248, 0, False)])
+def test_network_heads_whose_rows_tma_cannot_copy_keep_their_kernels(fake_native, size, shift, fused):
+    """Rows that are no whole 16-byte words, wider than one copy, or an image that starts between two words."""
+    from cuda_runtime import CUDABuffer
+
+    model, ir, dag = _network_head(_stem(), size)
+    flat = torch.randn(2 * 3 * size * size + shift, generator=torch.Generator().manual_seed(1)).half()
+    assert flat.data_ptr() % 16 == 0
+    x = flat[shift:].view(2, 3, size, size)
+    out = dag.execute({ir["graph_inputs"][0]["name"]: CUDABuffer(x)})
+    np.testing.assert_allclose(to_f32(out[ir["graph_outputs"][0]["name"]]), model(x.float()).detach().numpy(), rtol=4e-3, atol=4e-3)
+    assert fake_native.calls.count("conv_stem_pool") == int(fused) and fake_native.calls.count("conv2d") == 1
+
+
 class _Head(torch.nn.Module):
     """7x7 / 2 convolution, ReLU and pooling, in the ways that have to stay three kernels (or, "plain" and "slice", one)."""
 
