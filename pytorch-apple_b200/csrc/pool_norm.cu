@@ -256,9 +256,16 @@ extern "C" int b200_adaptive_avg_pool2d(const b200_tensor* x, const b200_tensor*
   B200_CHECK_ARG(fill_pool(&p, x, y) == 0 && p.OH > 0 && p.OW > 0, "b200_adaptive_avg_pool2d: bad arguments");
   const int64_t total = p.N * p.C * p.OH * p.OW;
   if (total == 0) return B200_OK;
+  // The block per output pixel pays where its 256 channels exist, the window gives its warps work or all blocks are resident at once.
+  // us, thread per output -> block per pixel, channels x window at 20000 pixels: 8 x 49 11 -> 101, 64 x 64 118 -> 138, 64 x 196 333 -> 299,
+  // 128 x 16 69 -> 88, 128 x 36 159 -> 111, 192 x 4 83 -> 69, 320 x 16 166 -> 180, 320 x 36 382 -> 224, 384 x 1 110 -> 126, 248 x 1 72 -> 64; 1200
+  // pixels 8 x 16 3.9 -> 5.9, 64 x 36 12.5 -> 7.9; 600 pixels 8 x 1 2.8 -> 2.8, 64 x 16 3.9 -> 3.4 (fewer blocks always gain).
+  const int64_t px = p.N * p.OH * p.OW, blocks = px * ceil_div(p.C, 256), idle = ceil_div(p.C, 256) * 256 - p.C;
+  const int64_t window = (p.H / p.OH) * (p.W / p.OW);   // the smallest
+  const bool pays = blocks <= 4 * sm_count() || window * p.C >= 48 * idle;
   // (the windows are counted in 32 bits; grid.y holds the output pixels)
-  if (words_of_channels(p) && p.N * p.OH * p.OW <= 65535 && p.H < (1 << 15) && p.W < (1 << 15) && p.OH < (1 << 15) && p.OW < (1 << 15)) {
-    const dim3 grid(static_cast<unsigned>(ceil_div(p.C, 256)), static_cast<unsigned>(p.N * p.OH * p.OW));
+  if (pays && words_of_channels(p) && px <= 65535 && p.H < (1 << 15) && p.W < (1 << 15) && p.OH < (1 << 15) && p.OW < (1 << 15)) {
+    const dim3 grid(static_cast<unsigned>(ceil_div(p.C, 256)), static_cast<unsigned>(px));
     if (p.x_dtype == B200_F16) launch_pdl(adaptive_avg_pool2d_cl8_kernel<__half>, grid, dim3(AVG_WARPS * 32), 0, static_cast<cudaStream_t>(stream), p);
     else launch_pdl(adaptive_avg_pool2d_cl8_kernel<__nv_bfloat16>, grid, dim3(AVG_WARPS * 32), 0, static_cast<cudaStream_t>(stream), p);
     B200_CHECK_LAUNCH("adaptive_avg_pool2d_cl8_kernel");

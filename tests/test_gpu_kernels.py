@@ -1270,6 +1270,26 @@ def test_adaptive_avg_pool_channels_last(lib, dtype, N, Cn, H, W, OH, OW):
     assert (err <= want.abs() * (2.0 ** -11 if dtype == torch.float16 else 2.0 ** -8) + size * 2.0 ** -20 + 6e-8).all(), float(err.max())
 
 
+@pytest.mark.parametrize("N,Cn,H,OH,kernel", [(592, 8, 2, 1, "adaptive_avg_pool2d_cl8_kernel"), (593, 8, 7, 1, "adaptive_avg_pool2d_kernel"), (4000, 64, 11, 1, "adaptive_avg_pool2d_kernel"),
+                                              (2000, 64, 13, 1, "adaptive_avg_pool2d_cl8_kernel"), (700, 248, 2, 1, "adaptive_avg_pool2d_cl8_kernel"), (700, 512, 7, 7, "adaptive_avg_pool2d_cl8_kernel"),
+                                              (40, 512, 14, 7, "adaptive_avg_pool2d_cl8_kernel"), (700, 264, 6, 1, "adaptive_avg_pool2d_kernel"), (700, 264, 7, 1, "adaptive_avg_pool2d_cl8_kernel")])
+def test_adaptive_avg_pool_runs_on_the_kernel_that_its_shape_calls_for(lib, N, Cn, H, OH, kernel):
+    """Both sides of each line of the rule (resident blocks, work per block, idle channels), and the result there."""
+    x = gen((N, Cn, H, H), torch.float16).cuda().contiguous(memory_format=torch.channels_last)
+    y = torch.empty(N, OH, OH, Cn, dtype=torch.float16, device="cuda").permute(0, 3, 1, 2)
+    a, b = bt(x), bt(y)
+    names = []
+    for _ in range(3):   # (a profiling session now and then reports nothing)
+        with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CUDA]) as prof:
+            ok(lib, lib.b200_adaptive_avg_pool2d(C.byref(a), C.byref(b), stream()))
+            torch.cuda.synchronize()
+        names = names or [e.key for e in prof.key_averages() if "_kernel" in e.key]
+    assert len(names) == 1 and kernel in names[0], names
+    want = torch.nn.functional.adaptive_avg_pool2d(x.double(), OH)
+    size = torch.nn.functional.adaptive_avg_pool2d(x.double().abs(), OH)
+    assert ((y.double() - want).abs() <= want.abs() * 2.0 ** -11 + size * 2.0 ** -20 + 6e-8).all()
+
+
 @pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
 @pytest.mark.parametrize("N,H,W,Cn,O,res,relu", [
     (7, 56, 56, 64, 64, False, True), (12, 56, 56, 64, 64, True, True),      # weights resident, two issuing threads; with residual
