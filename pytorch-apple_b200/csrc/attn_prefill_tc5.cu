@@ -227,15 +227,23 @@ __global__ void __launch_bounds__(PF5_THREADS, 1)
   tc5::tc_fence_after();
   const uint32_t tmem_base = tmem_holder;
   const int N = s_count;
-  // Tile 0 is not the first one: its copies count as a phase of stage 0 that nobody works on.
+  // Tile 0 is not the first one: its copies count as a phase of stage 0 that nobody works on.  Nobody may look at these barriers
+  // before that phase is complete: a wait for the phase behind it would take the parity of the one before it for done, run a phase
+  // ahead of its operands from then on, and leave with copies in flight.  (With no tile at all nobody else looks for Q either:
+  // every copy has landed before the CTA leaves.)
   const uint32_t missed = N == 0 || (s_tile[0] & (MIXED - 1)) != 0;
+  if (missed) {
+    if (warp == 9 && lane == 0 && !(tc5::mbar_wait(&k_full[0], 0) & tc5::mbar_wait(&v_full[0], 0) & tc5::mbar_wait(&q_full, 0))) {
+      failed = 1;
+      atomicExch(&g_tc5_error, 29);
+    }
+    __syncthreads();
+  }
   auto full_parity = [&](int n) { return ((n >> 1) + (n & 1 ? 0 : missed)) & 1; };   // of k_full and v_full
 
   if (warp == 9) {
     if (lane == 0) {   // ---- TMA producer: one instruction per tile (the maps split the head dimension into (64, 2): two panels) ----
       int n = 0;
-      // (with no tile at all nobody else looks for Q: every copy has landed before the CTA leaves)
-      if (missed && !(tc5::mbar_wait(&k_full[0], 0) & tc5::mbar_wait(&v_full[0], 0) & tc5::mbar_wait(&q_full, 0))) { failed = 1; atomicExch(&g_tc5_error, 29); }
       uint32_t masks = 0;   // mixed tiles so far of each buffer, 16 bits each
       for (; n < N; ++n) {
         const int st = n & 1, j = s_tile[n] & (MIXED - 1);

@@ -696,6 +696,41 @@ def test_attn_prefill_many_launches_in_a_row(lib, T):
     assert code.value == 0
 
 
+@pytest.mark.parametrize("lead", [64, 128, 1000, 3000])
+def test_attn_prefill_first_key_tiles_masked_and_keys_far_away(lib, lead):
+    """The first key tile is requested before the mask is known.  Where it is not wanted its copies, from memory that no cache
+    holds, may be the last thing to arrive: nobody may take them for the first tile that is.  Launch after launch over
+    caches that together outgrow the L2: equal to a launch whose operands are at hand, and to float64."""
+    dtype, B, T, S, Hq, Hkv, D, sets = torch.bfloat16, 8, 16, 4096, 12, 2, 128, 5
+    mask = torch.zeros(1, T, S).to(dtype)
+    mask[..., :lead] = torch.finfo(dtype).min
+    Q, M = gen((B, Hq, T, D), dtype).cuda(), mask.cuda()
+    K = [gen((B, Hkv, S, D), dtype, 1 + i).cuda() for i in range(sets)]
+    V = [gen((B, Hkv, S, D), dtype, 9 + i).cuda() for i in range(sets)]
+    tiles = torch.empty(1, 1, S // 128, dtype=torch.uint8, device="cuda")
+    ok(lib, lib.b200_mask_tiles(M.data_ptr(), 1, T, S, 0, S, 2, tiles.data_ptr(), stream()))
+    st = lambda t: (C.c_int64 * 3)(*t.stride()[:3])
+
+    def call(i):
+        out = torch.full((B, T, Hq, D), float("nan"), dtype=dtype, device="cuda")
+        ok(lib, lib.b200_attn_prefill_tiles(Q.data_ptr(), K[i].data_ptr(), V[i].data_ptr(), M.data_ptr(), tiles.data_ptr(), out.data_ptr(), B, Hq, Hkv,
+                                            T, S, D, st(Q), st(K[i]), st(V[i]), 0, S, D ** -0.5, 2, stream()))
+        return out
+
+    cold = [[call(i) for i in range(sets)] for _ in range(8)]
+    for i in range(sets):
+        call(i)
+        warm = call(i)
+        assert all(torch.equal(warm, c[i]) for c in cold)
+        p = ((Q.double() @ K[i][:, :, lead:].double().repeat_interleave(6, 1).transpose(2, 3)) * D ** -0.5).softmax(-1)
+        vd = V[i][:, :, lead:].double().repeat_interleave(6, 1)
+        want, size = (p @ vd).transpose(1, 2), (p @ vd.abs()).transpose(1, 2)
+        assert ((warm.double() - want).abs() <= (size + want.abs()) * 2.0 ** -8 * 1.01 + 1e-5).all()
+    code = C.c_int(0)
+    ok(lib, lib.b200_debug_device_error(C.byref(code), 1))
+    assert code.value == 0
+
+
 @pytest.mark.parametrize("scale", [0.0, -0.07])
 @pytest.mark.parametrize("S", [100, 129, 200, 256])
 @pytest.mark.parametrize("masked", [None, "zero", "causal"])
