@@ -467,9 +467,10 @@ __global__ void __launch_bounds__(128) attn_prefill_kernel(const __grid_constant
       for (int i = 0; i < 4; ++i) {
         const int idx = i * 128 + threadIdx.x, row = idx >> 3, ch = idx & 7;   // 64 rows x 8 chunks of 8 keys
         const int64_t qrow = min(static_cast<int64_t>(blockIdx.x) * 64 + row, p.T - 1);
-        const bool ok = kb + ch * 8 < p.S;   // S is a multiple of 8 here; chunks past the end are never read as valid keys
+        const int64_t left = p.S - kb - ch * 8;       // keys of this chunk; those past the end are not read, and never taken for valid ones
         cp_async16(smk + row * 128 + ((ch ^ (row & 7)) << 4),
-                   ok ? static_cast<const void*>(mask_t + b * p.mask_b + qrow * p.mask_t + kb + ch * 8) : static_cast<const void*>(mask_t), ok ? 16 : 0);
+                   left > 0 ? static_cast<const void*>(mask_t + b * p.mask_b + qrow * p.mask_t + kb + ch * 8) : static_cast<const void*>(mask_t),
+                   left >= 8 ? 16 : left > 0 ? static_cast<int>(left) * 2 : 0);
       }
     }
   };
@@ -807,9 +808,9 @@ extern "C" int b200_attn_prefill_tiles(const void* q, const void* k, const void*
   p.q = q; p.k = k; p.v = v; p.mask = mask; p.out = out; p.B = B; p.T = T; p.S = S; p.Hq = Hq; p.Hkv = Hkv;
   for (int i = 0; i < 3; ++i) { p.qs[i] = q_strides[i]; p.ks[i] = k_strides[i]; p.vs[i] = v_strides[i]; }
   p.tiles = static_cast<const uint8_t*>(tiles); p.mask_b = mask_b; p.mask_t = mask_t; p.scale = scale; p.mask_dtype = dtype;
-  p.mask_staged = (mask && aligned16(mask) && mask_b % 8 == 0 && mask_t % 8 == 0 && S % 8 == 0) ? 1 : 0;   // mask dtype == activation dtype by contract
+  p.mask_staged = (mask && aligned16(mask) && mask_b % 8 == 0 && mask_t % 8 == 0) ? 1 : 0;   // mask dtype == activation dtype by contract
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  if (tc5_enabled()) {   // tcgen05 kernel first; the mma.sync kernel below takes what it cannot (odd strides, other mask types)
+  if (tc5_enabled()) {   // tcgen05 kernel first; the mma.sync kernel below takes up to 64 keys and what that cannot (unaligned mask rows)
     const int rc = attn_prefill_tc5(p, dtype, st);
     if (rc == B200_ELAUNCH) B200_FAIL(B200_ELAUNCH, "attn_prefill_tc5_kernel: launch failed");
     if (rc != B200_ENOTSUP) return rc;

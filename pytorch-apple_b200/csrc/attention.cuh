@@ -20,7 +20,7 @@ struct PrefillParams {
   int mask_staged;   // the mask can travel through shared memory (activation dtype, 16-byte-aligned rows)
 };
 
-// Prefill attention on the tcgen05 path (head_dim 128, 16-bit types, 16-byte aligned strides, at most 32768 keys, mask
+// Prefill attention on the tcgen05 path (head_dim 128, 16-bit types, 16-byte aligned strides, 65 to 32768 keys, mask
 // absent or in the activation type).  Returns B200_ENOTSUP for anything else; the caller then uses the mma.sync kernel.
 int attn_prefill_tc5(const PrefillParams& p, int dtype, cudaStream_t stream);
 // code left by a bounded wait of that kernel that ran out (0 = none); optionally cleared

@@ -29,7 +29,7 @@
 // Bounds: per tile 1024 tensor cycles (16 MMAs of N = 128), 1024 cycles of ex2 per scheduler and 64 KB of K and V into
 // the SM, which are level; short prompts are bound by the chain Q, K -> S -> softmax -> O of their longest row block.
 // us per launch (12 heads over 2 KV heads, causal mask), the 64-key kernel with two threads per
-// row that this one replaced -> this one, in chains of launches: 17 tokens 5.4 -> 5.3, 128 8.8 -> 6.7, 512 18.3 -> 10.2,
+// row that this one replaced -> this one, in chains of launches: 128 tokens 8.8 -> 6.7, 512 18.3 -> 10.2,
 // 777 24.0 -> 13.0, 1024 30.5 -> 15.4, 2048 59.9 -> 26.0 (whole prompts of 512 and 2048 tokens 2930 -> 2680, 8300 -> 7250).
 // Of the 2600 cycles that a tile of a long row block takes, exponentials are 1150 (both groups at once), the scores' way
 // from tensor memory to their maximum 450, barrier waits that find their phase complete 100 to 250 each.
@@ -524,6 +524,10 @@ int attn_prefill_tc5_error(bool clear) {
 
 int attn_prefill_tc5(const PrefillParams& p, int dtype, cudaStream_t stream) {
   if (dtype != B200_BF16 && dtype != B200_F16) return B200_ENOTSUP;
+  // One 64-key tile of the mma.sync kernel: no barriers, tensor memory or 128-key tile to set up for it.  us, 12 heads, here -> there: 16 x 16
+  // 5.5 -> 3.8 (64-key tiles on this path had taken 5.1), 63 x 63 6.1 -> 4.6, 64 x 64 5.8 -> 4.7, 16 sequences of 64 11.2 -> 6.9, 128 x 64 6.5 -> 4.8;
+  // 65 keys, 16 sequences 12.6 -> 12.3, two queries 4.8 -> 5.6; 128 x 128 7.1 -> 6.2, 16 sequences 13.4 -> 14.6.
+  if (p.S <= 64) return B200_ENOTSUP;
   if (p.S > static_cast<int64_t>(BKV) * MAX_TILES || (p.T + BQ - 1) / BQ > 65535 || p.Hq % p.Hkv) return B200_ENOTSUP;
   // The mask's mixed tiles travel by TMA: aligned rows, of any length (the mma.sync kernel's staged copies need lengths that
   // are multiples of eight besides).  777 tokens: 145 us there, 13 here.

@@ -676,6 +676,47 @@ def test_attn_prefill_mask_tiles(lib, kind, B, T, S, rows):
     assert code.value == 0
 
 
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("kind", [None, "causal", "bias", "last"])
+@pytest.mark.parametrize("B,T,S", [(1, 1, 1), (2, 5, 7), (1, 16, 16), (3, 17, 17), (1, 63, 63), (2, 64, 64), (1, 65, 64), (2, 130, 33), (1, 3, 64), (1, 20, 65)])
+def test_attn_prefill_few_keys(lib, B, T, S, kind, dtype):
+    """Up to 64 keys are one tile of the mma.sync kernel, whose mask rows are copied to the last key and no further (what lies
+    behind is no number here).  Bound: probabilities and outputs rounded to the activation type, of what is added up."""
+    Hq, Hkv, D = 4, 2, 128
+    q, k, v = gen((B, Hq, T, D), dtype), gen((B, Hkv, S, D), dtype, 1), gen((B, Hkv, S, D), dtype, 2)
+    mask = torch.zeros(B, T, S).to(dtype)
+    if kind == "last":   # one key each
+        mask[:] = torch.finfo(dtype).min
+        mask[..., S - 1] = 0
+    elif kind:
+        mask = _mask_of(kind, B, T, S, dtype)
+        if kind == "causal" and dtype == torch.float16:
+            # a row of nothing but fp16's lowest value (-65504) keeps its scores to a half unit of fp32 there, 2^-9: half a per cent of each probability
+            mask[:, :max(T - S, 0), 0] = 0
+    s = (q.double() @ k.double().repeat_interleave(Hq // Hkv, 1).transpose(2, 3)) * D ** -0.5 + mask.double()[:, None]
+    p = s.softmax(-1) * ~(mask.double() <= -1e30).all(-1)[:, None, :, None]
+    vd = v.double().repeat_interleave(Hq // Hkv, 1)
+    want, size = (p @ vd).transpose(1, 2), (p @ vd.abs()).transpose(1, 2)
+    pitch = -(-S // 8) * 8
+    M = torch.full((B, T, pitch), float("nan"), dtype=dtype, device="cuda")
+    M[..., :S] = mask.cuda()
+    Q, K, V = q.cuda(), k.cuda(), v.cuda()
+    st = lambda t: (C.c_int64 * 3)(*t.stride()[:3])
+    out = torch.empty((B, T, Hq, D), dtype=dtype, device="cuda")
+    names = []
+    for _ in range(3):   # (a profiling session now and then reports nothing)
+        out.fill_(float("nan"))
+        with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CUDA]) as prof:
+            ok(lib, lib.b200_attn_prefill(Q.data_ptr(), K.data_ptr(), V.data_ptr(), M.data_ptr() if kind else None, out.data_ptr(), B, Hq, Hkv, T, S, D, st(Q), st(K), st(V),
+                                          T * pitch, pitch, D ** -0.5, DT[dtype], stream()))
+            torch.cuda.synchronize()
+        names = names or [e.key for e in prof.key_averages() if "attn_prefill" in e.key]
+    assert len(names) == 1 and ("tc5" in names[0]) == (S > 64), names
+    eps = 2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -11
+    err = (out.double().cpu() - want).abs()
+    assert (err <= (size + want.abs()) * eps * 1.01 + 1e-5).all(), float(err.max())
+
+
 @pytest.mark.parametrize("T", [128, 400])
 def test_attn_prefill_many_launches_in_a_row(lib, T):
     """The first key tile is requested before it is known to be wanted, so its scores may be complete before the producer
@@ -732,7 +773,7 @@ def test_attn_prefill_first_key_tiles_masked_and_keys_far_away(lib, lead):
 
 
 @pytest.mark.parametrize("scale", [0.0, -0.07])
-@pytest.mark.parametrize("S", [100, 129, 200, 256])
+@pytest.mark.parametrize("S", [60, 100, 129, 200, 256])
 @pytest.mark.parametrize("masked", [None, "zero", "causal"])
 def test_attn_prefill_scales_that_are_not_positive(lib, masked, S, scale):
     """Scale 0 weighs all keys alike and a negative one turns their order round, also where the last key tile, or half of it,
