@@ -414,6 +414,9 @@ int b200_attn_prefill_tiles(const void* q, const void* k, const void* v, const v
  * 0 no element above -1e30, 1 all elements zero, 2 anything else. */
 int b200_mask_tiles(const void* mask, int64_t B, int64_t T, int64_t S, int64_t mask_b, int64_t mask_t, int dtype,
                     void* tiles, void* stream);
+/* 1 where b200_attn_prefill_tiles reads the states of such a mask, 0 where the kernel that takes the call has no use for them
+ * (few or very many keys, rows that are not 16-byte aligned): looking for them would be a launch for nothing. */
+int b200_attn_prefill_reads_tiles(const void* mask, int64_t S, int64_t mask_b, int64_t mask_t, int dtype);
 
 #ifdef __cplusplus
 }

@@ -42,6 +42,7 @@
 // barrier wait is bounded; on a time-out the CTA records a code in the library's device error
 // word, stops issuing, frees its tensor memory and returns.
 #include "attention.cuh"
+#include "gemm_tc5.cuh"
 #include "tc5.cuh"
 
 namespace b200 {
@@ -522,16 +523,20 @@ int attn_prefill_tc5_error(bool clear) {
   return v;
 }
 
+// Keys and masks that this kernel takes.
+// One 64-key tile of the mma.sync kernel: no barriers, tensor memory or 128-key tile to set up for it.  us, 12 heads, here -> there: 16 x 16
+// 5.5 -> 3.8 (64-key tiles on this path had taken 5.1), 63 x 63 6.1 -> 4.6, 64 x 64 5.8 -> 4.7, 16 sequences of 64 11.2 -> 6.9, 128 x 64 6.5 -> 4.8;
+// 65 keys, 16 sequences 12.6 -> 12.3, two queries 4.8 -> 5.6; 128 x 128 7.1 -> 6.2, 16 sequences 13.4 -> 14.6.
+static bool keys_fit(int64_t S) { return S > 64 && S <= static_cast<int64_t>(BKV) * MAX_TILES; }
+// The mask's mixed tiles travel by TMA: aligned rows, of any length.
+static bool mask_fits(const void* mask, int mask_dtype, int64_t S, int64_t mask_b, int64_t mask_t, int dtype) {
+  return mask_dtype == dtype && aligned16(mask) && mask_b % 8 == 0 && mask_b >= 0 && mask_t >= S && mask_t % 8 == 0;
+}
+
 int attn_prefill_tc5(const PrefillParams& p, int dtype, cudaStream_t stream) {
   if (dtype != B200_BF16 && dtype != B200_F16) return B200_ENOTSUP;
-  // One 64-key tile of the mma.sync kernel: no barriers, tensor memory or 128-key tile to set up for it.  us, 12 heads, here -> there: 16 x 16
-  // 5.5 -> 3.8 (64-key tiles on this path had taken 5.1), 63 x 63 6.1 -> 4.6, 64 x 64 5.8 -> 4.7, 16 sequences of 64 11.2 -> 6.9, 128 x 64 6.5 -> 4.8;
-  // 65 keys, 16 sequences 12.6 -> 12.3, two queries 4.8 -> 5.6; 128 x 128 7.1 -> 6.2, 16 sequences 13.4 -> 14.6.
-  if (p.S <= 64) return B200_ENOTSUP;
-  if (p.S > static_cast<int64_t>(BKV) * MAX_TILES || (p.T + BQ - 1) / BQ > 65535 || p.Hq % p.Hkv) return B200_ENOTSUP;
-  // The mask's mixed tiles travel by TMA: aligned rows, of any length (the mma.sync kernel's staged copies need lengths that
-  // are multiples of eight besides).  777 tokens: 145 us there, 13 here.
-  if (p.mask && (p.mask_dtype != dtype || !aligned16(p.mask) || p.mask_b % 8 || p.mask_b < 0 || p.mask_t < p.S || p.mask_t % 8)) return B200_ENOTSUP;
+  if (!keys_fit(p.S) || (p.T + BQ - 1) / BQ > 65535 || p.Hq % p.Hkv) return B200_ENOTSUP;
+  if (p.mask && !mask_fits(p.mask, p.mask_dtype, p.S, p.mask_b, p.mask_t, dtype)) return B200_ENOTSUP;
   // TMA: 16-byte aligned bases (checked by the caller) and strides that are multiples of 16 bytes
   for (int i = 0; i < 3; ++i)
     if (p.qs[i] % 8 || p.ks[i] % 8 || p.vs[i] % 8 || p.qs[i] < 0 || p.ks[i] < 0 || p.vs[i] < 0) return B200_ENOTSUP;
@@ -554,4 +559,8 @@ extern "C" int b200_mask_tiles(const void* mask, int64_t B, int64_t T, int64_t S
   });
   B200_CHECK_LAUNCH("mask_tiles_kernel");
   return B200_OK;
+}
+
+extern "C" int b200_attn_prefill_reads_tiles(const void* mask, int64_t S, int64_t mask_b, int64_t mask_t, int dtype) {
+  return tc5_enabled() && mask && (dtype == B200_BF16 || dtype == B200_F16) && keys_fit(S) && mask_fits(mask, dtype, S, mask_b, mask_t, dtype) ? 1 : 0;
 }

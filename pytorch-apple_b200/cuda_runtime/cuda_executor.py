@@ -733,6 +733,8 @@ class CUDAExecutor:
         if m is None:
             return None
         key = _mask_key(m)
+        if not self._lib.b200_attn_prefill_reads_tiles(self._ptr(m), key[4], m.strides[0], m.strides[2], DTYPE_CODES[m.dtype]):
+            return None
         tiles = self._tiles[key].data_ptr()
         if key not in plan.masks_seen:
             plan.masks_seen.add(key)

@@ -83,6 +83,7 @@ SIGNATURES = {
     "b200_attn_decode_noalloc": (_i, [_vp, _vp, _vp, _vp, _vp, _i64, _i, _i, _i64, _i, _i64, _i64, _i64, _i64, _f, _i, _vp]),
     "b200_attn_decode_workspace_bytes": (_i64, [_i64, _i, _i, _i64, _i]),
     "b200_attn_prefill_tiles": (_i, [_vp, _vp, _vp, _vp, _vp, _vp, _i64, _i, _i, _i64, _i64, _i, _I64P, _I64P, _I64P, _i64, _i64, _f, _i, _vp]),
+    "b200_attn_prefill_reads_tiles": (_i, [_vp, _i64, _i64, _i64, _i]),
     "b200_mask_tiles": (_i, [_vp, _i64, _i64, _i64, _i64, _i64, _i, _vp, _vp]),
     "b200_attn_prefill": (_i, [_vp, _vp, _vp, _vp, _vp, _i64, _i, _i, _i64, _i64, _i, _I64P, _I64P, _I64P, _i64, _i64, _f, _i, _vp]),
 }

@@ -285,7 +285,7 @@ def test_qwen_tiny_golden_prefill_then_decode(fake_native):
     assert fake_native.calls.count("attn_decode") == L and fake_native.calls.count("attn_prefill") == L
 
 
-@pytest.mark.parametrize("B,T", [(1, 13), (2, 9), (1, 16)])
+@pytest.mark.parametrize("B,T", [(1, 13), (2, 9), (1, 16), (1, 64), (1, 65), (2, 130)])
 def test_prefill_mask_rows_are_aligned_once_per_call(fake_native, B, T):
     """A prompt whose length is no multiple of eight: one copy of the mask with padded rows, read by every layer;
     an aligned mask is read in place."""
@@ -302,6 +302,7 @@ def test_prefill_mask_rows_are_aligned_once_per_call(fake_native, B, T):
     assert np.abs(to_f32(out[name]) - ref.float().numpy()).max() < 0.1
     copies = [st for st in compile_subgraph(ir).steps if getattr(st, "kernel_name", "") == "strided_copy"]
     assert len(copies) == (0 if T % 8 == 0 else 1)
+    assert fake_native.calls.count("mask_tiles") == (1 if T > 64 else 0)   # for all layers, and where the attention reads the states
     assert fake_native.calls.count("attn_prefill") == cfg.num_hidden_layers
 
 
