@@ -1611,18 +1611,21 @@ int launch_persistent(const Tc5Args& a, cudaStream_t st, const Tc5Conv* g = null
 }
 
 // The CTA-pair kernel takes a linear layer when its tiles (256 columns x up to 256 rows) give at least half of the 74 pairs a tile
-// (even half empty it beats 128-wide tiles on every SM; with one tile of rows from 65 on: gate/up of 128 rows 16.1 -> 13.9 us,
-// of 65 rows 15.0 -> 14.7, vocabulary 92 -> 86) and the reduction is long enough to hide the plain epilogue.
+// (even half empty it beats 128-wide tiles on every SM) and the reduction is long enough to hide the plain epilogue.
+// With one tile of up to 128 rows it does so where the one-tile kernel's 64-wide tiles need a second wave (us, one-tile kernel -> pairs;
+// K = 1536: 65 x 10240 13.4 -> 12.1, 128 x 17920 gated 16.2 -> 13.9; K = 4096: 65 x 10240 30.2 -> 23.6; 100 x 151936 97 -> 89) and not where they
+// are all resident (9472 columns are 148 of them: 65 rows 10.4 -> 11.5, 128 rows 12.1 -> 12.5, K = 4096 20.0 -> 22.5).
 bool pair_shape(const Tc5Args& a) {
   // (N >= 1024: a tall activation matrix against one or two column tiles - the 1x1 convolutions 1024 -> 256 / 512
   // over 50176 pixels - measured slower here than with the bulk-copy epilogue of the persistent kernel)
   if (a.M <= 64 || a.N < 1024 || a.K < 1024) return false;
+  if (a.M <= 128 && ceil_div(a.N, 64) <= sm_count()) return false;
   return ceil_div(a.M, 256) * ceil_div(a.N, 256) >= 37;
 }
 
 // Few tiles but a long reduction (the down projection of a 512- or 1024-token prompt: 12 or 24 tiles, K = 8960): the
 // pairs split K among themselves and leave fp32 partial sums in the caller's workspace; measured 21.8 us (512 rows)
-// and 30.7 us (1024) against 33.9 and 70.5 us for 128 x 128 tiles with split-K inside a cluster.  Returns the split
+// and 29.0 us (1024) against 33.9 and 70.5 us for 128 x 128 tiles with split-K inside a cluster.  Returns the split
 // count (1: none).
 int pair_splits(int64_t M, int64_t N, int64_t K) {
   if (M <= 128 || N < 256 || K < 4096 || N % 8) return 1;

@@ -263,6 +263,8 @@ def test_linear_few_rows_edges(lib, M, N, K, shift, ldx, dtype):
     (16, 17920, 1536, False, "gemm_stream_kernel"), (17, 17920, 1536, False, "gemm_tc5_kernel"), (8, 200, 328, False, "gemm_tc5_kernel"),
     (777, 2048, 1536, False, "gemm_tc5_kernel"), (777, 1536, 1536, True, "gemm_tc5p_kernel"), (777, 1500, 1536, True, "gemm_tc5_kernel"),
     (2048, 1536, 1536, True, "gemm_pair_kernel"),
+    (65, 9472, 1536, False, "gemm_tc5_kernel"), (128, 9472, 1536, False, "gemm_tc5_kernel"), (129, 9472, 1536, False, "gemm_pair_kernel"),
+    (65, 9480, 1536, False, "gemm_pair_kernel"), (128, 17920, 1536, False, "gemm_pair_kernel"), (64, 17920, 1536, False, "gemm_tc5_kernel"),
 ])
 def test_linear_runs_on_the_kernel_that_its_shape_calls_for(lib, M, N, K, res, kernel):
     t = torch.zeros(M * K + N * K + 2 * M * N, dtype=torch.bfloat16, device="cuda")
