@@ -71,9 +71,10 @@ constexpr int DEC_ACC_PITCH = HD + 4;          // row pitch of the cross-warp ac
 // heads it owns (head h belongs to rank h % splits) and writes the final output.  2 <= splits <= 16.
 //
 // NW = 8 warps instead of 4, one CTA per SM, where all clusters are resident even so (up to three sequences) and a split has
-// more than four blocks: what a warp does with its blocks one after the other is then half as long.  us, one sequence: 4097 keys
-// 7.7 -> 6.3, 8000 keys 9.9 -> 7.2, 16000 keys 16.8 -> 11.0, 1111 keys (80 per split) 4.6 -> 4.3, 790 keys (64 per split) would
-// lose, 3.9 -> 4.2; three sequences of 4097 8.3 -> 7.4.  With a second wave of clusters it loses (four: 13.6), and a third ring
+// more than six blocks, with one or two clusters more than four: what a warp does with its blocks one after the other is then half as long.
+// us, one sequence: 4097 keys 7.7 -> 6.3, 8000 keys 9.9 -> 7.2, 16000 keys 16.8 -> 11.0, 1111 keys (80 per split) 4.7 -> 4.5, 790 keys (64
+// per split) would lose, 3.9 -> 4.2; three sequences of 4352 8.3 -> 7.4, of 1800 (128 per split) 5.5 -> 5.5; two of 1800 5.0 -> 4.8, of 1300 (96
+// per split, an eighth filled) would lose, 4.5 -> 4.7.  With a second wave of clusters it loses (four: 13.6), and a third ring
 // stage for four warps gains nothing (7.8, 8.6): this is not the memory's latency.
 template <typename T, int STAGES, bool CM, int NW = 4>
 __global__ void __launch_bounds__(NW * 32, NW == 8 ? 1 : STAGES == 2 ? 3 : 2) attn_decode_kernel(const __grid_constant__ DecodeParams p) {
@@ -721,7 +722,7 @@ extern "C" int b200_attn_decode(const void* q, const void* k, const void* v, con
     cudaGetLastError();
   }
   const DecodePlan d = plan_decode(B, Hkv, S, Hq / Hkv, resident16->n4);
-  const bool eight_warps = d.cluster && d.splits > 8 && d.split_len > 64 && B * Hkv <= resident16->n8;
+  const bool eight_warps = d.cluster && d.splits > 8 && d.split_len > (B * Hkv <= 2 ? 64 : 96) && B * Hkv <= resident16->n8;
   const int64_t need = b200_attn_decode_workspace_bytes(B, Hq, Hkv, S, D);
   if (need > 0 && (!workspace || workspace_bytes < need))
     B200_FAIL(B200_EINVAL, "b200_attn_decode: workspace of %lld bytes required (got %lld)", (long long)need, (long long)workspace_bytes);

@@ -470,9 +470,9 @@ def test_attn_decode_small_batches_in_both_dtypes(lib, dtype, B):
 
 @pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
 @pytest.mark.parametrize("Hq,Hkv", [(12, 2), (7, 7), (8, 1)])
-@pytest.mark.parametrize("B,S", [(1, 1024), (1, 1040), (3, 1111), (1, 4352), (4, 2048), (1, 16383)])
+@pytest.mark.parametrize("B,S", [(1, 1024), (1, 1040), (3, 1111), (3, 1536), (3, 1800), (1, 4352), (4, 2048), (1, 16383)])
 def test_attn_decode_eight_warps(lib, dtype, Hq, Hkv, B, S):
-    """Few sequences with more than 64 keys per split take eight warps per CTA: on both sides of that line and of the number
+    """Few sequences with more than 64 or 96 keys per split take eight warps per CTA: on both sides of that line and of the number
     of clusters that fit, masks with a filled prefix, with holes, with one key; against float64 within the rounding
     of probabilities and outputs (2^-8 of what is added up in bf16, 2^-11 in fp16; fp32 elsewhere)."""
     D, neg = 128, torch.finfo(dtype).min
