@@ -7,18 +7,22 @@
 //
 // NT is any multiple of 16 up to 256, so that a prompt is cut into equal tiles instead of leaving the last one mostly empty: 777 rows are four
 // tiles of 208 (256-row tiles: 1024 rows), 128 rows one of 128.  Accumulator rows are output columns and accumulator columns tokens: the epilogue
-// turns 32 tokens at a time round in shared memory and writes (and reads residuals of) whole 16-byte words of a token's row.
+// turns 32 tokens at a time round in shared memory, a word for two tokens of a column, and writes (and reads residuals of) whole 16-byte words of a
+// token's row; where rows are no such words a warp writes 32 columns of a token straight from its registers.
 // Few tiles but a long reduction: the pairs split K (units of (tile, split)) and leave fp32 partial sums in p.partial, which a
 // second kernel adds up.
 //
 // Bound by what an SM can take in (32 KB per k-block and CTA at 256 tokens: ~78 KB per us) and, before a ring stage held two k-blocks, by
 // the issuing thread (a barrier probe and a commit per k-block: 0.41 us whatever NT).  us, 256 x 256 tiles with tokens on the 256-row side and a k-block
-// per stage -> this (gate/up 17920 x 1536, down 1536 x 8960 with its reduce kernel, vocabulary 151936 x 1536):
-//    128 rows  gate/up 16.1 -> 13.9 (one-tile kernel there), vocabulary 96 -> 91;   256 rows 15.8 -> 16.6, 109 -> 106
-//    512 rows  25.0 -> 24.6   down 22.2 -> 21.9   192 -> 185;    777 rows 43.2 -> 38.4   31.0 -> 25.4   339 -> 303
-//   2048 rows  86.5 -> 79.7        72.8 -> 66.4   679 -> 637 (1.50 PFLOP/s, 0.90 of the cuBLAS burst)
-// Measured and not used: two producer threads per operand (the epilogue then has 128 registers; with 168 it requests the next 32 tokens
-// while it finishes 32: 2048 rows gate/up 88.3 -> 79.7), partial sums without that (down of 512 rows 24.9).
+// per stage -> this, weights from memory (gate/up 17920 x 1536, down 1536 x 8960 with its reduce kernel, vocabulary 151936 x 1536):
+//     65 rows  gate/up 15.1 -> 12.8, 128 rows 16.1 -> 13.4 (one-tile kernel there), vocabulary 96 -> 91;   256 rows 16.3 -> 16.1, 134 -> 128
+//    512 rows  26.2 -> 24.8   down 22.2 -> 21.9   192 -> 185;    777 rows 45.1 -> 38.6   29.4 -> 25.1   339 -> 303
+//   2048 rows  86.5 -> 79.7        60.0 -> 53.2   679 -> 637 (1.50 PFLOP/s, 0.90 of the cuBLAS burst)
+//   256 x 12288 x 1536 plain 17.3 -> 15.4, with a residual 18.8 -> 15.9; 2048 x 12288 69.6 -> 61.6, 88 -> 68; 512 x 9999 81 -> 25, 91 -> 38
+// By single tokens and through fp32 the epilogue cost more than it saved in one wave of 256-token tiles (gate/up of 256 rows 16.9, 256 x 9352 x 1536
+// with a residual 15.7 -> 17.8, here 14.9).  Measured and not used: two producer threads per operand (the epilogue then has 128 registers; with
+// 168 it requests the next 32 tokens while it finishes 32: 2048 rows gate/up 88.3 -> 79.7), partial sums without that (down of 512 rows 24.9), staging
+// the next 32 tokens before the 32 in shared memory are finished (plain epilogues 1 to 2 % slower, gated ones level).
 #include "gemm_epilogue.cuh"
 #include "tc5.cuh"
 
@@ -35,7 +39,16 @@ constexpr int PR_W = 128 * 128, PR_KB = 2 * PR_W, PR_STAGE = PR_KPS * PR_KB;   /
 constexpr int PR_CHUNK = 32, PR_BUF = PR_CHUNK * 128 * 2;        // 32 tokens x 128 output columns, 16-bit
 constexpr int PR_SMEM = PR_ST * PR_STAGE + 4 * PR_BUF + 1024;
 
-template <typename T>
+// What a tile's results become: one kernel each, since a launch is a few tiles long and fetches its epilogue's code while it runs (gate/up of 65
+// rows: 13.0 us, with the code of the other forms between 13.5)
+enum class PairForm {
+  SPLIT,   // fp32 partial sums
+  GATED,   // silu(gate) * up
+  WORDS,   // bias, residual, ReLU, silu(.) * aux; rows of whole 16-byte words
+  ANY      // the same, any rows
+};
+
+template <typename T, PairForm FORM>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PR_THREADS, 1)
     gemm_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_w, const __grid_constant__ Tc5Params p, const int nt,
                      const int tiles_t, const int n_tiles) {
@@ -135,9 +148,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PR_THREADS, 1)
     const int q = warp & 3, g = warp >= 7 ? 1 : 0, t = q * 32 + lane;   // t: accumulator row, output column of the block
     uint8_t* const buf = smem + PR_ST * PR_STAGE + g * 2 * PR_BUF;
     pdl_wait();
-    const bool glu = (p.epilogue & B200_EPI_GLU) != 0, silu = (p.epilogue & B200_EPI_SILU_MUL) != 0, relu = (p.epilogue & B200_EPI_RELU) != 0;
+    const bool silu = (p.epilogue & B200_EPI_SILU_MUL) != 0, relu = (p.epilogue & B200_EPI_RELU) != 0;
     const T* const res = static_cast<const T*>(p.residual);
-    const bool res_vec = res && p.ldr % 8 == 0 && p.N % 8 == 0 && (reinterpret_cast<uintptr_t>(res) & 15u) == 0;
     const uint32_t lead_acc_empty0 = tc5::map_to_rank(tc5::smem_addr(&acc_empty[0]), 0);
     // the group's four warps leave together: they meet at a barrier of their own
     auto any = [&](bool v) {
@@ -149,12 +161,12 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PR_THREADS, 1)
     for (int unit = pair; unit < n_units; unit += n_pairs, ++ti) {
       const int b = ti & 1, tile = unit % n_tiles;
       const int64_t n0 = static_cast<int64_t>(tile / tiles_t) * 256 + rank * 128, m0 = static_cast<int64_t>(tile % tiles_t) * nt;   // of this CTA
-      const float bias = p.bias && p.splits == 1 && n0 + t < p.N ? load_as_f32(p.bias, n0 + t, p.bias_dtype) : 0.f;
+      const float bias = FORM != PairForm::SPLIT && p.bias && n0 + t < p.N ? load_as_f32(p.bias, n0 + t, p.bias_dtype) : 0.f;
       const bool ok = tc5::mbar_wait(&acc_full[b], (ti >> 1) & 1);
       if (any(!ok || dead())) { if (!ok) fail(43); break; }
       tc5::tc_fence_after();
       const uint32_t t_row = tmem_base + b * 256 + (static_cast<uint32_t>(q * 32) << 16);
-      if (p.splits > 1) {
+      if constexpr (FORM == PairForm::SPLIT) {
         // raw partial sums of this unit's k-range, 32 tokens in flight while 32 are stored: a warp writes 128 consecutive bytes per token
         float* dst = p.partial + (static_cast<int64_t>(unit / n_tiles) * p.M + m0 + PR_CHUNK * g) * p.N + n0 + t;
         const int tokens = n0 + t < p.N ? static_cast<int>(p.M - m0 < nt ? p.M - m0 : nt) : 0;
@@ -187,68 +199,126 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PR_THREADS, 1)
         for (int c = PR_CHUNK * g; c < nt; c += 2 * PR_CHUNK) {
           const int cnt = nt - c < PR_CHUNK ? nt - c : PR_CHUNK;
           const int tokens = static_cast<int>(p.M - m0 - c < cnt ? (p.M - m0 - c < 0 ? 0 : p.M - m0 - c) : cnt);   // that exist
-          // 16-byte words of the result that this thread finishes: token i / 16, columns 8 (i % 16) .. (gated: i / 8, i % 8); residual requested now
+          if constexpr (FORM == PairForm::ANY) {   // a warp writes (and reads) 32 consecutive columns of a token, the reads of a chunk in flight together
+            const int64_t n = n0 + t;
+            auto there = [&](int j) { return j < tokens && n < p.N; };
+            auto column = [&](const void* base, int64_t ld, T (&x)[PR_CHUNK]) {
+#pragma unroll
+              for (int j = 0; j < PR_CHUNK; ++j) x[j] = there(j) ? static_cast<const T*>(base)[(m0 + c + j) * ld + n] : from_f32<T>(0.f);
+            };
+            T x[PR_CHUNK];
+            if (res) column(res, p.ldr, x);
+            tc5::tmem_ld_wait();
+#pragma unroll
+            for (int j = 0; j < PR_CHUNK; ++j) v[j] += bias;
+            if (res) {
+#pragma unroll
+              for (int j = 0; j < PR_CHUNK; ++j) v[j] = round_as<T>(v[j]) + to_f32<T>(x[j]);
+            }
+            if (relu) {
+#pragma unroll
+              for (int j = 0; j < PR_CHUNK; ++j) v[j] = fmaxf(v[j], 0.f);
+            }
+            if (silu) {
+              column(p.aux, p.ldaux, x);
+#pragma unroll
+              for (int j = 0; j < PR_CHUNK; ++j) v[j] = round_as<T>(silu_f32(round_as<T>(v[j]))) * to_f32<T>(x[j]);
+            }
+#pragma unroll
+            for (int j = 0; j < PR_CHUNK; ++j)
+              if (there(j)) static_cast<T*>(p.out)[(m0 + c + j) * p.ldo + n] = from_f32<T>(v[j]);
+            __syncwarp();
+            if (c + 2 * PR_CHUNK < nt) tc5::tmem_ld_32x32_async(t_row + c + 2 * PR_CHUNK, v);
+            continue;
+          }
+          // 16-byte words of the result that this thread finishes: two items of two tokens 2 (i / 16) .. and columns 8 (i % 16) ..; residual requested now
           uint4 r[4];
-          if (res_vec) {
+          if (FORM == PairForm::WORDS && res) {
 #pragma unroll
             for (int k = 0; k < 4; ++k) {
-              const int i = t + 128 * k, j = i >> 4;
+              const int i = t + 128 * (k >> 1), j = 2 * (i >> 4) + (k & 1);
               const int64_t n = n0 + 8 * (i & 15);
               r[k] = j < tokens && n < p.N ? __ldg(reinterpret_cast<const uint4*>(res + (m0 + c + j) * p.ldr + n)) : make_uint4(0u, 0u, 0u, 0u);
             }
           }
-          T* const turn = reinterpret_cast<T*>(buf + (round & 1) * PR_BUF);
+          // [pair of tokens][column], a word each: half the stores of single values, and no two of a warp in one bank
+          uint32_t* const pairs = reinterpret_cast<uint32_t*>(buf + (round & 1) * PR_BUF);
           ++round;
           tc5::tmem_ld_wait();
 #pragma unroll
-          for (int j = 0; j < PR_CHUNK; ++j) turn[j * 128 + t] = from_f32<T>(v[j] + bias);
+          for (int j = 0; j < PR_CHUNK; j += 2) pairs[(j >> 1) * 128 + t] = pack2<T>(v[j] + bias, v[j + 1] + bias);
           if (c + 2 * PR_CHUNK < nt) tc5::tmem_ld_32x32_async(t_row + c + 2 * PR_CHUNK, v);   // the next 32 tokens, while these are finished
           // (two buffers: whoever writes one again has passed the barrier behind which everybody had read it)
           asm volatile("bar.sync %0, 128;" ::"r"(1 + g) : "memory");
-          if (glu) {
+          const int turned = (t >> 2) & 1;   // half of the threads take their words in the other order: no bank twice
+          if constexpr (FORM == PairForm::GATED) {
+            const int j = 2 * (t >> 3), cc = 8 * (t & 7);
+            if (j < tokens && n0 < p.N) {   // (N is a multiple of 128: the block is whole)
+              uint32_t lo[2][2], hi[2][2];   // of the first and the second token: four columns at a time
 #pragma unroll
-            for (int k = 0; k < 2; ++k) {
-              const int i = t + 128 * k, j = i >> 3, cc = 8 * (i & 7);
-              if (j < tokens && n0 < p.N) {   // (N is a multiple of 128: the block is whole)
-                float gt[8], up[8];
-                unpack8<T>(*reinterpret_cast<const uint4*>(turn + j * 128 + cc), gt);
-                unpack8<T>(*reinterpret_cast<const uint4*>(turn + j * 128 + 64 + cc), up);
+              for (int k = 0; k < 2; ++k) {
+                const uint32_t* src = pairs + (j >> 1) * 128 + cc + 4 * (k ^ turned);
+                const uint4 gw = *reinterpret_cast<const uint4*>(src), uw = *reinterpret_cast<const uint4*>(src + 64);
+                const uint32_t gv[4] = {gw.x, gw.y, gw.z, gw.w}, uv[4] = {uw.x, uw.y, uw.z, uw.w};
+                float f0[4], f1[4];
 #pragma unroll
-                for (int e = 0; e < 8; e += 2) {
-                  float a = silu_f32(gt[e]), d = silu_f32(gt[e + 1]);
+                for (int e = 0; e < 4; ++e) {
+                  float a, d, x, y;
+                  unpack2<T>(gv[e], a, d);
+                  unpack2<T>(uv[e], x, y);
+                  a = silu_f32(a); d = silu_f32(d);
                   round2<T>(a, d);
-                  gt[e] = a * up[e]; gt[e + 1] = d * up[e + 1];
+                  f0[e] = a * x; f1[e] = d * y;
                 }
-                store_cols<T, 8>(static_cast<T*>(p.out) + (m0 + c + j) * p.ldo + n0 / 2 + cc, gt, 8);
+                lo[k][0] = pack2<T>(f0[0], f0[1]); lo[k][1] = pack2<T>(f0[2], f0[3]);
+                hi[k][0] = pack2<T>(f1[0], f1[1]); hi[k][1] = pack2<T>(f1[2], f1[3]);
               }
+              T* const dst = static_cast<T*>(p.out) + (m0 + c + j) * p.ldo + n0 / 2 + cc;
+              auto put = [&](T* d, const uint32_t (&w)[2][2]) {
+                const uint4 o = turned ? make_uint4(w[1][0], w[1][1], w[0][0], w[0][1]) : make_uint4(w[0][0], w[0][1], w[1][0], w[1][1]);
+                float f[8];
+                if (p.ldo % 8 == 0 && (reinterpret_cast<uintptr_t>(p.out) & 15u) == 0) { *reinterpret_cast<uint4*>(d) = o; return; }
+                unpack8<T>(o, f);
+                store_cols<T, 8>(d, f, 8);
+              };
+              put(dst, lo);
+              if (j + 1 < tokens) put(dst + p.ldo, hi);
             }
           } else {
 #pragma unroll
-            for (int k = 0; k < 4; ++k) {
-              const int i = t + 128 * k, j = i >> 4;
-              const int64_t n = n0 + 8 * (i & 15), m = m0 + c + j;
+            for (int k = 0; k < 2; ++k) {
+              const int i = t + 128 * k, j = 2 * (i >> 4);
+              const int64_t n = n0 + 8 * (i & 15);
               if (j >= tokens || n >= p.N) continue;
-              const int left = static_cast<int>(p.N - n < 8 ? p.N - n : 8);
-              float f[8];
-              unpack8<T>(*reinterpret_cast<const uint4*>(turn + j * 128 + 8 * (i & 15)), f);
-              if (res) {
-                float rf[8];
-                if (res_vec) unpack8<T>(r[k], rf);
-                else load_cols<T, 8>(res, p.ldr, m, n, left, rf);
+              const uint32_t* src = pairs + (j >> 1) * 128 + 8 * (i & 15);
+              const uint4 w0 = *reinterpret_cast<const uint4*>(src + 4 * turned), w1 = *reinterpret_cast<const uint4*>(src + 4 * (turned ^ 1));
+              const uint4 a = turned ? w1 : w0, d = turned ? w0 : w1;
 #pragma unroll
-                for (int e = 0; e < 8; ++e) f[e] += rf[e];
-              }
-              if (relu) {
+              for (int e = 0; e < 2; ++e) {   // the first and the second token
+                if (j + e >= tokens) continue;
+                const int64_t m = m0 + c + j + e;
+                const uint32_t half = e ? 0x7632u : 0x5410u;
+                uint32_t o[4] = {__byte_perm(a.x, a.y, half), __byte_perm(a.z, a.w, half), __byte_perm(d.x, d.y, half), __byte_perm(d.z, d.w, half)};
+                T* const dst = static_cast<T*>(p.out) + m * p.ldo + n;
+                const uint32_t rv[4] = {r[2 * k + e].x, r[2 * k + e].y, r[2 * k + e].z, r[2 * k + e].w};
 #pragma unroll
-                for (int e = 0; e < 8; ++e) f[e] = fmaxf(f[e], 0.f);
-              }
-              if (silu) {
-                float x[8];
-                load_cols<T, 8>(static_cast<const T*>(p.aux), p.ldaux, m, n, left, x);
+                for (int q = 0; q < 4; ++q) {
+                  if (res) o[q] = add2<T>(o[q], rv[q]);   // (the exact sum of two 16-bit numbers rounded once: what an fp32 addition and its rounding give)
+                  if (relu) o[q] = relu2<T>(o[q]);
+                }
+                if (silu) {
+                  float f[8], x[8];
+                  unpack8<T>(make_uint4(o[0], o[1], o[2], o[3]), f);
+                  unpack8<T>(__ldg(reinterpret_cast<const uint4*>(static_cast<const T*>(p.aux) + m * p.ldaux + n)), x);
 #pragma unroll
-                for (int e = 0; e < 8; ++e) f[e] = round_as<T>(silu_f32(round_as<T>(f[e]))) * x[e];
+                  for (int q = 0; q < 8; q += 2) {
+                    float y0 = silu_f32(f[q]), y1 = silu_f32(f[q + 1]);
+                    round2<T>(y0, y1);
+                    o[q >> 1] = pack2<T>(y0 * x[q], y1 * x[q + 1]);
+                  }
+                }
+                *reinterpret_cast<uint4*>(dst) = make_uint4(o[0], o[1], o[2], o[3]);
               }
-              store_cols<T, 8>(static_cast<T*>(p.out) + m * p.ldo + n, f, left);
             }
           }
           __syncwarp();
@@ -265,12 +335,12 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PR_THREADS, 1)
   if (warp == 1) { tc5::tc_fence_after(); tc5::tmem_dealloc_pair(tmem_base, 512); }
 }
 
-template <typename T> int launch_pair_t(const Tc5Args& a, Tc5Params p, cudaStream_t st) {
+template <typename T, PairForm FORM> int launch_pair_t(const Tc5Args& a, Tc5Params p, cudaStream_t st) {
   static PerDevice<bool> configured_on;
   bool* configured = configured_on.slot();
   if (!configured) return B200_ENOTSUP;
   if (!*configured) {
-    if (cudaFuncSetAttribute(gemm_pair_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, PR_SMEM) != cudaSuccess) {
+    if (cudaFuncSetAttribute(gemm_pair_kernel<T, FORM>, cudaFuncAttributeMaxDynamicSharedMemorySize, PR_SMEM) != cudaSuccess) {
       cudaGetLastError();
       return B200_ENOTSUP;
     }
@@ -288,15 +358,23 @@ template <typename T> int launch_pair_t(const Tc5Args& a, Tc5Params p, cudaStrea
   CUtensorMap mx, mw;
   if (!map(&mx, a.A, a.M, a.lda, nt / 2) || !map(&mw, a.W, a.N, a.ldw, 128)) return B200_ENOTSUP;
   const int pairs = static_cast<int>(units < sm_count() / 2 ? units : sm_count() / 2);
-  launch_pdl(gemm_pair_kernel<T>, dim3(2 * pairs), dim3(PR_THREADS), PR_SMEM, st, mx, mw, p, nt, static_cast<int>(ceil_div(a.M, nt)), static_cast<int>(tiles));
+  launch_pdl(gemm_pair_kernel<T, FORM>, dim3(2 * pairs), dim3(PR_THREADS), PR_SMEM, st, mx, mw, p, nt, static_cast<int>(ceil_div(a.M, nt)), static_cast<int>(tiles));
   B200_CHECK_LAUNCH("gemm_pair_kernel");
   return B200_OK;
+}
+
+template <typename T> int launch_pair_form(const Tc5Args& a, const Tc5Params& p, cudaStream_t st) {
+  if (p.splits > 1) return launch_pair_t<T, PairForm::SPLIT>(a, p, st);
+  if (p.epilogue & B200_EPI_GLU) return launch_pair_t<T, PairForm::GATED>(a, p, st);
+  const bool words = p.N % 8 == 0 && p.ldo % 8 == 0 && aligned16(p.out) && (!p.residual || (p.ldr % 8 == 0 && aligned16(p.residual))) &&
+                     (!(p.epilogue & B200_EPI_SILU_MUL) || (p.ldaux % 8 == 0 && aligned16(p.aux)));
+  return words ? launch_pair_t<T, PairForm::WORDS>(a, p, st) : launch_pair_t<T, PairForm::ANY>(a, p, st);
 }
 
 }  // namespace
 
 int gemm_pair(const Tc5Args& a, const Tc5Params& p, cudaStream_t st) {
-  return a.dtype == B200_BF16 ? launch_pair_t<__nv_bfloat16>(a, p, st) : launch_pair_t<__half>(a, p, st);
+  return a.dtype == B200_BF16 ? launch_pair_form<__nv_bfloat16>(a, p, st) : launch_pair_form<__half>(a, p, st);
 }
 
 int gemm_pair_error(bool clear) {

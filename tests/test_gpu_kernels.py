@@ -1421,50 +1421,56 @@ def test_conv3x3_runs_on_the_kernel_that_its_shape_calls_for(lib, N, H, Cn, O, k
     assert len(names) == 1 and kernel in names[0], names
 
 
-@pytest.mark.parametrize("M", [65, 80, 128, 129, 250, 257, 273, 500, 777])
-@pytest.mark.parametrize("form", ["plain", "residual", "residual unaligned", "gated", "silu mul", "split"])
+@pytest.mark.parametrize("M,form", [(M, form) for M in (65, 80, 128, 129, 250, 257, 273, 500, 777) for form in (
+    "plain", "plain odd", "residual", "residual relu", "residual unaligned", "gated", "gated unaligned", "silu mul", "silu mul aligned", "split") if form != "split" or M > 256])
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
 def test_linear_pair_token_tiles(lib, M, form, dtype):
     """Token tiles of every width (multiples of 16, a last one that is short), each epilogue, partial sums; columns that end inside a
-    block.  Bound: fp32 sums of K products (2^-20 of their magnitudes), each rounding to the activation type 2^-8 (bf16) or 2^-11."""
+    block; rows that are whole 16-byte words and rows that are not.  Bound: fp32 sums of K products (2^-20 of their magnitudes), each
+    rounding to the activation type 2^-8 (bf16) or 2^-11."""
     N, K = (9600, 1032) if form != "split" else (1536, 4104)
     if form in ("residual unaligned", "silu mul"):
         N = 9500
-    if form == "split" and M <= 256:
-        pytest.skip("too few tiles to split")
+    if form == "plain odd":
+        N = 9501
     a, w, bias = gen((M, K), dtype).cuda(), gen((N, K), dtype, 1, 0.05).cuda(), gen((N,), torch.float32, 2).cuda()
     eps = 2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -11
     s, size = a.double() @ w.double().T + bias.double(), a.double().abs() @ w.double().abs().T + bias.double().abs()
     slack = s.abs() * eps + size * 2.0 ** -20 + 1e-6
     epi, res, aux, out_cols = 0, None, None, N
-    if form == "gated":
+    if form in ("gated", "gated unaligned"):
         epi, out_cols = 4, N // 2
         blocks, sb = s.view(M, N // 128, 2, 64), slack.view(M, N // 128, 2, 64)
         gate, up = blocks[:, :, 0], blocks[:, :, 1]
         act = gate * torch.sigmoid(gate)
         want = (act * up).reshape(M, -1)
         slack = ((sb[:, :, 0] * 1.1 + act.abs() * (eps + 1e-5)) * up.abs() + act.abs() * sb[:, :, 1] + 2 * sb[:, :, 0] * sb[:, :, 1]).reshape(M, -1) + want.abs() * eps + 1e-6
-    elif form == "silu mul":
+    elif form in ("silu mul", "silu mul aligned"):
         epi, aux = 2, gen((M, N), dtype, 3).cuda()
         act = s * torch.sigmoid(s)
         want = act * aux.double()
         slack = (slack * 1.1 + act.abs() * (eps + 1e-5)) * aux.double().abs() + want.abs() * eps + 1e-6
-    elif form == "plain":
+    elif form in ("plain", "plain odd"):
         want = s
     else:
         res = gen((M, N), dtype, 3).cuda()
         want = s + res.double()
         slack = slack + want.abs() * eps
-    out = torch.full((M, out_cols), float("nan"), dtype=dtype, device="cuda")
+        if form == "residual relu":
+            epi, want = 1, torch.relu(want)
+    ldo = out_cols + (3 if form == "gated unaligned" else 0)
+    rows = torch.full((M, ldo), float("nan"), dtype=dtype, device="cuda")
+    out = rows[:, :out_cols]
     need = lib.b200_linear_workspace_bytes(M, N, K)
     assert (need > 0) == (form == "split")
     ws = torch.zeros(max(need, 16), dtype=torch.uint8, device="cuda")
     for _ in range(2):
-        ok(lib, lib.b200_linear(a.data_ptr(), w.data_ptr(), bias.data_ptr(), res.data_ptr() if res is not None else None, out.data_ptr(), M, N, K, K, K, out_cols,
+        ok(lib, lib.b200_linear(a.data_ptr(), w.data_ptr(), bias.data_ptr(), res.data_ptr() if res is not None else None, out.data_ptr(), M, N, K, K, K, ldo,
                                 N if res is not None else 0, DT[dtype], 0, epi, aux.data_ptr() if aux is not None else None, N if aux is not None else 0,
                                 ws.data_ptr(), need, stream()))
         err = (out.double() - want).abs()
         assert (err <= slack * 1.01).all(), float((err / slack).max())
+    assert rows[:, out_cols:].isnan().all()
     code = C.c_int(0)
     ok(lib, lib.b200_debug_device_error(C.byref(code), 1))
     assert code.value == 0
