@@ -50,16 +50,24 @@ def _mask_key(m: TensorView) -> tuple:
     return (m.buffer, m.offset, 1 if m.strides[0] == 0 else B, T, S, m.strides[0], m.strides[2])
 
 
-def _views_of(value):
-    """Every TensorView in a step's parameters."""
-    if isinstance(value, TensorView):
-        yield value
-    elif isinstance(value, dict):
-        for v in value.values():
-            yield from _views_of(v)
-    elif isinstance(value, (list, tuple)):
-        for v in value:
-            yield from _views_of(v)
+def _users(steps, names) -> dict[str, list[int]]:
+    """Steps whose parameters hold a view of each of the buffers ``names``, in order."""
+    found = {n: [] for n in names}
+
+    def look(i, values):
+        for v in values:
+            kind = type(v)
+            if kind is TensorView:
+                if v.buffer in found and found[v.buffer][-1:] != [i]:
+                    found[v.buffer].append(i)
+            elif kind is dict:
+                look(i, v.values())
+            elif kind is list or kind is tuple:
+                look(i, v)
+
+    for i, params in steps:
+        look(i, params.values())
+    return found
 
 
 def _find_stems(program: CUDAProgram, lib) -> list[tuple[int, int, int]]:
@@ -71,28 +79,25 @@ def _find_stems(program: CUDAProgram, lib) -> list[tuple[int, int, int]]:
     images 223 wide 32 against 42 / 301 against 583, 256 wide 35 against 44 / 360 against 798, 33 wide 15 against 16 / 41
     against 50; 200 wide, by TMA, 30 against 12 / 259 against 81)."""
     steps = [(i, s.params) for i, s in enumerate(program.steps) if getattr(s, "params", None)]
-    users: dict[str, list[int]] = {}
-    for i, p in steps:
-        for name in {v.buffer for v in _views_of(p)}:
-            users.setdefault(name, []).append(i)
-    for spec in program.output_specs:
-        view = program.views.get(spec.name)
-        if view is not None:
-            users.setdefault(view.buffer, []).append(-1)
+    convs = {p["x"].buffer: i for i, p in steps if p.get("op") == "conv2d"}
     inputs = {s.name for s in program.input_specs}
+    results = {program.views[s.name].buffer for s in program.output_specs if s.name in program.views}
     params, found = dict(steps), []
     for i, copy in steps:
-        if copy.get("op") != "strided_copy" or copy["in_view"].buffer not in inputs or len(copy["in_view"].shape) != 4:
+        if copy.get("op") != "strided_copy" or copy["in_view"].buffer not in inputs or len(copy["in_view"].shape) != 4 or copy["out_view"].buffer not in convs:
             continue
         x, mid = copy["in_view"], copy["out_view"].buffer
-        others = [j for j in users[mid] if j != i]
-        conv = params.get(others[0]) if len(others) == 1 else None
-        if conv is None or conv.get("op") != "conv2d" or conv["x"].buffer != mid or conv["residual"] is not None:
-            continue
+        at = convs[mid]
+        conv = params[at]
         y = conv["y"]
-        others = [j for j in users[y.buffer] if j != others[0]] + [others[0]]
-        pool = params.get(others[0]) if len(others) == 2 else None
-        if pool is None or pool.get("op") != "max_pool2d" or pool["x"].buffer != y.buffer or pool["y"].buffer == y.buffer:
+        if {mid, y.buffer} & results or conv["residual"] is not None:
+            continue
+        users = _users(steps, (mid, y.buffer))
+        if users[mid] != [i, at] or users[y.buffer][:1] != [at] or len(users[y.buffer]) != 2:
+            continue
+        last = users[y.buffer][1]
+        pool = params[last]
+        if pool.get("op") != "max_pool2d" or pool["x"].buffer != y.buffer or pool["y"].buffer == y.buffer:
             continue
         N, Cn, H, W = x.shape
         O, PH, PW = y.shape[1], (y.shape[2] - 1) // 2 + 1, (y.shape[3] - 1) // 2 + 1
@@ -103,7 +108,7 @@ def _find_stems(program: CUDAProgram, lib) -> list[tuple[int, int, int]]:
                 and [pool[k] for k in ("kernel_h", "kernel_w", "stride_h", "stride_w", "pad_h", "pad_w")] == [3, 3, 2, 2, 1, 1]
                 and tuple(pool["y"].shape) == (N, O, PH, PW) and tuple(pool["y"].strides) == (PH * PW * O, 1, PW * O, O)
                 and pool["y"].offset % 8 == 0 and lib.b200_conv_stem_pool_supported(Cn, H, W, *cv, DTYPE_CODES[y.dtype])):
-            found.append((i, others[1], others[0]))
+            found.append((i, at, last))
     return found
 
 
