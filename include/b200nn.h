@@ -349,7 +349,8 @@ int b200_conv2d_nhwc(const void* x, const void* w, const float* bias, const void
 /* The head of a convolution network in one launch: 7-wide / stride-2 convolution of a planar image [N, C <= 4, H, W], bias, ReLU
  * (epilogue), and the 3x3 / stride-2 / padding-1 max-pooling behind it (replaces the input repack, conv2d and
  * max_pool2d_kernel steps: cuda_executor.py:275-356, cuda_templates.py:315-352).  w: [O, KH, 7, 8] from b200_conv_weight_prep;
- * y: [N, PH, PW, O] of the pooled size.  b200_conv_stem_pool_supported tells (1 / 0) which shapes it takes. */
+ * y: [N, PH, PW, O] of the pooled size.  b200_conv_stem_pool_supported tells (1 / 0) which shapes it takes.  Rows that are no whole
+ * 16-byte words, or wider than 240, are copied element by element: the three kernels are faster there. */
 int b200_conv_stem_pool(const void* x, const void* w, const float* bias, void* y, int N, int C, int H, int W, int C_pad,
                         int O, int KH, int KW, int sh, int sw, int ph, int pw, int dtype, int epilogue, void* stream);
 int b200_conv_stem_pool_supported(int C, int H, int W, int C_pad, int O, int KH, int KW, int sh, int sw, int ph, int pw,

@@ -16,9 +16,10 @@
 //   tiles come into the same buffers beforehand).
 // - With resident weights two threads issue the MMAs of the tiles in turn: probes and commits of one (~0.4 us per tile) run
 //   beside the other's MMAs.
-// Bound by shared memory, which the MMAs read at 48 to 64 of 64 cycles while boxes and results pass through it.  us per layer, im2col boxes ->
-// this: 64 channels, 56 x 56, 256 / 32 / 16 images 143 -> 72, 24 -> 14, 14 -> 9; 128 channels, 28 x 28 77 -> 56, 16.4 -> 13.2, 14.8 -> 9.1;
-// 256 channels, 14 x 14, 32 images 24 -> 13.
+// Busiest unit, 256 images: the shared-memory pipe with the MMAs' operand reads, 64 % of the active cycles for 64 channels (tensor pipe 43 %) and
+// 62 % (62 %) for 128, where the last wave leaves a fifth of the time empty besides; L2 14 %, DRAM 23 % and below.  What fills the
+// rest is not measured.  us per layer, im2col boxes -> this: 64 channels, 56 x 56, 256 / 32 / 16 images 144 -> 73, 24 -> 14, 15 -> 10;
+// 128 channels, 28 x 28 86 -> 63, 17.7 -> 13.8, 15.0 -> 9.2; 256 channels, 14 x 14, 32 images 24 -> 13.
 #include "gemm_epilogue.cuh"
 #include "tc5.cuh"
 

@@ -444,7 +444,7 @@ class FakeLibrary:
         return 0
 
     def b200_attn_prefill_reads_tiles(self, mask, S, mask_b, mask_t, dtype):
-        return int(64 < S <= 32768 and mask % 16 == 0 and mask_b % 8 == 0 and mask_t % 8 == 0 and mask_t >= S and dtype in (1, 2))
+        return int(64 < S <= 32768 and mask % 16 == 0 and mask_b % 8 == 0 and mask_b >= 0 and mask_t % 8 == 0 and mask_t >= S and dtype in (1, 2))
 
     def b200_attn_prefill_tiles(self, q, k, v, mask, tiles, out, B, Hq, Hkv, T, S, D, qs, ks, vs, mask_b, mask_t, scale, dtype, stream):
         assert bool(_addr(tiles)) == bool(_addr(mask) and self.b200_attn_prefill_reads_tiles(_addr(mask), S, mask_b, mask_t, dtype))

@@ -37,6 +37,19 @@ def test_host_only_entry_points(native_lib):
     assert native_lib.b200_attn_decode_workspace_bytes(64, 12, 2, 32768, 128) == 64 * 2 * 64 * 6 * 130 * 4   # longer caches: 512-key splits + merge kernel
 
 
+def test_stand_in_and_library_agree_on_the_masks_whose_states_are_read(native_lib):
+    from fake_b200nn import FakeLibrary
+
+    fake = FakeLibrary()
+    for mask in (0x1000, 0x1008):
+        for S in (1, 64, 65, 100, 2048, 32768, 32769):
+            for mask_b in (0, 4096, 4100, -8):
+                for mask_t in (0, S, -(-S // 8) * 8, S + 8):
+                    for dtype in (0, 1, 2):
+                        args = (mask, S, mask_b, mask_t, dtype)
+                        assert native_lib.b200_attn_prefill_reads_tiles(*args) == fake.b200_attn_prefill_reads_tiles(*args), args
+
+
 def test_compiler_and_library_agree_on_the_splitk_shapes(native_lib):
     """The compiler appends an RMSNorm to a GEMM only for the shapes it expects the library to split over CTA pairs
     (`_pair_splitk_shape` of the lowering pass).  The library's own rule shows in its workspace sizing: for rows > 64 a
