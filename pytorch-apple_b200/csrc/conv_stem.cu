@@ -20,8 +20,8 @@
 //   one of the next), then bias and rounding to the activation type, which change no order; the column maxima go to shared memory;
 // - poolers (128 threads): the maximum over three columns, ReLU, 16 bytes per thread and step, to global memory.
 // Bounds: the tensor core, 14 MMAs of N = 64 per row at ~80 cycles (45 with swizzled operands, which sliding windows cannot be): 110
-// us for 256 images; the memory 28 us.  us, repack + convolution + pooling -> this: 256 images 90 + 344 + 166 = 600 -> 173, 32
-// images 90 -> 32, one image 18 -> 14.  On the way there: a window of one entry per two pixels x four channels, read in place at
+// us for 256 images; the memory 28 us.  us, repack + convolution + pooling -> this, images from memory: 256 images 584 -> 172,
+// 32 images 87 -> 29, one image 15 -> 8.  On the way there: a window of one entry per two pixels x four channels, read in place at
 // shifted addresses 205 (MMAs of 143 cycles); the same written four times 312 (the loaders); one MMA thread for all rows 205; a
 // division per pooled row in each role 216.
 #include "gemm_tc5.cuh"
