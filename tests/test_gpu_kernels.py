@@ -5,6 +5,7 @@ bit-exact; floating point uses the op-level tolerance of the reference's CUDA te
 
 import ctypes as C
 import math
+import subprocess
 
 import numpy as np
 import pytest
@@ -27,6 +28,11 @@ def ok(lib, rc):
     torch.cuda.synchronize()
 
 
+def go(lib, rc):
+    """The call was taken; nothing waits for it (the next launch may follow at once)."""
+    assert rc == 0, lib.b200_last_error().decode()
+
+
 def stream():
     return torch.cuda.current_stream().cuda_stream
 
@@ -39,6 +45,34 @@ def bt(t):
     from cuda_runtime import native
 
     return native.make_tensor(t.data_ptr(), str(t.dtype).replace("torch.", ""), tuple(t.shape), tuple(t.stride()))
+
+
+class _KernelNode(C.Structure):   # CUDA_KERNEL_NODE_PARAMS of the driver API, version 2
+    _fields_ = [("func", C.c_void_p), ("dims", C.c_uint * 7), ("params", C.c_void_p), ("extra", C.c_void_p), ("kern", C.c_void_p), ("ctx", C.c_void_p)]
+
+
+def kernels_of(call):
+    """Names of the kernels that a call launches: the nodes of a graph that it is captured into.  (The profiler now and then
+    reports nothing, more often the more tests ran before.)"""
+    call()
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph(keep_graph=True)
+    with torch.cuda.graph(graph):
+        call()
+    cu = C.CDLL("libcuda.so.1")
+    raw, n, names = C.c_void_p(graph.raw_cuda_graph()), C.c_size_t(0), []
+    assert cu.cuGraphGetNodes(raw, None, C.byref(n)) == 0
+    nodes = (C.c_void_p * n.value)()
+    assert cu.cuGraphGetNodes(raw, nodes, C.byref(n)) == 0
+    for node in nodes:
+        kind, p, name = C.c_int(-1), _KernelNode(), C.c_char_p()
+        assert cu.cuGraphNodeGetType(C.c_void_p(node), C.byref(kind)) == 0
+        if kind.value != 0:   # not a kernel
+            continue
+        assert cu.cuGraphKernelNodeGetParams_v2(C.c_void_p(node), C.byref(p)) == 0
+        assert (cu.cuFuncGetName(C.byref(name), C.c_void_p(p.func)) if p.func else cu.cuKernelGetName(C.byref(name), C.c_void_p(p.kern))) == 0
+        names.append(subprocess.run(["c++filt", name.value.decode()], capture_output=True, text=True, check=True).stdout)
+    return names
 
 
 def close(got, ref, rtol=2e-2, atol=1e-2):
@@ -269,9 +303,7 @@ def test_linear_few_rows_edges(lib, M, N, K, shift, ldx, dtype):
 def test_linear_runs_on_the_kernel_that_its_shape_calls_for(lib, M, N, K, res, kernel):
     t = torch.zeros(M * K + N * K + 2 * M * N, dtype=torch.bfloat16, device="cuda")
     a, w, o, r = (t[n:].data_ptr() for n in (0, M * K, M * K + N * K, M * K + N * K + M * N))
-    with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CUDA]) as prof:
-        ok(lib, lib.b200_linear(a, w, None, r if res else None, o, M, N, K, K, K, N, N if res else 0, 2, 2, 8, None, 0, None, 0, stream()))
-    ran = [e.key for e in prof.key_averages() if "gemm" in e.key]
+    ran = kernels_of(lambda: go(lib, lib.b200_linear(a, w, None, r if res else None, o, M, N, K, K, K, N, N if res else 0, 2, 2, 8, None, 0, None, 0, stream())))
     assert len(ran) == 1 and kernel + "<" in ran[0], ran
 
 
@@ -704,19 +736,22 @@ def test_attn_prefill_few_keys(lib, B, T, S, kind, dtype):
     M[..., :S] = mask.cuda()
     Q, K, V = q.cuda(), k.cuda(), v.cuda()
     st = lambda t: (C.c_int64 * 3)(*t.stride()[:3])
-    out = torch.empty((B, T, Hq, D), dtype=dtype, device="cuda")
-    names = []
-    for _ in range(3):   # (a profiling session now and then reports nothing)
-        out.fill_(float("nan"))
-        with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CUDA]) as prof:
-            ok(lib, lib.b200_attn_prefill(Q.data_ptr(), K.data_ptr(), V.data_ptr(), M.data_ptr() if kind else None, out.data_ptr(), B, Hq, Hkv, T, S, D, st(Q), st(K), st(V),
-                                          T * pitch, pitch, D ** -0.5, DT[dtype], stream()))
-            torch.cuda.synchronize()
-        names = names or [e.key for e in prof.key_averages() if "attn_prefill" in e.key]
-    assert len(names) == 1 and ("tc5" in names[0]) == (S > 64), names
+    out = torch.full((B, T, Hq, D), float("nan"), dtype=dtype, device="cuda")
+    ok(lib, lib.b200_attn_prefill(Q.data_ptr(), K.data_ptr(), V.data_ptr(), M.data_ptr() if kind else None, out.data_ptr(), B, Hq, Hkv, T, S, D, st(Q), st(K), st(V),
+                                  T * pitch, pitch, D ** -0.5, DT[dtype], stream()))
     eps = 2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -11
     err = (out.double().cpu() - want).abs()
     assert (err <= (size + want.abs()) * eps * 1.01 + 1e-5).all(), float(err.max())
+
+
+@pytest.mark.parametrize("T,S,kernel", [(16, 16, "attn_prefill_kernel"), (200, 64, "attn_prefill_kernel"), (3, 65, "attn_prefill_tc5_kernel"), (129, 100, "attn_prefill_tc5_kernel")])
+def test_attn_prefill_runs_on_the_kernel_that_its_keys_call_for(lib, T, S, kernel):
+    Q, K = torch.zeros(1, 4, T, 128, dtype=torch.bfloat16, device="cuda"), torch.zeros(1, 2, S, 128, dtype=torch.bfloat16, device="cuda")
+    out = torch.empty(1, T, 4, 128, dtype=torch.bfloat16, device="cuda")
+    st = lambda t: (C.c_int64 * 3)(*t.stride()[:3])
+    names = kernels_of(lambda: go(lib, lib.b200_attn_prefill(Q.data_ptr(), K.data_ptr(), K.data_ptr(), None, out.data_ptr(), 1, 4, 2, T, S, 128, st(Q), st(K), st(K),
+                                                             0, 0, 0.1, 2, stream())))
+    assert len(names) == 1 and kernel + "<" in names[0], names
 
 
 @pytest.mark.parametrize("T", [128, 400])
@@ -731,7 +766,7 @@ def test_attn_prefill_many_launches_in_a_row(lib, T):
     st = lambda t: (C.c_int64 * 3)(*t.stride()[:3])
     outs = [torch.empty((1, T, Hq, D), dtype=dtype, device="cuda") for _ in range(200)]
     for out in outs:
-        ok(lib, lib.b200_attn_prefill_tiles(Q.data_ptr(), K.data_ptr(), V.data_ptr(), M.data_ptr(), tiles.data_ptr(), out.data_ptr(), 1, Hq, Hkv,
+        go(lib, lib.b200_attn_prefill_tiles(Q.data_ptr(), K.data_ptr(), V.data_ptr(), M.data_ptr(), tiles.data_ptr(), out.data_ptr(), 1, Hq, Hkv,
                                             T, T, D, st(Q), st(K), st(V), 0, T, D ** -0.5, 2, stream()))
     assert all(torch.equal(outs[0], out) for out in outs[1:])
     code = C.c_int(0)
@@ -756,7 +791,7 @@ def test_attn_prefill_first_key_tiles_masked_and_keys_far_away(lib, lead):
 
     def call(i):
         out = torch.full((B, T, Hq, D), float("nan"), dtype=dtype, device="cuda")
-        ok(lib, lib.b200_attn_prefill_tiles(Q.data_ptr(), K[i].data_ptr(), V[i].data_ptr(), M.data_ptr(), tiles.data_ptr(), out.data_ptr(), B, Hq, Hkv,
+        go(lib, lib.b200_attn_prefill_tiles(Q.data_ptr(), K[i].data_ptr(), V[i].data_ptr(), M.data_ptr(), tiles.data_ptr(), out.data_ptr(), B, Hq, Hkv,
                                             T, S, D, st(Q), st(K[i]), st(V[i]), 0, S, D ** -0.5, 2, stream()))
         return out
 
@@ -813,7 +848,7 @@ def test_attn_prefill_row_blocks_without_keys(lib, known):
     st = lambda t: (C.c_int64 * 3)(*t.stride()[:3])
     outs = [torch.full((1, T, Hq, D), float("nan"), dtype=dtype, device="cuda") for _ in range(50)]
     for out in outs:
-        ok(lib, lib.b200_attn_prefill_tiles(Q.data_ptr(), K.data_ptr(), V.data_ptr(), M.data_ptr(), tiles.data_ptr() if known else None, out.data_ptr(), 1, Hq, Hkv,
+        go(lib, lib.b200_attn_prefill_tiles(Q.data_ptr(), K.data_ptr(), V.data_ptr(), M.data_ptr(), tiles.data_ptr() if known else None, out.data_ptr(), 1, Hq, Hkv,
                                             T, S, D, st(Q), st(K), st(V), 0, 304, D ** -0.5, 2, stream()))
     rows = slice(128 * 3, 128 * 5)
     p = ((q[:, :, rows].double() @ k.double().repeat_interleave(6, 1).transpose(2, 3)) * D ** -0.5).softmax(-1)
@@ -1312,10 +1347,10 @@ def test_conv_stem_pool_behind_the_kernel_that_prepares_its_weights(lib, dtype):
 
     def call(i, out, wait):
         w, b = sets[i]
-        ok(lib, lib.b200_conv_weight_prep(w.data_ptr(), b.data_ptr(), None, None, None, None, packed.data_ptr(), bias.data_ptr(), O, 3, 7, 7, 8, 0.0, 0, 0, DT[dtype], stream()))
+        go(lib, lib.b200_conv_weight_prep(w.data_ptr(), b.data_ptr(), None, None, None, None, packed.data_ptr(), bias.data_ptr(), O, 3, 7, 7, 8, 0.0, 0, 0, DT[dtype], stream()))
         if wait:
             torch.cuda.synchronize()
-        ok(lib, lib.b200_conv_stem_pool(x.data_ptr(), packed.data_ptr(), bias.data_ptr(), out.data_ptr(), N, 3, H, W, 8, O, 7, 7, 2, 2, 3, 3, DT[dtype], 1, stream()))
+        go(lib, lib.b200_conv_stem_pool(x.data_ptr(), packed.data_ptr(), bias.data_ptr(), out.data_ptr(), N, 3, H, W, 8, O, 7, 7, 2, 2, 3, 3, DT[dtype], 1, stream()))
 
     for i in range(len(sets)):
         call(i, outs[i], False)
@@ -1356,12 +1391,7 @@ def test_adaptive_avg_pool_runs_on_the_kernel_that_its_shape_calls_for(lib, N, C
     x = gen((N, Cn, H, H), torch.float16).cuda().contiguous(memory_format=torch.channels_last)
     y = torch.empty(N, OH, OH, Cn, dtype=torch.float16, device="cuda").permute(0, 3, 1, 2)
     a, b = bt(x), bt(y)
-    names = []
-    for _ in range(3):   # (a profiling session now and then reports nothing)
-        with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CUDA]) as prof:
-            ok(lib, lib.b200_adaptive_avg_pool2d(C.byref(a), C.byref(b), stream()))
-            torch.cuda.synchronize()
-        names = names or [e.key for e in prof.key_averages() if "_kernel" in e.key]
+    names = kernels_of(lambda: go(lib, lib.b200_adaptive_avg_pool2d(C.byref(a), C.byref(b), stream())))
     assert len(names) == 1 and kernel in names[0], names
     want = torch.nn.functional.adaptive_avg_pool2d(x.double(), OH)
     size = torch.nn.functional.adaptive_avg_pool2d(x.double().abs(), OH)
@@ -1411,13 +1441,8 @@ def test_conv3x3_rows(lib, dtype, N, H, W, Cn, O, res, relu):
 def test_conv3x3_runs_on_the_kernel_that_its_shape_calls_for(lib, N, H, Cn, O, kernel):
     x, w = torch.zeros(N, H, H, Cn, dtype=torch.float16, device="cuda"), torch.zeros(O, 3, 3, Cn, dtype=torch.float16, device="cuda")
     y = torch.empty(N, H, H, O, dtype=torch.float16, device="cuda")
-    call = lambda: ok(lib, lib.b200_conv2d_nhwc(x.data_ptr(), w.data_ptr(), None, None, y.data_ptr(), N, H, H, Cn, Cn, O, 3, 3, 1, 1, 1, 1, H, H, 1, 0, stream()))
-    names = []
-    for _ in range(3):   # (a profiling session now and then reports nothing)
-        with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CUDA]) as prof:
-            call()
-            torch.cuda.synchronize()
-        names = names or [e.key for e in prof.key_averages() if "_kernel" in e.key]
+    call = lambda: go(lib, lib.b200_conv2d_nhwc(x.data_ptr(), w.data_ptr(), None, None, y.data_ptr(), N, H, H, Cn, Cn, O, 3, 3, 1, 1, 1, 1, H, H, 1, 0, stream()))
+    names = kernels_of(call)
     assert len(names) == 1 and kernel in names[0], names
 
 
