@@ -150,6 +150,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PR_THREADS, 1)
     pdl_wait();
     const bool silu = (p.epilogue & B200_EPI_SILU_MUL) != 0, relu = (p.epilogue & B200_EPI_RELU) != 0;
     const T* const res = static_cast<const T*>(p.residual);
+    const T* const early = res ? res : silu ? static_cast<const T*>(p.aux) : nullptr;
+    const int64_t early_ld = res ? p.ldr : p.ldaux;
     const uint32_t lead_acc_empty0 = tc5::map_to_rank(tc5::smem_addr(&acc_empty[0]), 0);
     // the group's four warps leave together: they meet at a barrier of their own
     auto any = [&](bool v) {
@@ -231,14 +233,15 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PR_THREADS, 1)
             if (c + 2 * PR_CHUNK < nt) tc5::tmem_ld_32x32_async(t_row + c + 2 * PR_CHUNK, v);
             continue;
           }
-          // 16-byte words of the result that this thread finishes: two items of two tokens 2 (i / 16) .. and columns 8 (i % 16) ..; residual requested now
+          // 16-byte words of the result that this thread finishes: two items of two tokens 2 (i / 16) .. and columns 8 (i % 16) ..; what is read with
+          // them (residual, else the other factor) is requested now
           uint4 r[4];
-          if (FORM == PairForm::WORDS && res) {
+          if (FORM == PairForm::WORDS && early) {
 #pragma unroll
             for (int k = 0; k < 4; ++k) {
               const int i = t + 128 * (k >> 1), j = 2 * (i >> 4) + (k & 1);
               const int64_t n = n0 + 8 * (i & 15);
-              r[k] = j < tokens && n < p.N ? __ldg(reinterpret_cast<const uint4*>(res + (m0 + c + j) * p.ldr + n)) : make_uint4(0u, 0u, 0u, 0u);
+              r[k] = j < tokens && n < p.N ? __ldg(reinterpret_cast<const uint4*>(early + (m0 + c + j) * early_ld + n)) : make_uint4(0u, 0u, 0u, 0u);
             }
           }
           // [pair of tokens][column], a word each: half the stores of single values, and no two of a warp in one bank
@@ -309,7 +312,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PR_THREADS, 1)
                 if (silu) {
                   float f[8], x[8];
                   unpack8<T>(make_uint4(o[0], o[1], o[2], o[3]), f);
-                  unpack8<T>(__ldg(reinterpret_cast<const uint4*>(static_cast<const T*>(p.aux) + m * p.ldaux + n)), x);
+                  unpack8<T>(res ? __ldg(reinterpret_cast<const uint4*>(static_cast<const T*>(p.aux) + m * p.ldaux + n)) : r[2 * k + e], x);
 #pragma unroll
                   for (int q = 0; q < 8; q += 2) {
                     float y0 = silu_f32(f[q]), y1 = silu_f32(f[q + 1]);
